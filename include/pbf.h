@@ -249,11 +249,10 @@ pbf_status pbf_batch_use_graphs(pbf_batch* b, int on);
  * the windows of 32 particles), whether every particle does, the order in
  * which the passes take particles (the cell order of the grid, or the cell
  * each particle is in at that iteration), how many warps of the dense kernel
- * split a batch's windows, how many neighbour chunks a thread queues before
- * running their pair terms, and how many candidate positions a block of each
- * pass kernel may stage in shared memory (bulk asynchronous copies of the
- * column runs its particles' windows share, read there instead of through
- * L1) -- by running `steps` steps per choice from copies of the
+ * split a batch's windows, how many neighbour chunks its threads queue before
+ * running their pair terms, and how many candidate positions a block of that
+ * kernel may stage in shared memory (bulk asynchronous copies of the column
+ * runs its particles' windows share, read there instead of through L1) -- by running `steps` steps per choice from copies of the
  * caller's state (pos, vel, iid: device, n entries; they are not modified),
  * and keeps the fastest for the solver's following steps.  The window and
  * dense choices change the order in which window sums are added, so results
@@ -272,14 +271,16 @@ typedef struct pbf_tuning {
   int order;          /* 1: current-cell order (the default); 0: grid order */
   int bwd_lanes;      /* pbf_backward, steps under 131072 particles: lanes per particle, 8, 16
                          or 32 (0: the default, 32); not timed by pbf_autotune */
-  int stage_sparse;   /* slots (16 bytes each) a block of the one-thread-per-particle kernel
-                         copies into shared memory when its particles share one column of
-                         cells (0: none; at most 4096) */
-  int stage_dense;    /* the same for a block of the dense kernel */
-  int queue_sparse;   /* neighbour chunks of 32 candidates whose hits a thread of the
-                         one-thread-per-particle kernel queues before running their pair terms
-                         in one loop (1: each chunk's right away; at most 16) */
-  int queue_dense;    /* the same for the dense kernel (at most 8) */
+  int stage_sparse;   /* kept (at most 4096), no effect: the one-thread-per-particle kernel has
+                         no staged variant any more */
+  int stage_dense;    /* slots (16 bytes each) a block of the dense kernel copies into shared
+                         memory when its particles share one column of cells (0: none; at
+                         most 4096) */
+  int queue_sparse;   /* kept (at most 16), no effect: that kernel always queues the hits of a
+                         window */
+  int queue_dense;    /* neighbour chunks of 32 candidates whose hits a thread of the dense
+                         kernel queues before running their pair terms in one loop (1: each
+                         chunk's right away; at most 8) */
   int dense_split;    /* warps of the dense kernel that split one batch of 32 particles'
                          windows: 1, 2, 4 or 8 (a block of 8 warps takes 8 / dense_split
                          batches at a time) */

@@ -18,11 +18,8 @@
 
 #include "pbf_internal.cuh"
 
-// The kernels index per-particle tables with int: the neighbour masks
-// (kMaskWords words per particle) and the group hash (8 ints per particle)
-// are the largest.
-static_assert((long long)pbf::kMaskWords * PBF_MAX_PARTICLES - 1 <= 2147483647LL,
-              "mask index overflows int at PBF_MAX_PARTICLES");
+// The kernels index per-particle tables with int (the hit lists with size_t):
+// the group hash (8 ints per particle) is the largest.
 static_assert(8LL * PBF_MAX_PARTICLES - 1 <= 2147483647LL, "group hash index overflows int at PBF_MAX_PARTICLES");
 
 // Executable graphs of recent steps.  A step's launches depend only on its
@@ -316,9 +313,7 @@ pbf::StepConsts make_consts(const pbf_params& p, const float ulim[3], const floa
   c.dense_window = pbf::kDefaultDenseWindow;
   c.dense_all = -1;
   c.order = 1;
-  c.stage_sparse = pbf::kDefaultStageSparse;
   c.stage_dense = pbf::kDefaultStageDense;
-  c.queue_sparse = pbf::kDefaultQueueSparse;
   c.queue_dense = pbf::kDefaultQueueDense;
   c.dense_split = pbf::kDefaultDenseSplit;
   c.dense_interleave = pbf::kDefaultDenseInterleave;
@@ -394,12 +389,26 @@ cudaError_t alloc_groups(pbf::SolverScratch& sol, int max_particles) {
   return e;
 }
 
+// Positions with lambda, component copies and hit lists of the passes.
+cudaError_t alloc_pass_lists(pbf::SolverScratch& sol, int max_particles) {
+  const size_t stride = (size_t)pbf::particle_stride(max_particles);
+  sol.stride = (int)stride;
+  cudaError_t e = alloc(&sol.xl, (size_t)max_particles);
+  if (e == cudaSuccess) e = alloc(&sol.sa, 3 * stride);
+  if (e == cudaSuccess) e = alloc(&sol.sb, 3 * stride);
+  const size_t slots = pbf::list_slots(max_particles);
+  sol.hit_stride = (int)slots;
+  if (e == cudaSuccess) e = alloc(&sol.hits, (size_t)pbf::kHitCap * slots);
+  if (e == cudaSuccess) e = alloc(&sol.hit_n, slots);
+  return e;
+}
+
 // Current-cell buckets (StepConsts::order) for up to np particles and nc - 1 cells.
 cudaError_t alloc_buckets(pbf::SolverScratch& sol, size_t np, size_t nc) {
   cudaError_t e = alloc(&sol.bcnt, nc);
   if (e == cudaSuccess) e = alloc(&sol.bstart, nc);
   if (e == cudaSuccess) e = alloc(&sol.bent, np);
-  if (e == cudaSuccess) e = alloc(&sol.bucket, np);
+  if (e == cudaSuccess) e = alloc(&sol.bucket, pbf::list_slots((int)np));
   if (e == cudaSuccess) e = alloc(&sol.bpart, (size_t)pbf::kMaxScanPartials);
   return e;
 }
@@ -408,7 +417,8 @@ void free_all(pbf_solver* s) {
   void* ptrs[] = {s->grid.keys_a, s->grid.keys_b, s->grid.vals_a, s->grid.vals_b,
                   s->grid.cell_count, s->grid.cell_start, s->grid.radix_counts,
                   s->grid.scan_partials, s->sol.xs, s->sol.xa, s->sol.xb, s->sol.iid_s,
-                  s->sol.lambda, s->sol.rho, s->sol.flags, s->sol.dense, s->sol.masks,
+                  s->sol.lambda, s->sol.rho, s->sol.flags, s->sol.dense, s->sol.xl, s->sol.sa,
+                  s->sol.sb, s->sol.hits, s->sol.hit_n,
                   s->sol.cell_flags, s->sol.grp_cell, s->sol.grp_off, s->sol.grp_n, s->sol.grp_rep, s->sol.grp_cnt,
                   s->sol.grp_pos, s->sol.grp_sum, s->sol.grp_aux, s->sol.grp_id, s->sol.grp_hash,
                   s->sol.grp_max, s->sol.grp_acc, s->sol.grp_list, s->sol.grp_list_n, s->sol.grp_done,
@@ -550,8 +560,7 @@ pbf_status pbf_create(const pbf_params* params, const float ulim[3], const float
   if (e == cudaSuccess) e = alloc(&s->sol.flags, (size_t)pbf::kFlagWords);
   if (e == cudaSuccess) e = cudaMemset(s->sol.flags, 0, sizeof(uint32_t) * pbf::kFlagWords);
   if (e == cudaSuccess) e = alloc(&s->sol.dense, pbf::dense_list_len(max_particles));
-  if (e == cudaSuccess) e = alloc(&s->sol.masks, (size_t)pbf::kMaskWords * np);
-  s->sol.mask_stride = (int)np;
+  if (e == cudaSuccess) e = alloc_pass_lists(s->sol, max_particles);
   if (e == cudaSuccess) e = alloc(&s->sol.cell_flags, nc);
   if (e == cudaSuccess) e = alloc_groups(s->sol, max_particles);
   if (e == cudaSuccess) e = alloc_buckets(s->sol, np, nc);
@@ -817,9 +826,7 @@ pbf_status pbf_step(pbf_solver* s, void* pos, void* npos, void* vel, void* nvel,
   if (s->tune_window > 0) P.c.dense_window = s->tune_window;
   P.c.dense_all = s->tune_all;
   if (s->tune_order >= 0) P.c.order = s->tune_order;
-  if (s->tune_stage_sparse >= 0) P.c.stage_sparse = s->tune_stage_sparse;
   if (s->tune_stage_dense >= 0) P.c.stage_dense = s->tune_stage_dense;
-  if (s->tune_queue_sparse > 0) P.c.queue_sparse = s->tune_queue_sparse;
   if (s->tune_queue_dense > 0) P.c.queue_dense = s->tune_queue_dense;
   if (s->tune_split > 0) P.c.dense_split = s->tune_split;
   if (s->tune_interleave >= 0) P.c.dense_interleave = s->tune_interleave;
@@ -1171,7 +1178,8 @@ void batch_free(pbf_batch* b) {
   void* ptrs[] = {b->grid.keys_a, b->grid.keys_b, b->grid.vals_a, b->grid.vals_b,
                   b->grid.cell_count, b->grid.cell_start, b->grid.radix_counts,
                   b->grid.scan_partials, b->sol.xs, b->sol.xa, b->sol.xb, b->sol.iid_s,
-                  b->sol.lambda, b->sol.rho, b->sol.flags, b->sol.dense, b->sol.masks,
+                  b->sol.lambda, b->sol.rho, b->sol.flags, b->sol.dense, b->sol.xl, b->sol.sa,
+                  b->sol.sb, b->sol.hits, b->sol.hit_n,
                   b->sol.cell_flags, b->sol.grp_cell, b->sol.grp_off, b->sol.grp_n, b->sol.grp_rep, b->sol.grp_cnt,
                   b->sol.grp_pos, b->sol.grp_sum, b->sol.grp_aux, b->sol.grp_id, b->sol.grp_hash,
                   b->sol.grp_max, b->sol.grp_acc, b->sol.grp_list, b->sol.grp_list_n, b->sol.grp_done,
@@ -1261,8 +1269,7 @@ pbf_status pbf_batch_create(const pbf_params* params, int nscenes, const float* 
   if (e == cudaSuccess) e = alloc(&b->sol.flags, (size_t)pbf::kFlagWords);
   if (e == cudaSuccess) e = cudaMemset(b->sol.flags, 0, sizeof(uint32_t) * pbf::kFlagWords);
   if (e == cudaSuccess) e = alloc(&b->sol.dense, pbf::dense_list_len((int)np));
-  if (e == cudaSuccess) e = alloc(&b->sol.masks, (size_t)pbf::kMaskWords * np);
-  b->sol.mask_stride = (int)np;
+  if (e == cudaSuccess) e = alloc_pass_lists(b->sol, (int)np);
   if (e == cudaSuccess) e = alloc(&b->sol.cell_flags, nc);
   if (e == cudaSuccess) e = alloc_groups(b->sol, (int)np);
   if (e == cudaSuccess) e = alloc_buckets(b->sol, np, nc);
@@ -1348,9 +1355,7 @@ pbf_status pbf_batch_step(pbf_batch* b, void* pos, void* npos, void* vel, void* 
   if (b->tune_window > 0) P.c.dense_window = b->tune_window;
   P.c.dense_all = b->tune_all;
   if (b->tune_order >= 0) P.c.order = b->tune_order;
-  if (b->tune_stage_sparse >= 0) P.c.stage_sparse = b->tune_stage_sparse;
   if (b->tune_stage_dense >= 0) P.c.stage_dense = b->tune_stage_dense;
-  if (b->tune_queue_sparse > 0) P.c.queue_sparse = b->tune_queue_sparse;
   if (b->tune_queue_dense > 0) P.c.queue_dense = b->tune_queue_dense;
   if (b->tune_split > 0) P.c.dense_split = b->tune_split;
   if (b->tune_interleave >= 0) P.c.dense_interleave = b->tune_interleave;
@@ -1443,9 +1448,7 @@ namespace {
 constexpr int kTuneWindows[] = {64, 128, 256, 512, 1024, 2048};
 constexpr int kTuneSplits[] = {1, 2, 4, 8};
 constexpr int kTuneInterleave[] = {0, 1};
-constexpr int kTuneQueueSparse[] = {1, 10, 16};
 constexpr int kTuneQueueDense[] = {1, 4, 8};
-constexpr int kTuneStageSparse[] = {0, 1024, 2048};
 constexpr int kTuneStageDense[] = {0, 1536, 3072};
 
 // One configuration of the neighbour passes (the fields of pbf_tuning that
@@ -1513,7 +1516,7 @@ void fill_tuning(const TuneState& t, pbf_tuning* out) {
 // step(choice, bufs...) and returns the fastest choice: first over the
 // window, dense and order choices with the other fields at their defaults,
 // then, from the best so far, one field at a time: the dense split, the
-// sparse and dense hit queues, the sparse and dense stages.
+// dense kernel's hit queue and its stage.
 template <class Step>
 pbf_status autotune(int n, const void* pos, const void* vel, const uint32_t* iid, int steps, cudaStream_t st,
                     Step step, pbf_tuning* out) {
@@ -1585,9 +1588,7 @@ pbf_status autotune(int n, const void* pos, const void* vel, const uint32_t* iid
   };
   sweep(&TuneChoice::split, kTuneSplits, 4);
   if (best_ch.split > 1) sweep(&TuneChoice::interleave, kTuneInterleave, 2);
-  if (!best_ch.all) sweep(&TuneChoice::queue_sparse, kTuneQueueSparse, 3);
   sweep(&TuneChoice::queue_dense, kTuneQueueDense, 3);
-  if (!best_ch.all) sweep(&TuneChoice::stage_sparse, kTuneStageSparse, 3);
   sweep(&TuneChoice::stage_dense, kTuneStageDense, 3);
   for (void* q : {(void*)p[0], (void*)p[1], (void*)v[0], (void*)v[1], (void*)id})
     if (q) cudaFree(q);

@@ -62,13 +62,14 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // ---- exclusive scan of a uint32 array (reduce, scan partials, downsweep) -------
 
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_reduce(const uint32_t* __restrict__ in, int len, uint32_t* __restrict__ partials) {
+k_scan_reduce(const uint32_t* __restrict__ in, int len, uint32_t* __restrict__ partials, const uint32_t* __restrict__ groups) {
   __shared__ uint32_t smem[kScanThreads / 32 + 1];
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  const bool apart = groups && *groups != 0u;
   uint32_t sum = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k)
-    if (base + k < len) sum += in[base + k];
+    if (base + k < len) sum += groups ? pair_slots(in[base + k], apart) : in[base + k];
   uint32_t total;
   block_exclusive_scan<kScanThreads>(sum, smem, &total);
   if (threadIdx.x == 0) partials[blockIdx.x] = total;
@@ -96,16 +97,19 @@ k_scan_top(uint32_t* __restrict__ partials, int count) {
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_down(const uint32_t* in, int len, const uint32_t* __restrict__ partials, uint32_t* out) {
+k_scan_down(const uint32_t* in, int len, const uint32_t* __restrict__ partials, uint32_t* out,
+            const uint32_t* __restrict__ groups) {
   // in and out may alias (in-place scan): every thread reads its items before
   // writing them, and no thread touches another thread's items.
   __shared__ uint32_t smem[kScanThreads / 32 + 1];
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  const bool apart = groups && *groups != 0u;
   uint32_t v[kScanItems];
   uint32_t sum = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     v[k] = base + k < len ? in[base + k] : 0u;
+    if (groups) v[k] = pair_slots(v[k], apart);
     sum += v[k];
   }
   uint32_t total;
@@ -120,13 +124,13 @@ k_scan_down(const uint32_t* in, int len, const uint32_t* __restrict__ partials, 
 
 }  // namespace
 
-cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t* partials,
-                           cudaStream_t stream) {
+cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t* partials, cudaStream_t stream,
+                           const uint32_t* groups) {
   const int tiles = (len + kScanTile - 1) / kScanTile;
   if (tiles > kMaxScanPartials) return cudaErrorInvalidValue;
-  k_scan_reduce<<<tiles, kScanThreads, 0, stream>>>(in, len, partials);
+  k_scan_reduce<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, groups);
   k_scan_top<<<1, kTopThreads, 0, stream>>>(partials, tiles);
-  k_scan_down<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, out);
+  k_scan_down<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, out, groups);
   return cudaGetLastError();
 }
 

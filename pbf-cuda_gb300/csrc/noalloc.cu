@@ -50,6 +50,8 @@ pbf_status validate_step_buffers(const void* pos, const void* npos, const void* 
 namespace {
 
 constexpr int kNoAllocMaxParticles = 32768;
+// every particle takes the dense kernel: no component copies, no hit lists
+static_assert(kNoAllocMaxParticles < pbf::kDenseAllBelow, "the one-thread-per-particle kernel needs its lists");
 constexpr int kNoAllocMaxCells = 131072;
 constexpr size_t kAlign = 256;
 
@@ -75,8 +77,8 @@ constexpr size_t kOffLambda = kOffIid + align_up(4 * kNp);
 constexpr size_t kOffRho = kOffLambda + align_up(4 * kNp);
 constexpr size_t kOffFlags = kOffRho + align_up(4 * kNp);
 constexpr size_t kOffDense = kOffFlags + align_up(4 * (size_t)pbf::kFlagWords);
-constexpr size_t kOffMasks = kOffDense + align_up(4 * pbf::dense_list_len(kNoAllocMaxParticles));
-constexpr size_t kOffCellFlags = kOffMasks + align_up(4 * (size_t)pbf::kMaskWords * kNp);
+constexpr size_t kOffXl = kOffDense + align_up(4 * pbf::dense_list_len(kNoAllocMaxParticles));
+constexpr size_t kOffCellFlags = kOffXl + align_up(16 * kNp);
 constexpr size_t kSlots = (size_t)kNoAllocMaxParticles / pbf::kGroupCell + 1;
 constexpr size_t kEntries = kNp;
 constexpr size_t kOffGrpCell = kOffCellFlags + align_up(4 * kNc);
@@ -196,8 +198,7 @@ extern "C" pbf_status pbf_step_noalloc(const pbf_params* params, const float uli
   s.rho = (float*)(base + kOffRho);
   s.flags = (uint32_t*)(base + kOffFlags);
   s.dense = (uint32_t*)(base + kOffDense);
-  s.masks = (uint32_t*)(base + kOffMasks);
-  s.mask_stride = kNoAllocMaxParticles;
+  s.xl = (float4*)(base + kOffXl);
   s.cell_flags = (uint32_t*)(base + kOffCellFlags);
   s.grp_pool = kNoAllocMaxParticles;
   s.grp_cell = (int*)(base + kOffGrpCell);

@@ -58,10 +58,8 @@ struct StepConsts {
   int dense_window;        // candidates above which a warp takes the dense kernel
   int dense_all;           // 1: every warp takes the dense kernel; 0: never; -1: by particle count
   int order;               // 1: the passes take particles in current-cell order (bucketed); 0: grid order
-  int stage_sparse;        // slots a sparse-kernel block may stage in shared memory (0: none)
   int stage_dense;         // slots a dense-kernel block may stage in shared memory (0: none)
-  int queue_sparse;        // hit-queue chunks per thread of the sparse / dense kernel (1: none)
-  int queue_dense;
+  int queue_dense;         // hit-queue chunks per thread of the dense kernel (1: none)
   int dense_split;         // warps of the dense kernel sharing one item's windows: 1, 2, 4 or 8
   int dense_interleave;    // 1: those warps take every dense_split-th chunk; 0: contiguous parts
   SceneGeom geom;          // the box of a single-scene step
@@ -184,8 +182,14 @@ struct SolverScratch {
   float* rho;
   uint32_t* flags;     // [kNumFlags] per-step flags and dense-list counters, zeroed by reorder
   uint32_t* dense;     // [dense_list_len(max_particles)] work slots handed to the dense kernels
-  uint32_t* masks;     // [kMaskWords][mask_stride] the lambda pass's neighbour masks
-  int mask_stride;     // >= particles
+  float4* xl;          // [max_particles] (position, lambda): the delta_p passes' positions
+  // one-thread-per-particle kernels only (null where no step runs them):
+  float* sa;           // [3][stride] component copies of xa and xb
+  float* sb;
+  int stride;          // particle_stride(max_particles)
+  uint32_t* hits;      // [kHitCap][hit_stride] the lambda pass's hit lists, by thread slot
+  int* hit_n;          // [hit_stride] their lengths, or a HitCode
+  int hit_stride;      // list_slots(max_particles)
   uint32_t* cell_flags;         // [max_cells + 1] CellFlag bits per cell, zeroed by reorder
   const uint32_t* keys_sorted;  // the grid's sorted cell ids (set before the passes)
   const uint32_t* cell_start;   // the grid's cell prefix (set before the passes)
@@ -223,7 +227,7 @@ struct SolverScratch {
   uint32_t* bcnt;      // [max_cells + 1] particles per current cell
   uint32_t* bstart;    // [max_cells + 1] exclusive prefix of bcnt
   uint2* bent;         // [max_particles] (current cell, rank in it) of each computing particle
-  int* bucket;         // [max_particles] the computing particles, bucket by bucket
+  int* bucket;         // [list_slots(max_particles)] the computing particles, bucket by bucket
   uint32_t* bpart;     // [kMaxScanPartials] scan partials
 };
 
@@ -274,9 +278,24 @@ inline size_t group_items(int max_particles) {
   return (size_t)max_particles / kGroupChunk + group_slots(max_particles) + 1;
 }
 
-// Neighbour masks a particle keeps between the lambda and delta_p passes of
-// one iteration: one 32-bit mask per chunk of 32 consecutive candidates.
-constexpr int kMaskWords = 16;
+// Hits a particle keeps between the lambda and delta_p passes of one
+// iteration (fluid at rest density has ~33).
+constexpr int kHitCap = 64;
+// Particle stride of the component copies and hit lists: the candidate tests
+// read aligned groups of four, so the last group may pass the last particle.
+constexpr int particle_stride(int max_particles) { return (max_particles + 7) & ~3; }
+// Slots that a cell of `count` particles takes in the paired buckets: pairs of
+// its particles, or in a step with grouped cells one particle and an empty slot
+// each.  Such a step's particles are piled up: its passes last as long as their
+// heaviest threads, which two particles one after the other would double
+// (1,048,576 particles, steps 150-160 of the sweep with the dam-break
+// parameters: 2.92 ms a step apart, 3.27 in pairs; at rest density 1.74 and
+// 1.39).
+__host__ __device__ constexpr uint32_t pair_slots(uint32_t count, bool apart) {
+  return apart ? 2u * count : (count + 1u) & ~1u;
+}
+// Slots of a pass's list; whole groups of a warp's pairs.
+constexpr size_t list_slots(int max_particles) { return (2 * (size_t)max_particles + 127) / 64 * 64; }
 
 // Words of SolverScratch::flags.  The two step flags are raised by a pass
 // when a later pass must take its exact (slow) path to reproduce the
@@ -307,8 +326,8 @@ enum ErrorBit : uint32_t {
   kErrStageTimeout = 1u,     // a shared-memory staging copy did not complete in time
 };
 
-// Largest stage (slots, 16 bytes each) a neighbour-pass block may ask for;
-// the staged pass kernels allow that much dynamic shared memory beside their
+// Largest stage (slots, 16 bytes each) a dense-kernel block may ask for; the
+// staged kernels allow that much dynamic shared memory beside their
 // hit queue (set_pass_kernel_attributes).
 constexpr int kStageMax = 4096;
 cudaError_t set_pass_kernel_attributes();
@@ -348,8 +367,10 @@ constexpr int kDefaultDenseWindow = 512;
 #endif
 constexpr int kDenseBlocksPerSm = PBF_DENSE_BLOCKS_PER_SM;
 constexpr int kDenseAllBelow = 131072;
-// Slots a block of the sparse / dense pass kernel stages in shared memory
-// (defaults; 0: no staging; pbf_autotune can override, up to kStageMax).
+// Slots a block of the dense pass kernel stages in shared memory (0: no
+// staging; pbf_autotune can override, up to kStageMax).  The tuning's
+// stage_sparse and queue_sparse are kept and have no effect: the sparse kernel
+// reads through L1 and always queues.
 constexpr int kDefaultStageSparse = 0;
 constexpr int kDefaultStageDense = 0;
 // Hit-queue capacities (chunks per thread; 1: the pair body right after each
@@ -456,8 +477,10 @@ cudaError_t backward(const BackwardArgs& args, const BackwardTape& tape, const u
                      cudaStream_t stream);
 
 // Exclusive prefix of in[0, len) into out (may alias in): 3 launches,
-// partials holds kMaxScanPartials entries.
-cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t* partials, cudaStream_t stream);
+// partials holds kMaxScanPartials entries.  groups: of pair_slots of the values,
+// apart where *groups (device) is not zero.
+cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t* partials, cudaStream_t stream,
+                           const uint32_t* groups = nullptr);
 
 // Launches (and memset nodes) of one bucketing by current cell; an ordered
 // step buckets before every lambda pass and before XSPH.

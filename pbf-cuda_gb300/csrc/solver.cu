@@ -16,10 +16,12 @@
 // Jacobi iterations ping-pong between two position buffers instead of the
 // reference's tpos -> npos copy (fluids/Simulator.cu:247-248).
 //
-// Each pass is two kernels.  The sparse kernel gives every particle one
-// thread and walks its window in a compact loop (fluid at rest: ~200
-// candidates; a window whose grouped cells -- see pbf_internal.cuh -- bring
-// it under dense_window entries is walked group by group).  A particle whose
+// Each pass is two kernels.  The sparse kernel walks a particle's window in
+// one thread (fluid at rest: ~200 candidates; a window whose grouped cells --
+// see pbf_internal.cuh -- bring it under dense_window entries is walked group
+// by group): the lambda pass lists the particle's hits, the delta_p passes of
+// the iteration read the list.  In current-cell order a thread of the lambda
+// and xsph passes takes two particles of one cell.  A particle whose
 // window still exceeds dense_window entries (particles piled into a few
 // cells) instead appends itself to a dense list; the persistent dense kernel
 // takes the list in batches of 32 particles from a counter, splits each
@@ -30,9 +32,9 @@
 // SMs idle).  Both orders are fixed, so results stay deterministic; they
 // differ from the reference's sequential sums only by rounding.  The walks
 // test chunks of 32 candidates into hit masks and run the pair body on the
-// hits, optionally through a hit queue; each kernel has a variant that
-// stages its block's column runs in shared memory by bulk asynchronous
-// copies.  Neither changes any sum.
+// hits, through a queue of masks (the dense kernel: optionally); the dense
+// kernel has a variant that stages its block's column runs in shared memory
+// by bulk asynchronous copies.  None of this changes any sum.
 //
 // Particles piled onto one position (a grouped cell's position group) have
 // bitwise the same window, position and, within a step, lambda: their lambda
@@ -75,6 +77,9 @@ constexpr int kDenseThreads = 32 * kDenseWarps;
 constexpr int kMaxFields = 6;                   // partial-sum fields of the largest pass
 constexpr unsigned kFull = 0xffffffffu;
 
+// Whether every particle takes the dense kernel.
+bool dense_for_all(const StepConsts& c, int n) { return c.dense_all >= 0 ? c.dense_all != 0 : n < kDenseAllBelow; }
+
 enum PassKind { kLambda = 0, kDeltaP = 1, kDeltaPFinal = 2, kXsph = 3 };
 
 // Everything any pass kernel needs (passed by value).
@@ -91,13 +96,21 @@ struct PassArgs {
   int dense_all;          // every warp takes the dense kernel (small n)
   uint32_t* flags;
   uint32_t* dense;
-  uint32_t* masks;        // neighbour masks: lambda saves them, delta_p reads them
-  int mask_stride;
+  // the positions by component (x at S, y at S + stride, z at S + 2 stride):
+  // the sparse kernel's candidate tests read four at a time
+  const float* S;
+  float* S_out;           // delta_p: out, beside T / npos (null when no sparse kernel runs)
+  int stride;             // of S
+  uint32_t* hits;         // hit lists: lambda writes them, delta_p reads them
+  int* hit_n;
+  int hit_stride;
   uint32_t* cell_flags;   // CellFlag bits per cell
   const uint32_t* skeys;  // stale cell of each sorted slot
   float* lambda;          // lambda: out;  delta_p: in
-  float* rho;             // lambda: out;  xsph: in
+  float4* XL;             // lambda: out, (position, lambda): the delta_p passes' X
+  float* rho;             // lambda: out;  delta_p_final and xsph: in
   float4* T;              // delta_p: out
+  float4* VR;             // (velocity, rho): delta_p_final: out;  xsph: in
   const float4* xs;       // delta_p_final: sorted x at t
   const uint32_t* iid_s;  // delta_p_final: sorted iid
   float4* npos;           // delta_p_final: out
@@ -120,6 +133,10 @@ struct PassArgs {
   const int* list;
   int count_word;
   int identity_word;
+  // the list is the buckets with every cell's on an even slot (pair_slots; an
+  // empty slot holds -1): the sparse kernel of the lambda and xsph passes takes
+  // the two slots of a pair in one thread
+  int paired;
 };
 
 // The particle that thread slot t of a pass computes (t < work_count(a)).
@@ -128,6 +145,13 @@ __device__ __forceinline__ int work_count(const PassArgs& a) {
 }
 __device__ __forceinline__ int work_particle(const PassArgs& a, int t) {
   return a.list && !(a.identity_word >= 0 && a.flags[a.identity_word]) ? __ldg(a.list + t) : t;
+}
+
+// Component copy of position x of particle i (PassArgs::S).
+__device__ __forceinline__ void put_components(float* S, int stride, int i, float4 x) {
+  S[i] = x.x;
+  S[stride + i] = x.y;
+  S[2 * (size_t)stride + i] = x.z;
 }
 
 // ---- windows ------------------------------------------------------------------------
@@ -154,27 +178,6 @@ __device__ __forceinline__ int window_total(const SceneGeom& g, const uint32_t* 
       int s, e;
       column_run(g, cs, n, x, y, q.z, s, e);
       total += e - s;
-    }
-  }
-  return total;
-}
-
-// Candidates of the window and the chunks of 32 consecutive candidates it
-// splits into (per run), from one walk over its runs.
-__device__ __forceinline__ int window_total_chunks(const SceneGeom& g, const uint32_t* __restrict__ cs, int n,
-                                                   int3 q, int& chunks) {
-  int total = 0;
-  chunks = 0;
-  for (int dx = -1; dx <= 1; ++dx) {
-    const int x = q.x + dx;
-    if (x < 0 || x >= g.dims[0]) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = q.y + dy;
-      if (y < 0 || y >= g.dims[1]) continue;
-      int s, e;
-      column_run(g, cs, n, x, y, q.z, s, e);
-      total += e - s;
-      chunks += (e - s + 31) >> 5;
     }
   }
   return total;
@@ -261,9 +264,10 @@ __device__ __forceinline__ void visit_window(const SceneGeom& g, const uint32_t*
 // loop, so the warp pays max-over-lanes of the hits of the whole queued span.
 // Hits are visited in the order they were queued -- the window's visiting
 // order -- so the sums are bitwise those of visiting each chunk's hits right
-// away.  The capacity (chunks queued per thread before a flush) comes from
-// the step's tuning (StepConsts::queue_sparse / queue_dense); capacity 1 runs
-// each chunk's hits right away, straight from registers.
+// away.  The dense kernel's capacity (chunks queued per thread before a flush)
+// comes from the step's tuning (StepConsts::queue_dense); capacity 1 runs
+// each chunk's hits right away, straight from registers.  The sparse kernel
+// has a queue of its own (QueueColumn).
 struct HitQueue {
   uint32_t* mask;  // this thread's column: entry k at mask[k * stride]
   int* base;       // where queued chunk k starts (Src::tag)
@@ -353,21 +357,12 @@ __device__ __forceinline__ void visit_run(const Src& src, int j0, int j1, int r,
   }
 }
 
-// Every candidate of the window, in order, in two stages per chunk of 32
-// consecutive slots of a run: a cheap test p.hit() of each candidate (four
-// loads in flight) into a bit mask, then p.visit() on the set bits in
-// ascending order, through the hit queue.  p.visit() leaves non-hits
-// untouched, so the result is that of visit_window.
-//
-// save_masks: store chunk k's mask at masks[k * stride + i] (k < kMaskWords;
-// i: the particle's mask slot) for the next pass over the same positions.
+// Every candidate of the window, in order: a hit mask per chunk of 32
+// consecutive slots of a run, p.visit() on the set bits.  p.visit() leaves
+// non-hits untouched, so the result is that of visit_window.
 template <class P, class Src>
-__device__ __forceinline__ void visit_window_masked(const SceneGeom& g,
-                                                    const uint32_t* __restrict__ cs, int n,
-                                                    int3 q, const Src& src, P& p,
-                                                    uint32_t* __restrict__ masks, int stride,
-                                                    int i, HitQueue& hq) {
-  int chunk = 0;
+__device__ __forceinline__ void visit_window_masked(const SceneGeom& g, const uint32_t* __restrict__ cs, int n,
+                                                    int3 q, const Src& src, P& p, HitQueue& hq) {
   for (int dx = -1; dx <= 1; ++dx) {
     const int x = q.x + dx;
     if (x < 0 || x >= g.dims[0]) continue;
@@ -377,47 +372,7 @@ __device__ __forceinline__ void visit_window_masked(const SceneGeom& g,
       const int r = 3 * (dx + 1) + (dy + 1);
       int s, e;
       column_run(g, cs, n, x, y, q.z, s, e);
-      for (int j0 = s; j0 < e; j0 += 32) {
-        const uint32_t mask = chunk_mask(src, j0, e, r, p);
-        if (masks && chunk < kMaskWords) masks[chunk * stride + i] = mask;
-        ++chunk;
-        hq.push(mask, src.tag(j0, r), src, p);
-      }
-    }
-  }
-  hq.flush(src, p);
-}
-
-// The window's neighbours from the masks a previous pass over the same
-// positions saved (visit_window_masked with save): p.visit() on the set bits,
-// in order, through the hit queue.  The saved hits are a superset of p's
-// (p.visit re-tests).
-// chunks: the window's chunk count (at most kMaskWords); each chunk's mask is
-// loaded two chunks ahead of its use, so its latency overlaps the pair work.
-template <class P, class Src>
-__device__ __forceinline__ void visit_window_saved(const SceneGeom& g,
-                                                   const uint32_t* __restrict__ cs, int n, int3 q,
-                                                   const Src& src, P& p,
-                                                   const uint32_t* __restrict__ masks, int stride,
-                                                   int i, int chunks, HitQueue& hq) {
-  int chunk = 0;
-  uint32_t m0 = chunks > 0 ? __ldg(masks + i) : 0u;
-  uint32_t m1 = chunks > 1 ? __ldg(masks + stride + i) : 0u;
-  for (int dx = -1; dx <= 1; ++dx) {
-    const int x = q.x + dx;
-    if (x < 0 || x >= g.dims[0]) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = q.y + dy;
-      if (y < 0 || y >= g.dims[1]) continue;
-      const int r = 3 * (dx + 1) + (dy + 1);
-      int s, e;
-      column_run(g, cs, n, x, y, q.z, s, e);
-      for (int j0 = s; j0 < e; j0 += 32, ++chunk) {
-        const uint32_t m = m0;
-        m0 = m1;
-        m1 = chunk + 2 < chunks ? __ldg(masks + (chunk + 2) * stride + i) : 0u;
-        hq.push(m, src.tag(j0, r), src, p);
-      }
+      visit_run(src, s, e, r, p, true, hq);
     }
   }
   hq.flush(src, p);
@@ -574,6 +529,50 @@ __device__ __forceinline__ void visit_window_grouped(const SceneGeom& g, const P
 
 // ---- the passes: per-candidate visit, partial-sum fields, finish ----------------------
 
+// Two floats in one register pair: packed arithmetic rounds each as the scalar
+// operation does and takes one issue slot for both.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 dist2_2(f32x2 ex, f32x2 ey, f32x2 ez) {
+  return fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
+}
+
+// rsqrtf of a normal number (bitwise the same there, without the scaling of
+// subnormal arguments; a zero gives +inf).
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 struct LambdaPass {
   static constexpr int kFields = 5;
   static constexpr int kGroupUnroll = 2;
@@ -593,19 +592,54 @@ struct LambdaPass {
   __device__ __forceinline__ void visit(float4 xj, int j) {
     const float ex = xi.x - xj.x, ey = xi.y - xj.y, ez = xi.z - xj.z;
     const float r2 = dist2(ex, ey, ez);
-    if (!(r2 >= c.h2)) {  // NaN-inclusive, as getPoly6
-      pho += poly6_inside(c, r2);
-      if (!(r2 < c.keps2)) {  // as getSpikyGrad's |r| < KERNAL_EPS test
-        const float ir = rsqrtf(r2);
-        const float t = c.h - r2 * ir;
-        const float sc = c.spiky_coef_rho0 * t * t * ir;
-        const float ax = sc * ex, ay = sc * ey, az = sc * ez;
-        gx += ax;
-        gy += ay;
-        gz += az;
-        if (j != i) gl2 += dist2(ax, ay, az);
-      }
+    if (!(r2 >= c.h2)) pair(ex, ey, ez, r2, j);  // NaN-inclusive, as getPoly6
+  }
+  __device__ __forceinline__ void pair(float ex, float ey, float ez, float r2, int j) {
+    pho += poly6_inside(c, r2);
+    if (!(r2 < c.keps2)) {  // as getSpikyGrad's |r| < KERNAL_EPS test
+      const float ir = rsqrtf(r2);
+      const float t = c.h - r2 * ir;
+      const float sc = c.spiky_coef_rho0 * t * t * ir;
+      const float ax = sc * ex, ay = sc * ey, az = sc * ez;
+      gx += ax;
+      gy += ay;
+      gz += az;
+      if (j != i) gl2 += dist2(ax, ay, az);
     }
+  }
+  // Two particles at r2 < h2, a then b (b only if `two`), keps2 > 0: pair() of
+  // each.  Below keps2 (i itself among them) the gradient's factor is zero,
+  // which adds nothing to the sums.
+  __device__ __forceinline__ void visit_two(float4 xa, float4 xb, float4, float4, bool two) {
+    const f32x2 ex = sub2(both(xi.x), pack2(xa.x, xb.x)), ey = sub2(both(xi.y), pack2(xa.y, xb.y)),
+                ez = sub2(both(xi.z), pack2(xa.z, xb.z));
+    const f32x2 r2 = dist2_2(ex, ey, ez);
+    float ra, rb;
+    unpack2(r2, ra, rb);
+    const f32x2 d = sub2(both(c.h2), r2);
+    const f32x2 w = mul2(mul2(both(c.poly6_coef), d), d);
+    const f32x2 ir = pack2(rsqrt_normal(ra), rsqrt_normal(rb));
+    const f32x2 t = fma2(r2, ir, both(-c.h));  // -(h - |r|); its sign cancels in t t
+    const f32x2 scu = mul2(mul2(mul2(both(c.spiky_coef_rho0), t), t), ir);
+    float sa, sb, wa, wb, da, db;
+    unpack2(scu, sa, sb);
+    unpack2(w, wa, wb);
+    unpack2(d, da, db);
+    sa = ra < c.keps2 ? 0.f : sa;
+    sb = rb < c.keps2 || !two ? 0.f : sb;
+    wb = two ? wb : 0.f;
+    const f32x2 sc = pack2(sa, sb);
+    const f32x2 ax = mul2(sc, ex), ay = mul2(sc, ey), az = mul2(sc, ez);
+    const f32x2 l = dist2_2(ax, ay, az);
+    float xa_, xb_, ya_, yb_, za_, zb_, la, lb;
+    unpack2(l, la, lb);
+    pho = fmaf(wa, da, pho);
+    pho = fmaf(wb, db, pho);
+    unpack2(ax, xa_, xb_), unpack2(ay, ya_, yb_), unpack2(az, za_, zb_);
+    gx += xa_, gy += ya_, gz += za_;
+    gx += xb_, gy += yb_, gz += zb_;
+    gl2 += la;
+    gl2 += lb;
   }
   // `cnt` particles at xg.  The group holding i itself lies at r2 = 0 <
   // keps2 (grouping needs keps2 > 0): no gradient, as the reference's j != i.
@@ -640,6 +674,7 @@ struct LambdaPass {
     const float lam = -(rho / c.pho0 - 1.f) / (grad_l2 + c.lambda_eps);
     a.lambda[i] = lam;
     a.rho[i] = rho;
+    a.XL[i] = make_float4(xi.x, xi.y, xi.z, lam);
     const uint32_t bits = (isfinite(lam) ? 0u : (uint32_t)kCellLambdaNonFinite) |
                           (rho > 0.f && isfinite(rho) ? 0u : (uint32_t)kCellRhoNotPositive);
     if (bits) {
@@ -659,8 +694,7 @@ struct DeltaPPass {
   static constexpr int kGroupUnroll = 2;
   const StepConsts& c;
   const SceneGeom& g;
-  const float* __restrict__ lambda;
-  float4 xi;
+  float4 xi;  // positions come with their lambda in w (PassArgs::XL)
   int i;
   float li;
   bool exact;
@@ -668,31 +702,64 @@ struct DeltaPPass {
   bool poison = false;
 
   __device__ DeltaPPass(const PassArgs& a, const SceneGeom& g_, float4 xi_, int i_, bool exact_)
-      : c(a.c), g(g_), lambda(a.lambda), xi(xi_), i(i_), li(a.lambda[i_]), exact(exact_) {}
+      : c(a.c), g(g_), xi(xi_), i(i_), li(xi_.w), exact(exact_) {}
   __device__ __forceinline__ bool skip_misses() const { return !exact; }
   __device__ __forceinline__ bool hit(float4 xj, int j) const {
     const float r2 = dist2(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
     return !(r2 >= c.h2) && !(r2 < c.keps2) && j != i;
   }
   __device__ __forceinline__ void visit(float4 xj, int j) {
-    // lambda_j first: its load overlaps the distance test (a visited candidate
-    // is almost always a neighbour, so the load is rarely wasted)
-    const float lj = __ldg(lambda + j);
     const float ex = xi.x - xj.x, ey = xi.y - xj.y, ez = xi.z - xj.z;
     const float r2 = dist2(ex, ey, ez);
     if (!(r2 >= c.h2) && !(r2 < c.keps2) && j != i) {  // NaN-inclusive, as the reference
-      const float wgt = poly6_inside(c, r2);
-      const float corr = c.coef_corr * pow_corr(c, wgt);
-      const float ir = rsqrtf(r2);
-      const float t = c.h - r2 * ir;
-      const float f = (li + lj + corr) * (c.spiky_coef * t * t * ir);
-      ax = fmaf(f, ex, ax);
-      ay = fmaf(f, ey, ay);
-      az = fmaf(f, ez, az);
+      pair(ex, ey, ez, r2, xj.w);
     } else if (exact && j != i) {
       // zero gradient: (lambda_i + lambda_j + s_corr) * 0 is NaN iff a lambda is not finite
-      poison |= !isfinite(li) || !isfinite(lj);
+      poison |= !isfinite(li) || !isfinite(xj.w);
     }
+  }
+  // Two particles at r2 < h2, a then b, keps2 > 0, not on the exact path:
+  // pair() of each.  Below keps2 (i itself among them) the factor is zero,
+  // which adds nothing to the sums.
+  __device__ __forceinline__ void visit_two(float4 xa, float4 xb, float4, float4, bool two) {
+    const f32x2 ex = sub2(both(xi.x), pack2(xa.x, xb.x)), ey = sub2(both(xi.y), pack2(xa.y, xb.y)),
+                ez = sub2(both(xi.z), pack2(xa.z, xb.z));
+    const f32x2 r2 = dist2_2(ex, ey, ez);
+    float ra, rb;
+    unpack2(r2, ra, rb);
+    const f32x2 d = sub2(both(c.h2), r2);
+    const f32x2 w = mul2(mul2(mul2(both(c.poly6_coef), d), d), d);
+    f32x2 pw;
+    if (c.npow == 4) {
+      const f32x2 w2 = mul2(w, w);
+      pw = mul2(w2, w2);
+    } else {
+      float wa, wb;
+      unpack2(w, wa, wb);
+      pw = pack2(pow_corr(c, wa), pow_corr(c, wb));
+    }
+    const f32x2 ll = add2(both(li), pack2(xa.w, xb.w));
+    const f32x2 lc = fma2(both(c.coef_corr), pw, ll);
+    const f32x2 ir = pack2(rsqrt_normal(ra), rsqrt_normal(rb));
+    const f32x2 t = fma2(r2, ir, both(-c.h));  // -(h - |r|); its sign cancels in t t
+    const f32x2 f = mul2(lc, mul2(mul2(mul2(both(c.spiky_coef), t), t), ir));
+    float fa, fb, xa_, xb_, ya_, yb_, za_, zb_;
+    unpack2(f, fa, fb);
+    fa = ra < c.keps2 ? 0.f : fa;
+    fb = rb < c.keps2 || !two ? 0.f : fb;
+    unpack2(ex, xa_, xb_), unpack2(ey, ya_, yb_), unpack2(ez, za_, zb_);
+    ax = fmaf(fa, xa_, ax), ay = fmaf(fa, ya_, ay), az = fmaf(fa, za_, az);
+    ax = fmaf(fb, xb_, ax), ay = fmaf(fb, yb_, ay), az = fmaf(fb, zb_, az);
+  }
+  __device__ __forceinline__ void pair(float ex, float ey, float ez, float r2, float lj) {
+    const float wgt = poly6_inside(c, r2);
+    const float corr = c.coef_corr * pow_corr(c, wgt);
+    const float ir = rsqrtf(r2);
+    const float t = c.h - r2 * ir;
+    const float f = (li + lj + corr) * (c.spiky_coef * t * t * ir);
+    ax = fmaf(f, ex, ax);
+    ay = fmaf(f, ey, ay);
+    az = fmaf(f, ez, az);
   }
   // `cnt` particles at xg with lambda_j summing to cnt sum.x + sum.y (each
   // lambda_j - sum.x finite, or lambda_j the same bits as sum.x).  exact: the
@@ -734,7 +801,8 @@ struct DeltaPPass {
     const float dz = fmaxf(fminf(sz / c.pho0, c.max_dp), -c.max_dp);
     const float4 xf = make_float4(fmaxf(fminf(xi.x + dx, g.hi[0]), g.lo[0]),
                                   fmaxf(fminf(xi.y + dy, g.hi[1]), g.lo[1]),
-                                  fmaxf(fminf(xi.z + dz, g.hi[2]), g.lo[2]), xi.w);
+                                  fmaxf(fminf(xi.z + dz, g.hi[2]), g.lo[2]), 0.f);
+    if (a.S_out) put_components(a.S_out, a.stride, i, xf);
     if (!kFinal) {
       a.T[i] = xf;
       return;
@@ -746,6 +814,7 @@ struct DeltaPPass {
     const float4 v = make_float4((xf.x - x0.x) * c.inv_dt, (xf.y - x0.y) * c.inv_dt,
                                  (xf.z - x0.z) * c.inv_dt, 0.f);
     a.vel[i] = v;
+    a.VR[i] = make_float4(v.x, v.y, v.z, a.rho[i]);
     if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z)) {
       atomicOr(&a.cell_flags[a.skeys[i]], (uint32_t)kCellVelNonFinite);
       atomicOr(&a.flags[kFlagXsphExact], 1u);
@@ -761,8 +830,7 @@ struct XsphPass {
   static constexpr int kFields = 6;
   static constexpr int kGroupUnroll = 2;
   const StepConsts& c;
-  const float4* __restrict__ V;
-  const float* __restrict__ rho;
+  const float4* __restrict__ VR;  // (velocity, rho)
   float4 xi, vi;
   float ri;
   int i;
@@ -771,31 +839,38 @@ struct XsphPass {
   bool px = false, py = false, pz = false;
 
   __device__ XsphPass(const PassArgs& a, const SceneGeom&, float4 xi_, int i_, bool exact_)
-      : c(a.c), V(a.V), rho(a.rho), xi(xi_), vi(a.V[i_]), ri(a.rho[i_]), i(i_), exact(exact_) {}
+      : c(a.c), VR(a.VR), xi(xi_), vi(a.VR[i_]), ri(vi.w), i(i_), exact(exact_) {}
   __device__ __forceinline__ bool skip_misses() const { return !exact; }
   __device__ __forceinline__ bool hit(float4 xj, int) const {
     return !(dist2(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z) >= c.h2);
   }
   __device__ __forceinline__ void visit(float4 xj, int j) {
-    // v_j and rho_j first: their loads overlap the distance test (a visited
+    // v_j and rho_j first: their load overlaps the distance test (a visited
     // candidate is almost always a neighbour)
-    const float4 vj = __ldg(V + j);
-    const float rj = __ldg(rho + j);
+    const float4 vj = __ldg(VR + j);
     const float r2 = dist2(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
     if (!(r2 >= c.h2)) {  // NaN-inclusive, as getPoly6
-      const float w2 = 2.f * poly6_inside(c, r2) / (ri + rj);
-      ax = fmaf(vj.x - vi.x, w2, ax);
-      ay = fmaf(vj.y - vi.y, w2, ay);
-      az = fmaf(vj.z - vi.z, w2, az);
+      pair(vj, r2);
     } else if (exact) {
       // W = 0: 2 (v_j - v_i) * 0 / (rho_i + rho_j) is NaN iff the velocity
       // difference is not finite or the denominator is 0 or NaN
-      const float den = ri + rj;
+      const float den = ri + vj.w;
       const bool bad_den = !(den != 0.f) || isnan(den);
       px |= bad_den || !isfinite(vj.x - vi.x);
       py |= bad_den || !isfinite(vj.y - vi.y);
       pz |= bad_den || !isfinite(vj.z - vi.z);
     }
+  }
+  // Two particles at r2 < h2, a then b (b only if `two`), not on the exact path.
+  __device__ __forceinline__ void visit_two(float4 xa, float4 xb, float4 va, float4 vb, bool two) {
+    pair(va, dist2(xi.x - xa.x, xi.y - xa.y, xi.z - xa.z));
+    if (two) pair(vb, dist2(xi.x - xb.x, xi.y - xb.y, xi.z - xb.z));
+  }
+  __device__ __forceinline__ void pair(float4 vj, float r2) {
+    const float w2 = 2.f * poly6_inside(c, r2) / (ri + vj.w);
+    ax = fmaf(vj.x - vi.x, w2, ax);
+    ay = fmaf(vj.y - vi.y, w2, ay);
+    az = fmaf(vj.z - vi.z, w2, az);
   }
   // `cnt` particles at xg sharing the density sum.w and the velocity aux.xyz
   // (sum.xyz: the sum over the group of v_j - aux.xyz, zero for the groups
@@ -1032,25 +1107,6 @@ __device__ __forceinline__ void stage_drain(StageState& st, uint32_t phase) {
 
 // ---- kernels ------------------------------------------------------------------------
 
-// The plain (not grouped) walk of a sparse-kernel particle's window.
-// t: the particle's thread slot in the pass's list, which indexes its saved
-// masks (the lambda and delta_p passes of an iteration take the same list, so
-// a particle keeps its slot; consecutive threads then store and load
-// consecutive words).
-template <int kKind, class P, class Src>
-__device__ __forceinline__ void sparse_visit(const PassArgs& a, const SceneGeom& g, int3 q, const Src& src,
-                                             P& p, bool exact, int t, int chunks, HitQueue& hq) {
-  if (exact) {
-    visit_window(g, a.cs, a.n, q, src, p);  // non-neighbours matter: visit every candidate
-  } else if (kKind == kLambda) {
-    visit_window_masked(g, a.cs, a.n, q, src, p, a.masks, a.mask_stride, t, hq);  // saves its masks
-  } else if ((kKind == kDeltaP || kKind == kDeltaPFinal) && chunks <= kMaskWords) {
-    visit_window_saved(g, a.cs, a.n, q, src, p, a.masks, a.mask_stride, t, chunks, hq);  // lambda's masks
-  } else {
-    visit_window_masked(g, a.cs, a.n, q, src, p, nullptr, 0, t, hq);
-  }
-}
-
 // The stage's barrier, before first use (thread 0).
 __device__ __forceinline__ void stage_init(StageState& st) {
   st.failed = 0;
@@ -1059,8 +1115,362 @@ __device__ __forceinline__ void stage_init(StageState& st) {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// One thread slot of the work list (or of all particles) per thread; the
-// grid covers every particle, blocks past the list's end return at once.
+// ---- hits of a window -------------------------------------------------------------------
+//
+// The sparse kernel's walk.  Candidates are tested four at a time on the
+// component copies of the positions (three 16-byte loads, two candidates to a
+// packed float instruction, rounded as dist2 rounds), and the sign of r2 - h2
+// is shifted into a hit mask, so a test costs no compare, no select and no
+// branch.  Runs start anywhere, so the groups start at the run's start rounded
+// down to four and the mask drops what lies outside the run.  Non-empty masks
+// are queued in shared memory and one flat loop visits the window's hits at
+// the end: a warp then iterates as often as its busiest lane has hits in the
+// whole window (~42 at rest density for 33 on average), not the sum over the
+// chunks of the busiest lane of each (~72).  Visiting order: slots ascending
+// in each run, runs in order -- the reference's.  The visits take two hits at
+// a time in packed arithmetic, rounded as pair() rounds them.
+//
+// This holds with kernel_eps a normal number (fast_hits) and for a particle at
+// a finite position (a NaN one would meet itself); others take
+// visit_window_masked.
+
+// The sign bits of d, the lower half's first.
+__device__ __forceinline__ uint32_t shift_in(uint32_t mask, f32x2 d) {
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(d));
+  return __funnelshift_l(hi, __funnelshift_l(lo, mask, 1), 1);
+}
+
+// The component copies of candidates j .. j + 3 (j a multiple of 4).
+struct Four {
+  ulonglong2 x, y, z;
+  __device__ __forceinline__ Four(const float* __restrict__ S, int stride, int j)
+      : x(__ldg(reinterpret_cast<const ulonglong2*>(S + j))),
+        y(__ldg(reinterpret_cast<const ulonglong2*>(S + stride + j))),
+        z(__ldg(reinterpret_cast<const ulonglong2*>(S + 2 * (size_t)stride + j))) {}
+};
+
+// The window's centre, negated, and the largest float below h2, twice each:
+// r2 is a hit when that minus r2 has no sign bit, i.e. when r2 < h2 or r2 is
+// NaN (a NaN result has none), the reference's !(r2 >= h2).
+struct HitTest {
+  f32x2 x, y, z, h;
+  __device__ __forceinline__ HitTest(float4 xi, float h2)
+      : x(both(-xi.x)), y(both(-xi.y)), z(both(-xi.z)),
+        h(both(below(h2))) {}
+  static __device__ __forceinline__ float below(float h2) {
+    return h2 > 0.f ? __uint_as_float(__float_as_uint(h2) - 1u) : -1.f;
+  }
+  __device__ __forceinline__ f32x2 pair(f32x2 px, f32x2 py, f32x2 pz) const {
+    return sub2(h, dist2_2(add2(px, x), add2(py, y), add2(pz, z)));
+  }
+  // the four's miss bits shifted into mask
+  __device__ __forceinline__ uint32_t four(const Four& f, uint32_t mask) const {
+    mask = shift_in(mask, pair(f.x.x, f.y.x, f.z.x));
+    return shift_in(mask, pair(f.x.y, f.y.y, f.z.y));
+  }
+};
+
+// A thread's column of shared memory: the queue grows from entry 0, the
+// window's runs [s, e) wait in entries kRunSlot.. until they are walked.
+// Queue entry k: the chunk's mask and its first slot in run[k], and, where two
+// particles share the walk, the second one's mask in second[k].
+constexpr int kQueueSlots = 12;
+constexpr int kRunSlot = kQueueSlots - 9;
+struct QueueColumn {
+  uint2* run;
+  uint32_t* second;
+};
+
+// The hits of one particle in queue entries [0, n), one after the other; the
+// caller counts them.
+template <bool kSecond>
+struct QueuedHits {
+  QueueColumn q;
+  uint32_t m = 0u;
+  int base = 0;
+  __device__ __forceinline__ explicit QueuedHits(QueueColumn q_) : q(q_) {}
+  __device__ __forceinline__ int next() {
+    while (!m) {  // (an entry of a pair may hold hits of the other particle only)
+      if (kSecond) {
+        m = *q.second;
+        base = (int)q.run->y;
+      } else {
+        const uint2 e = *q.run;
+        m = e.x;
+        base = (int)e.y;
+      }
+      q.run += kSparseThreads;
+      q.second += kSparseThreads;
+    }
+    const int bit = __clz(m);  // the first candidate is the highest bit
+    m ^= 0x80000000u >> bit;
+    return base + bit;
+  }
+};
+
+// Visits `hits` queued hits in order, two at a time, each two's loads issued
+// two ahead.  out: where the lambda pass lists them (null: nowhere).
+template <int kKind, bool kSecond, class P>
+__device__ __forceinline__ void visit_queued(const PassArgs& a, QueueColumn q, int hits, P& p, uint32_t* out) {
+  if (hits == 0) return;
+  QueuedHits<kSecond> h(q);
+  float4 xa, xb, va = make_float4(0.f, 0.f, 0.f, 0.f), vb = va;
+  // the next two hits (the second one the first again when only one is left)
+  auto fetch = [&](int left) {
+    const int ja = h.next(), jb = left > 1 ? h.next() : ja;
+    xa = __ldg(a.X + ja);
+    xb = __ldg(a.X + jb);
+    if constexpr (kKind == kXsph) {
+      va = __ldg(a.VR + ja);
+      vb = __ldg(a.VR + jb);
+    } else if (out) {
+      out[0] = (uint32_t)ja;
+      out[a.hit_stride] = (uint32_t)jb;  // (the last one twice: past the list's length)
+      out += 2 * (size_t)a.hit_stride;
+    }
+  };
+  fetch(hits);
+  for (; hits > 0; hits -= 2) {
+    const float4 x0 = xa, x1 = xb, v0 = va, v1 = vb;
+    if (hits > 2) fetch(hits - 2);
+    p.visit_two(x0, x1, v0, v1, hits > 1);
+  }
+}
+
+// Codes of PassArgs::hit_n besides a list's length.
+enum HitCode : int {
+  kHitsDense = -1,  // the particle went to the dense kernel
+  kHitsWalk = -2,   // no list: the delta_p passes walk the window again
+  kHitsMasks = -3,  // kHitsMasks - k: k chunks with hits (mask, first slot) in place of the list
+};
+
+// Chunk k with hits of list slot h.
+__device__ __forceinline__ void put_chunk(const PassArgs& a, int h, int k, uint32_t m, uint32_t base) {
+  uint32_t* out = a.hits + 2 * (size_t)k * a.hit_stride + h;
+  out[0] = m;
+  out[a.hit_stride] = base;
+}
+
+// Visits the hits of one chunk in order, two at a time.
+template <int kKind, class P>
+__device__ __forceinline__ void visit_mask(const PassArgs& a, uint32_t m, int base, P& p) {
+  while (m) {
+    const int ba = __clz(m), ja = base + ba;
+    m ^= 0x80000000u >> ba;
+    const bool two = m != 0u;
+    const int bb = two ? __clz(m) : ba, jb = base + bb;
+    if (two) m ^= 0x80000000u >> bb;
+    const float4 xa = __ldg(a.X + ja), xb = __ldg(a.X + jb);
+    if constexpr (kKind == kXsph)
+      p.visit_two(xa, xb, __ldg(a.VR + ja), __ldg(a.VR + jb), two);
+    else
+      p.visit_two(xa, xb, xa, xb, two);
+  }
+}
+
+// The chunks (up to 32 candidates from a multiple of four) of run r of the
+// window, in order: f(base, groups of four, the candidates that belong to it).
+template <class F>
+__device__ __forceinline__ void for_chunks(uint2 run, F&& f) {
+  const int s = (int)run.x, e = (int)run.y;
+  uint32_t valid = 0xffffffffu >> (s & 3);  // drops candidates before s from the first mask
+  for (int base = s & ~3; base < e; base += 32) {
+    if (e - base < 32) valid &= ~(0xffffffffu >> (e - base));
+    f(base, min((e - base + 3) >> 2, 8), valid);
+    valid = 0xffffffffu;
+  }
+}
+
+// Visits the queued hits (n entries) of one particle; returns the code of list
+// slot h, which the lambda pass fills: the hits, or where a warp has a particle
+// with more than fit its chunks (so that the delta_p pass's warps take one path).
+template <int kKind, bool kSecond, class P>
+__device__ __forceinline__ int finish_queued(const PassArgs& a, QueueColumn col, int n, int hits, P& p, int h) {
+  const bool list = kKind == kLambda && __all_sync(__activemask(), hits <= kHitCap);
+  visit_queued<kKind, kSecond>(a, col, hits, p, list ? a.hits + h : nullptr);
+  if (kKind != kLambda || list) return hits;
+  int chunks = 0;
+  for (int k = 0; k < n; ++k) {
+    const uint2 e = col.run[k * kSparseThreads];
+    const uint32_t m = kSecond ? col.second[k * kSparseThreads] : e.x;
+    if (m) put_chunk(a, h, chunks++, m, e.y);
+  }
+  return kHitsMasks - chunks;
+}
+
+// The hits of the window whose runs are in the column, visited in order;
+// returns the code of list slot h (lambda).  fits: the queue takes the whole
+// window (window_runs).  A window of more chunks is one of piled-up particles,
+// whose chunks hold many hits each: they are visited chunk by chunk, straight
+// from the mask.
+template <int kKind, class P>
+__device__ __forceinline__ int walk_hits(const PassArgs& a, QueueColumn col, P& p, int h, bool fits) {
+  const HitTest test(p.xi, a.c.h2);
+  int n = 0, hits = 0;
+  for (int r = 0; r < 9; ++r) {
+    for_chunks(col.run[(kRunSlot + r) * kSparseThreads], [&](int base, int groups, uint32_t valid) {
+      uint32_t m = 0u;
+#pragma unroll 2
+      for (int g = 0; g < groups; ++g) m = test.four(Four(a.S, a.stride, base + 4 * g), m);
+      m = ~m << (32 - 4 * groups) & valid;  // hits, the first candidate in the highest bit
+      if (!m) return;
+      if (fits) {
+        col.run[n * kSparseThreads] = make_uint2(m, (uint32_t)base);
+        hits += __popc(m);
+      } else {
+        if (kKind == kLambda && n < kHitCap / 2) put_chunk(a, h, n, m, (uint32_t)base);
+        visit_mask<kKind>(a, m, base, p);
+      }
+      ++n;
+    });
+  }
+  if (fits) return finish_queued<kKind, false>(a, col, n, hits, p, h);
+  return kKind == kLambda && n <= kHitCap / 2 ? kHitsMasks - n : (int)kHitsWalk;
+}
+
+// The same walk for two particles of one cell, up to the queue: the masks of
+// both (run.x, second); returns the entries and the hits of each.  The caller
+// has checked that the window's chunks fit (window_runs).
+__device__ __forceinline__ int3 queue_pair(const PassArgs& a, QueueColumn col, float4 x0, float4 x1) {
+  const HitTest t0(x0, a.c.h2), t1(x1, a.c.h2);
+  int n = 0;
+  int3 hits = make_int3(0, 0, 0);
+  for (int r = 0; r < 9; ++r) {
+    for_chunks(col.run[(kRunSlot + r) * kSparseThreads], [&](int base, int groups, uint32_t valid) {
+      uint32_t m0 = 0u, m1 = 0u;
+#pragma unroll 2
+      for (int g = 0; g < groups; ++g) {
+        const Four f(a.S, a.stride, base + 4 * g);
+        m0 = t0.four(f, m0);
+        m1 = t1.four(f, m1);
+      }
+      const int sh = 32 - 4 * groups;
+      m0 = ~m0 << sh & valid;
+      m1 = ~m1 << sh & valid;
+      if (m0 | m1) {
+        col.run[n * kSparseThreads] = make_uint2(m0, (uint32_t)base);
+        col.second[n * kSparseThreads] = m1;
+        ++n;
+        hits.x += __popc(m0);
+        hits.y += __popc(m1);
+      }
+    });
+  }
+  hits.z = n;
+  return hits;
+}
+
+// Visits the first n particles of a hit list in order, kListAhead loads in
+// flight (the last batch is filled up with the particle itself, which adds
+// nothing).
+constexpr int kListAhead = 4;
+template <class P>
+__device__ __forceinline__ void visit_list(const PassArgs& a, const uint32_t* __restrict__ list, int n, int i, P& p) {
+  int j[kListAhead];
+#pragma unroll
+  for (int u = 0; u < kListAhead; ++u) j[u] = u < n ? (int)__ldg(list + (size_t)u * a.hit_stride) : i;
+  for (int k = 0; k < n; k += kListAhead) {
+    float4 x[kListAhead];
+#pragma unroll
+    for (int u = 0; u < kListAhead; ++u) x[u] = __ldg(a.X + j[u]);
+    list += (size_t)kListAhead * a.hit_stride;
+#pragma unroll
+    for (int u = 0; u < kListAhead; ++u)
+      j[u] = k + kListAhead + u < n ? (int)__ldg(list + (size_t)u * a.hit_stride) : i;
+#pragma unroll
+    for (int u = 0; u < kListAhead; u += 2) p.visit_two(x[u], x[u + 1], x[u], x[u + 1], true);
+  }
+}
+
+// Visits the hits of the n chunks that took the list's place, the next chunk's
+// load issued one ahead.
+template <int kKind, class P>
+__device__ __forceinline__ void visit_chunks(const PassArgs& a, const uint32_t* __restrict__ list, int n, P& p) {
+  if (n == 0) return;
+  uint32_t m = __ldg(list), base = __ldg(list + a.hit_stride);
+  for (int k = 1; k <= n; ++k) {
+    list += 2 * (size_t)a.hit_stride;
+    const uint32_t mn = k < n ? __ldg(list) : 0u, bn = k < n ? __ldg(list + a.hit_stride) : 0u;
+    visit_mask<kKind>(a, m, (int)base, p);
+    m = mn;
+    base = bn;
+  }
+}
+
+// Whether walk_hits and the hit lists hold for a particle at xi: keps2 a normal
+// number (a pair below it has no gradient; rsqrt_normal), xi finite.
+__device__ __forceinline__ bool fast_hits(const PassArgs& a, float4 xi) {
+  return a.c.keps2 >= 1.17549435e-38f && isfinite(xi.x) && isfinite(xi.y) && isfinite(xi.z);
+}
+
+// The 9 column runs of the window of cell q into the column; returns the
+// candidates they hold.  Every load is issued before the first is used.
+// fits: the chunks of any prefix of the runs fit the queue entries that are
+// free by then.
+__device__ __forceinline__ int window_runs(const SceneGeom& g, const uint32_t* __restrict__ cs, int n, int3 q,
+                                           QueueColumn col, bool& fits) {
+  const int zlo = max(q.z - 1, 0), zhi = min(q.z + 1, g.dims[2] - 1);
+  uint32_t s[9], e[9];
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const int x = q.x + r / 3 - 1, y = q.y + r % 3 - 1;
+    const bool in = x >= 0 && x < g.dims[0] && y >= 0 && y < g.dims[1];
+    const int base = g.cell_base + (x * g.dims[1] + y) * g.dims[2];
+    s[r] = in ? __ldg(cs + base + zlo) : 0u;
+    e[r] = in ? __ldg(cs + base + zhi + 1) : 0u;
+  }
+  int total = 0, chunks = 0;
+  fits = true;
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const int end = max(min((int)e[r], n), (int)s[r]);  // as column_run
+    col.run[(kRunSlot + r) * kSparseThreads] = make_uint2(s[r], (uint32_t)end);
+    total += end - (int)s[r];
+    chunks += end > (int)s[r] ? (end - (int)(s[r] & ~3u) + 31) >> 5 : 0;
+    fits = fits && chunks <= kRunSlot + r + 1;
+  }
+  return total;
+}
+
+// Appends the first `count` (0, 1 or 2) of slots t, t + 1 of every lane to the
+// dense list, in slot order (one atomic per warp; every lane of the warp calls
+// it).
+__device__ __forceinline__ void append_dense(const PassArgs& a, int count, int t) {
+  const unsigned one = __ballot_sync(kFull, count > 0), two = __ballot_sync(kFull, count > 1);
+  if (!one) return;
+  const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+  uint32_t base = 0u;
+  if (lane == 0) base = atomicAdd(&a.flags[a.counter], (uint32_t)(__popc(one) + __popc(two)));
+  base = __shfl_sync(kFull, base, 0) + (uint32_t)(__popc(one & lt) + __popc(two & lt));
+  if (count > 0) a.dense[base] = (uint32_t)t;
+  if (count > 1) a.dense[base + 1u] = (uint32_t)t + 1u;
+}
+
+// A particle whose window of `entries` entries the sparse kernel walks, on its
+// own: group by group (grouped), every candidate (exact), or its hits; h: its
+// hit list's slot.
+template <int kKind>
+__device__ __forceinline__ void sparse_one(const PassArgs& a, const SceneGeom& g, int3 q, QueueColumn col, int h,
+                                           int i, float4 xi, bool exact, bool grouped, int entries, bool fits) {
+  typename PassOf<kKind>::type p(a, g, xi, i, exact);
+  int code = kHitsWalk;
+  if (grouped || exact || !fast_hits(a, xi)) {
+    HitQueue hq(nullptr, nullptr, kSparseThreads, 1);
+    const FromGlobal src{a.X};
+    if (grouped)
+      visit_window_grouped(g, a, q, src, p, 0, entries, hq);
+    else if (exact)
+      visit_window(g, a.cs, a.n, q, src, p);  // non-neighbours matter: visit every candidate
+    else
+      visit_window_masked(g, a.cs, a.n, q, src, p, hq);
+  } else {
+    code = walk_hits<kKind>(a, col, p, h, fits);
+  }
+  p.finish(a);
+  if (kKind == kLambda) a.hit_n[h] = code;
+}
+
 // PBF_SPARSE_MIN_BLOCKS (a build-time tuning macro): resident blocks per SM the
 // compiler must allow for, which caps the sparse kernels' registers.
 #ifdef PBF_SPARSE_MIN_BLOCKS
@@ -1069,77 +1479,141 @@ __device__ __forceinline__ void stage_init(StageState& st) {
 #define PBF_SPARSE_BOUNDS __launch_bounds__(kSparseThreads)
 #endif
 
-// kStage: the variant that stages its block's column runs (launched when
-// stage_sparse > 0); the other carries no staging code.
-template <int kKind, bool kStage>
+// One thread slot of the pass's list (or of all particles) per thread; the
+// grid covers every slot, blocks past the list's end return at once.  The
+// delta_p passes, and the others where the particles are not paired.
+//
+// The delta_p passes take the hits the lambda pass listed: each list entry
+// costs one coalesced load and one gathered one (position and lambda), kept
+// kListAhead ahead, and two entries share the packed arithmetic.  Bound by the
+// gathers (L1 data path 70% busy: 32 lanes' neighbours lie in ~10 lines).
+// 1,048,576 particles at rest density: 167 -> 72 us a pass (saved masks, whose
+// bits a warp visits chunk by chunk, before).
+template <int kKind>
 __global__ void PBF_SPARSE_BOUNDS k_sparse(PassArgs a) {
   using P = typename PassOf<kKind>::type;
-  __shared__ StageState st;
-  // dynamic shared memory: the hit queue (a.c.queue_sparse chunks per thread),
-  // then the stage (a.c.stage_sparse slots, kStage only); the queue is sized
-  // per launch so that a small queue leaves the SM's L1 its capacity
-  extern __shared__ __align__(16) float4 dyn_smem[];
-  uint32_t* q_mask = reinterpret_cast<uint32_t*>(dyn_smem);
-  int* q_base = reinterpret_cast<int*>(q_mask + a.c.queue_sparse * kSparseThreads);
-  float4* stage = dyn_smem + a.c.queue_sparse * kSparseThreads / 2;
-  if (a.dense_all) return;
+  constexpr bool kDp = kKind == kDeltaP || kKind == kDeltaPFinal;
+  __shared__ uint2 queue[kQueueSlots * kSparseThreads];
   const int count = work_count(a);
   if ((int)(blockIdx.x * kSparseThreads) >= count) return;  // uniform over the block
-  // the queue is flushed once, at the window's end: a window of more chunks
-  // than it holds runs each chunk's hits right away (a flush in mid-window
-  // would run for some lanes while the others wait)
-  HitQueue hq(q_mask + threadIdx.x, q_base + threadIdx.x, kSparseThreads, 1);
-  const int t = blockIdx.x * kSparseThreads + threadIdx.x;
-  const bool valid = t < count;
-  const int i = valid ? work_particle(a, t) : 0;
+  const QueueColumn col{queue + threadIdx.x, nullptr};
+  // h: the thread's hit list.  Paired, the lambda pass's warp w lists the first
+  // particles of its 32 pairs at 64 w + lane and the second ones at 64 w + 32 +
+  // lane, so that its stores and these loads take consecutive words.
+  const int h = blockIdx.x * kSparseThreads + threadIdx.x;
+  const int t = a.paired ? (h & ~63) + 2 * (h & 31) + (h >> 5 & 1) : h;
+  const int i = t < count ? work_particle(a, t) : -1;
+  const bool valid = i >= 0;
   const float4 xi = valid ? a.X[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   const SceneGeom g = geom_of(a.c, a.G, valid ? i : 0);
-  const int3 q = cell_of(a.c, g, xi);
-  int chunks = 0;
-  const int total = valid ? window_total_chunks(g, a.cs, a.n, q, chunks) : 0;
-  // a window over dense_window candidates that its grouped cells bring back
-  // under it is walked here, group by group (no masks)
-  const bool grouped = valid && total > a.c.dense_window && a.c.keps2 > 0.f;
-  const int entries = grouped ? window_total_grouped(g, a, q) : total;
+  // the delta_p passes take the lambda pass's routing and list where it left one
+  const int code = kDp && valid ? a.hit_n[h] : kHitsWalk;
+  const bool listed = kDp && (code >= 0 || code <= kHitsMasks);
+  const bool walk = valid && !listed && code != kHitsDense;
+  int3 q = make_int3(0, 0, 0);
+  int entries = 0;
+  bool grouped = false, fits = false;
+  if (walk) {
+    q = cell_of(a.c, g, xi);
+    entries = window_runs(g, a.cs, a.n, q, col, fits);
+    // a window over dense_window candidates that its grouped cells bring back
+    // under it is walked here, group by group
+    grouped = entries > a.c.dense_window && a.c.keps2 > 0.f && a.flags[kGroupCount] != 0u;
+    if (grouped) entries = window_total_grouped(g, a, q);
+  }
   // a window over dense_window entries goes to the dense kernel, particle by
-  // particle (one list slot each, warp-aggregated): which kernel sums a
-  // particle's window depends on its own window only, so results do not
-  // depend on the list's order or on the particle's warp-mates
-  const bool go_dense = valid && entries > a.c.dense_window;
-  const unsigned dmask = __ballot_sync(kFull, go_dense);
-  if (dmask) {
-    const int lane = threadIdx.x & 31, leader = __ffs(dmask) - 1;
-    uint32_t base = 0u;
-    if (lane == leader) base = atomicAdd(&a.flags[a.counter], (uint32_t)__popc(dmask));
-    base = __shfl_sync(kFull, base, leader);
-    if (go_dense) a.dense[base + __popc(dmask & ((1u << lane) - 1u))] = (uint32_t)t;
+  // particle: which kernel sums a particle's window depends on its own window
+  // only, so results do not depend on the list's order or on the particle's
+  // warp-mates
+  const bool go_dense = valid && (walk ? entries > a.c.dense_window : code == kHitsDense);
+  append_dense(a, go_dense ? 1 : 0, t);
+  // one path per warp (its lanes' windows mostly agree)
+  fits = __all_sync(kFull, fits || !walk || go_dense || grouped);
+  if (!valid) return;
+  if (go_dense) {
+    // a window with groups may count them again after the sums of lambda
+    if (kKind == kLambda) a.hit_n[h] = grouped ? kHitsWalk : kHitsDense;
+    return;
   }
-  const bool active = valid && !go_dense;
-  const bool exact = active && exact_path(kKind, a, g, q, i);
-  // the block's plain windows staged in shared memory (block-uniform branch)
-  const int cap = kStage ? a.c.stage_sparse : 0;
-  bool staged = false;
-  uint32_t phase = 0u;
-  if (kStage && cap > 0) {
-    if (threadIdx.x == 0) stage_init(st);
-    stage_vote(st, threadIdx.x >> 5, active && !grouped, g, q, i);
-    __syncthreads();
-    if (threadIdx.x == 0) stage_issue(st, kSparseThreads / 32, a, stage, cap);
-    __syncthreads();
-    staged = stage_wait(st, a, phase);
-  }
-  if (active) {
+  if (kDp && !walk && a.flags[kFlagLambdaNonFinite]) q = cell_of(a.c, g, xi);  // for exact_path
+  const bool exact = exact_path(kKind, a, g, q, i);
+  if (kDp && !walk && !exact) {
     P p(a, g, xi, i, exact);
-    if (!grouped && !exact && chunks <= a.c.queue_sparse) hq.cap = a.c.queue_sparse;
-    if (grouped)
-      visit_window_grouped(g, a, q, FromGlobal{a.X}, p, 0, entries, hq);
-    else if (kStage && staged)
-      sparse_visit<kKind>(a, g, q, FromStage{stage, st.D}, p, exact, t, chunks, hq);
+    if (code >= 0)
+      visit_list(a, a.hits + h, code, i, p);
     else
-      sparse_visit<kKind>(a, g, q, FromGlobal{a.X}, p, exact, t, chunks, hq);
+      visit_chunks<kKind>(a, a.hits + h, kHitsMasks - code, p);
     p.finish(a);
+  } else {
+    sparse_one<kKind>(a, g, q, col, h, i, xi, exact, grouped, entries, fits);
   }
-  if (kStage && cap > 0) stage_drain(st, phase);
+}
+
+// The lambda and xsph passes over paired buckets: two particles of one cell
+// per thread.  They share the window, so the candidates' loads and the walk
+// serve both; the hits are then visited one particle after the other.
+//
+// Bound by the L1 data path and instruction issue: a test reads 12 bytes per
+// lane whatever the lanes share (L1 returns 128 bytes a cycle), 800 cycles for
+// 32 particles when every thread tested for one.  1,048,576 particles at rest
+// density: lambda 226 -> 148 us, xsph 260 -> 205 us; one particle per thread
+// with the same queue and packed arithmetic 169 and 215.  Eight blocks (64
+// registers) beat seven (no spills) and nine by 1 and 4% of the step.
+template <int kKind>
+__global__ void __launch_bounds__(kSparseThreads, 8) k_sparse_pair(PassArgs a) {
+  using P = typename PassOf<kKind>::type;
+  __shared__ uint2 queue[kQueueSlots * kSparseThreads];
+  __shared__ uint32_t second[kQueueSlots * kSparseThreads];
+  const int count = work_count(a);  // even
+  if ((int)(2 * blockIdx.x * kSparseThreads) >= count) return;  // uniform over the block
+  const QueueColumn col{queue + threadIdx.x, second + threadIdx.x};
+  const int pair = blockIdx.x * kSparseThreads + threadIdx.x;
+  const int h = 2 * (pair & ~31) + (pair & 31);  // hit list of the first; the second's is h + 32
+  const bool valid = 2 * pair < count;
+  const int2 i = valid ? __ldg(reinterpret_cast<const int2*>(a.list) + pair) : make_int2(-1, -1);
+  const bool two = i.y >= 0;
+  const float4 x0 = valid ? a.X[i.x] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 x1 = two ? a.X[i.y] : x0;
+  const SceneGeom g = geom_of(a.c, a.G, valid ? i.x : 0);
+  const int3 q = cell_of(a.c, g, x0);  // x1's too
+  int entries = 0;
+  bool grouped = false, fits = false;
+  if (valid) {
+    entries = window_runs(g, a.cs, a.n, q, col, fits);
+    grouped = entries > a.c.dense_window && a.c.keps2 > 0.f && a.flags[kGroupCount] != 0u;
+    if (grouped) entries = window_total_grouped(g, a, q);
+  }
+  const bool go_dense = valid && entries > a.c.dense_window;  // as in k_sparse
+  append_dense(a, go_dense ? (two ? 2 : 1) : 0, 2 * pair);
+  fits = __all_sync(kFull, fits || !valid || go_dense || grouped);
+  if (!valid) return;
+  if (go_dense) {
+    if (kKind == kLambda) a.hit_n[h] = a.hit_n[h + 32] = grouped ? kHitsWalk : kHitsDense;
+    return;
+  }
+  const bool exact0 = exact_path(kKind, a, g, q, i.x), exact1 = two && exact_path(kKind, a, g, q, i.y);
+  if (!grouped && !exact0 && !exact1 && fits && fast_hits(a, x0) && fast_hits(a, x1)) {
+    const int3 hits = queue_pair(a, col, x0, x1);
+    {
+      P p(a, g, x0, i.x, false);
+      const int code = finish_queued<kKind, false>(a, col, hits.z, hits.x, p, h);
+      p.finish(a);
+      if (kKind == kLambda) a.hit_n[h] = code;
+    }
+    if (two) {
+      P p(a, g, x1, i.y, false);
+      const int code = finish_queued<kKind, true>(a, col, hits.z, hits.y, p, h + 32);
+      p.finish(a);
+      if (kKind == kLambda) a.hit_n[h + 32] = code;
+    }
+    return;
+  }
+  for (int u = 0; u < (two ? 2 : 1); ++u) {
+    bool f;
+    if (u) window_runs(g, a.cs, a.n, q, col, f);  // the first walk's queue has taken their place
+    sparse_one<kKind>(a, g, q, col, h + 32 * u, u ? i.y : i.x, u ? x1 : x0, u ? exact1 : exact0, grouped, entries,
+                      fits);
+  }
 }
 
 // PBF_DENSE_BLOCKS_PER_SM (a build-time tuning macro, pbf_internal.cuh): the
@@ -1250,8 +1724,8 @@ __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
 __global__ void __launch_bounds__(256)
 k_reorder(const uint32_t* __restrict__ perm, const float4* __restrict__ pos,
           const float4* __restrict__ vel, const uint32_t* __restrict__ iid, int n, StepConsts c,
-          float4* __restrict__ xs, float4* __restrict__ xa, uint32_t* __restrict__ iid_s,
-          uint32_t* __restrict__ flags, const uint32_t* __restrict__ skeys,
+          float4* __restrict__ xs, float4* __restrict__ xa, float* __restrict__ sa, int stride,
+          uint32_t* __restrict__ iid_s, uint32_t* __restrict__ flags, const uint32_t* __restrict__ skeys,
           const uint32_t* __restrict__ cs, uint32_t* __restrict__ cell_flags, int* __restrict__ grp_cell,
           int* __restrict__ grp_off, int* __restrict__ grp_item_off, int* __restrict__ grp_item_slot) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1277,7 +1751,9 @@ k_reorder(const uint32_t* __restrict__ perm, const float4* __restrict__ pos,
   const float vx = fmaf(c.dt, c.g[0], v.x), vy = fmaf(c.dt, c.g[1], v.y),
               vz = fmaf(c.dt, c.g[2], v.z);
   xs[k] = x;
-  xa[k] = make_float4(fmaf(c.dt, vx, x.x), fmaf(c.dt, vy, x.y), fmaf(c.dt, vz, x.z), x.w);
+  const float4 xp = make_float4(fmaf(c.dt, vx, x.x), fmaf(c.dt, vy, x.y), fmaf(c.dt, vz, x.z), x.w);
+  xa[k] = xp;
+  if (sa) put_components(sa, stride, k, xp);
   iid_s[k] = iid[p];
 }
 
@@ -1761,8 +2237,9 @@ k_work_list(const int* __restrict__ follow, const int* __restrict__ blocks, int 
 // The followers take their group's results.
 template <int kKind>
 __global__ void __launch_bounds__(256)
-k_follow(const int* __restrict__ follow, int n, StepConsts c, const float4* __restrict__ X, float* __restrict__ lambda,
-         float* __restrict__ rho, float4* __restrict__ T, const float4* __restrict__ xs,
+k_follow(const int* __restrict__ follow, int n, StepConsts c, float* __restrict__ lambda, float4* __restrict__ XL,
+         float* __restrict__ rho, float4* __restrict__ T, float* __restrict__ S_out, int stride,
+         float4* __restrict__ VR, const float4* __restrict__ xs,
          const uint32_t* __restrict__ iid_s, float4* __restrict__ npos, float4* __restrict__ vel,
          float4* __restrict__ pos, uint32_t* __restrict__ iid, const uint32_t* __restrict__ skeys,
          uint32_t* __restrict__ cell_flags, uint32_t* __restrict__ flags) {
@@ -1773,16 +2250,20 @@ k_follow(const int* __restrict__ follow, int n, StepConsts c, const float4* __re
   if constexpr (kKind == kLambda) {
     lambda[i] = lambda[r];
     rho[i] = rho[r];
+    XL[i] = XL[r];  // the same position
   } else if constexpr (kKind == kDeltaP) {
     const float4 t = T[r];
-    T[i] = make_float4(t.x, t.y, t.z, X[i].w);
+    T[i] = t;
+    if (S_out) put_components(S_out, stride, i, t);
   } else {
     // DeltaPPass<true>::finish with the group's final position
     const float4 xf = npos[r];
     const float4 x0 = xs[i];
     npos[i] = make_float4(xf.x, xf.y, xf.z, x0.w);
+    if (S_out) put_components(S_out, stride, i, xf);
     const float4 v = make_float4((xf.x - x0.x) * c.inv_dt, (xf.y - x0.y) * c.inv_dt, (xf.z - x0.z) * c.inv_dt, 0.f);
     vel[i] = v;
+    VR[i] = make_float4(v.x, v.y, v.z, rho[i]);
     if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z)) {
       atomicOr(&cell_flags[skeys[i]], (uint32_t)kCellVelNonFinite);
       atomicOr(&flags[kFlagXsphExact], 1u);
@@ -1804,9 +2285,7 @@ k_follow(const int* __restrict__ follow, int n, StepConsts c, const float4* __re
 __global__ void __launch_bounds__(256) k_bucket_count(PassArgs a, uint32_t* __restrict__ bcnt,
                                                       uint2* __restrict__ bent) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int count = work_count(a);
-  if (t == 0) a.flags[kBucketCount] = (uint32_t)count;
-  if (t >= count) return;
+  if (t >= work_count(a)) return;
   const int i = work_particle(a, t);
   const SceneGeom g = geom_of(a.c, a.G, i);
   const int3 q = cell_of(a.c, g, a.X[i]);
@@ -1821,12 +2300,19 @@ __global__ void __launch_bounds__(256) k_bucket_count(PassArgs a, uint32_t* __re
   bent[t] = make_uint2(cell, base + (uint32_t)__popc(same & ((1u << lane) - 1u)));
 }
 
-__global__ void __launch_bounds__(256) k_bucket_scatter(PassArgs a, const uint32_t* __restrict__ bstart,
+// bstart: the prefix of the counts, or where a.paired of pair_slots of them (the
+// slots left over hold -1).
+__global__ void __launch_bounds__(256) k_bucket_scatter(PassArgs a, const uint32_t* __restrict__ bcnt,
+                                                        const uint32_t* __restrict__ bstart,
                                                         const uint2* __restrict__ bent, int* __restrict__ bucket) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) a.flags[kBucketCount] = bstart[a.c.cells];
   if (t >= work_count(a)) return;
   const uint2 e = bent[t];
-  bucket[bstart[e.x] + e.y] = work_particle(a, t);
+  const bool apart = a.paired && a.flags[kGroupCount] != 0u;
+  const uint32_t slot = bstart[e.x] + (apart ? 2u * e.y : e.y);
+  bucket[slot] = work_particle(a, t);
+  if (a.paired && (apart || ((e.y & 1u) == 0u && e.y + 1u == bcnt[e.x]))) bucket[slot + 1u] = -1;
 }
 
 GroupArgs group_args(const SolverScratch& s, const float4* X, const float4* V, int n) {
@@ -1884,15 +2370,20 @@ PassArgs base_args(const StepConsts& c, const Geometry& G, const float4* X, cons
   a.X = X;
   a.cs = cs;
   a.n = n;
-  a.dense_all = c.dense_all >= 0 ? c.dense_all : n < kDenseAllBelow;
+  a.dense_all = dense_for_all(c, n);
   a.counter = kDenseCount0 + (pass & 1);
   a.next_counter = kDenseCount0 + ((pass + 1) & 1);
   a.item_counter = kItemCount0 + (pass & 1);
   a.next_item_counter = kItemCount0 + ((pass + 1) & 1);
   a.flags = s.flags;
   a.dense = s.dense;
-  a.masks = s.masks;
-  a.mask_stride = s.mask_stride;
+  // a position buffer's component copy: sa beside xa, sb beside xb; the final
+  // positions' beside the buffer that is free then
+  a.stride = s.stride;
+  a.hits = s.hits;
+  a.hit_n = s.hit_n;
+  a.hit_stride = s.hit_stride;
+  a.XL = s.xl;
   a.cell_flags = s.cell_flags;
   a.skeys = s.keys_sorted;
   a.lambda = s.lambda;
@@ -1908,42 +2399,47 @@ PassArgs base_args(const StepConsts& c, const Geometry& G, const float4* X, cons
   return a;
 }
 
+// The pass takes the buckets (the delta_p passes of an iteration those of its
+// lambda pass: the same positions).
+void use_buckets(PassArgs& a, const SolverScratch& s) {
+  a.list = s.bucket;
+  a.count_word = kBucketCount;
+  a.identity_word = -1;
+  a.paired = !a.dense_all;
+}
+
 // Makes the pass take its computing particles in current-cell order: buckets
 // them (kBucketLaunches launches) and points the pass at the buckets.
 cudaError_t bucket_by_cell(PassArgs& a, const SolverScratch& s, int n, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(s.bcnt, 0, sizeof(uint32_t) * (a.c.cells + 1), stream);
   if (e != cudaSuccess) return e;
   const int blocks = (n + 255) / 256;
+  a.paired = !a.dense_all;
   k_bucket_count<<<blocks, 256, 0, stream>>>(a, s.bcnt, s.bent);
-  if ((e = exclusive_scan(s.bcnt, s.bstart, a.c.cells + 1, s.bpart, stream)) != cudaSuccess) return e;
-  k_bucket_scatter<<<blocks, 256, 0, stream>>>(a, s.bstart, s.bent, s.bucket);
-  a.list = s.bucket;
-  a.count_word = kBucketCount;
-  a.identity_word = -1;
+  if ((e = exclusive_scan(s.bcnt, s.bstart, a.c.cells + 1, s.bpart, stream,
+                          a.paired ? s.flags + kGroupCount : nullptr)) != cudaSuccess)
+    return e;
+  k_bucket_scatter<<<blocks, 256, 0, stream>>>(a, s.bcnt, s.bstart, s.bent, s.bucket);
+  use_buckets(a, s);
   return cudaGetLastError();
-}
-
-// The delta_p passes of an iteration take the lambda pass's buckets (same positions).
-void use_buckets(PassArgs& a, const SolverScratch& s) {
-  a.list = s.bucket;
-  a.count_word = kBucketCount;
-  a.identity_word = -1;
 }
 
 template <int kKind>
 cudaError_t run_pass(const PassArgs& a, cudaStream_t stream) {
-  // dynamic shared memory: the hit queue (8 bytes per chunk and thread), then the stage
-  const size_t sparse_queue = (size_t)8 * a.c.queue_sparse * kSparseThreads;
+  // the dense kernel's dynamic shared memory: the hit queue (8 bytes per chunk
+  // and thread), then the stage
   const size_t dense_queue = (size_t)8 * a.c.queue_dense * kDenseThreads;
-  const size_t sparse_smem = sizeof(float4) * (size_t)max(a.c.stage_sparse, 0);
   const size_t dense_smem = sizeof(float4) * (size_t)max(a.c.stage_dense, 0);
-  const int sparse_blocks = (a.n + kSparseThreads - 1) / kSparseThreads;
+  const long long slots = a.paired ? 2ll * a.n : a.n;  // of the pass's list, at most
+  constexpr bool kPairs = kKind == kLambda || kKind == kXsph;
+  const int per_block = kPairs && a.paired ? 2 * kSparseThreads : kSparseThreads;
+  const int sparse_blocks = (int)((slots + per_block - 1) / per_block);
   if (a.dense_all) {
-    // else the sparse kernel has nothing to do
-  } else if (sparse_smem) {
-    k_sparse<kKind, true><<<sparse_blocks, kSparseThreads, sparse_queue + sparse_smem, stream>>>(a);
+    // the sparse kernel has nothing to do
+  } else if (kPairs && a.paired) {
+    if constexpr (kPairs) k_sparse_pair<kKind><<<sparse_blocks, kSparseThreads, 0, stream>>>(a);
   } else {
-    k_sparse<kKind, false><<<sparse_blocks, kSparseThreads, sparse_queue, stream>>>(a);
+    k_sparse<kKind><<<sparse_blocks, kSparseThreads, 0, stream>>>(a);
   }
   if (dense_smem)
     k_dense<kKind, true><<<a.c.dense_grid, kDenseThreads, dense_queue + dense_smem, stream>>>(a);
@@ -1954,19 +2450,16 @@ cudaError_t run_pass(const PassArgs& a, cudaStream_t stream) {
 
 template <int kKind>
 cudaError_t allow_stage(int bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k_sparse<kKind, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_dense<kKind, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e;
+  return cudaFuncSetAttribute(k_dense<kKind, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 }  // namespace
 
-// Lets the staged pass kernels take their largest hit queue and up to
+// Lets the staged dense kernels take their largest hit queue and up to
 // kStageMax staged slots of dynamic shared memory (the current device; call
 // before any capture).
 cudaError_t set_pass_kernel_attributes() {
-  const int queue = 8 * max(kMaxQueueSparse * kSparseThreads, kMaxQueueDense * kDenseThreads);
+  const int queue = 8 * kMaxQueueDense * kDenseThreads;
   const int bytes = (int)sizeof(float4) * kStageMax + queue;
   cudaError_t e = allow_stage<kLambda>(bytes);
   if (e == cudaSuccess) e = allow_stage<kDeltaP>(bytes);
@@ -1980,8 +2473,8 @@ cudaError_t reorder(const StepConsts& c, const uint32_t* perm, const float4* pos
   cudaError_t e = cudaMemsetAsync(s.cell_flags, 0, sizeof(uint32_t) * (c.cells + 1), stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(s.flags, 0, sizeof(uint32_t) * kNumFlags, stream);
   if (e != cudaSuccess) return e;
-  k_reorder<<<(n + 255) / 256, 256, 0, stream>>>(perm, pos, vel, iid, n, c, s.xs, s.xa, s.iid_s,
-                                                  s.flags, s.keys_sorted, s.cell_start, s.cell_flags,
+  k_reorder<<<(n + 255) / 256, 256, 0, stream>>>(perm, pos, vel, iid, n, c, s.xs, s.xa,
+                                                  dense_for_all(c, n) ? nullptr : s.sa, s.stride, s.iid_s, s.flags, s.keys_sorted, s.cell_start, s.cell_flags,
                                                   s.grp_cell, s.grp_off, s.grp_item_off, s.grp_item_slot);
   return cudaGetLastError();
 }
@@ -2003,11 +2496,16 @@ cudaError_t launch_work_list(const SolverScratch& s, int n, cudaStream_t stream)
 }
 
 template <int kKind>
-cudaError_t launch_follow(const StepConsts& c, const SolverScratch& s, const float4* X, int n, float4* T,
-                          float4* pos, float4* npos, float4* vel, uint32_t* iid, cudaStream_t stream) {
-  k_follow<kKind><<<(n + 255) / 256, 256, 0, stream>>>(s.work_follow, n, c, X, s.lambda, s.rho, T, s.xs, s.iid_s,
-                                                       npos, vel, pos, iid, s.keys_sorted, s.cell_flags, s.flags);
+cudaError_t launch_follow(const PassArgs& a, const SolverScratch& s, cudaStream_t stream) {
+  k_follow<kKind><<<(a.n + 255) / 256, 256, 0, stream>>>(s.work_follow, a.n, a.c, s.lambda, s.xl, s.rho, a.T, a.S_out,
+                                                         a.stride, a.VR, s.xs, s.iid_s, a.npos, a.vel, a.pos, a.iid,
+                                                         s.keys_sorted, s.cell_flags, s.flags);
   return cudaGetLastError();
+}
+
+// The component copy of position buffer X (null: no sparse kernel reads it).
+float* components_of(const StepConsts& c, const SolverScratch& s, const float4* X, int n) {
+  return dense_for_all(c, n) ? nullptr : (X == s.xa ? s.sa : s.sb);
 }
 
 }  // namespace
@@ -2019,10 +2517,11 @@ cudaError_t launch_lambda(const StepConsts& c, const Geometry& G, const float4* 
   const bool wl = use_work_list(c, n);
   if (wl && (e = launch_work_list(s, n, stream)) != cudaSuccess) return e;
   PassArgs a = base_args(c, G, X, cs, n, s, pass);
+  a.S = components_of(c, s, X, n);
   if (wl) a.list = s.work_list;
   if (c.order && (e = bucket_by_cell(a, s, n, stream)) != cudaSuccess) return e;
   if ((e = run_pass<kLambda>(a, stream)) != cudaSuccess) return e;
-  return wl ? launch_follow<kLambda>(c, s, X, n, nullptr, nullptr, nullptr, nullptr, nullptr, stream) : cudaSuccess;
+  return wl ? launch_follow<kLambda>(a, s, stream) : cudaSuccess;
 }
 
 cudaError_t launch_delta_p(const StepConsts& c, const Geometry& G, const float4* X, const uint32_t* cs, int n,
@@ -2030,12 +2529,14 @@ cudaError_t launch_delta_p(const StepConsts& c, const Geometry& G, const float4*
   cudaError_t e = launch_groups<kGroupsLambda>(c, s, X, nullptr, n, stream);
   if (e != cudaSuccess) return e;
   const bool wl = use_work_list(c, n);
-  PassArgs a = base_args(c, G, X, cs, n, s, pass);
+  PassArgs a = base_args(c, G, s.xl, cs, n, s, pass);  // X with its lambda
+  a.S = components_of(c, s, X, n);
+  a.S_out = components_of(c, s, T, n);
   a.T = T;
   if (wl) a.list = s.work_list;
   if (c.order) use_buckets(a, s);
   if ((e = run_pass<kDeltaP>(a, stream)) != cudaSuccess) return e;
-  return wl ? launch_follow<kDeltaP>(c, s, X, n, T, nullptr, nullptr, nullptr, nullptr, stream) : cudaSuccess;
+  return wl ? launch_follow<kDeltaP>(a, s, stream) : cudaSuccess;
 }
 
 cudaError_t launch_delta_p_final(const StepConsts& c, const Geometry& G, const float4* X, const uint32_t* cs, int n,
@@ -2044,7 +2545,10 @@ cudaError_t launch_delta_p_final(const StepConsts& c, const Geometry& G, const f
   cudaError_t e = launch_groups<kGroupsLambda>(c, s, X, nullptr, n, stream);
   if (e != cudaSuccess) return e;
   const bool wl = use_work_list(c, n);
-  PassArgs a = base_args(c, G, X, cs, n, s, pass);
+  PassArgs a = base_args(c, G, s.xl, cs, n, s, pass);
+  a.S = components_of(c, s, X, n);
+  a.VR = X == s.xa ? s.xb : s.xa;  // the positions go to npos: T's buffers are free
+  a.S_out = components_of(c, s, a.VR, n);
   a.xs = s.xs;
   a.iid_s = s.iid_s;
   a.npos = npos;
@@ -2054,7 +2558,7 @@ cudaError_t launch_delta_p_final(const StepConsts& c, const Geometry& G, const f
   if (wl) a.list = s.work_list;
   if (c.order) use_buckets(a, s);
   if ((e = run_pass<kDeltaPFinal>(a, stream)) != cudaSuccess) return e;
-  return wl ? launch_follow<kDeltaPFinal>(c, s, X, n, nullptr, pos, npos, vel, iid, stream) : cudaSuccess;
+  return wl ? launch_follow<kDeltaPFinal>(a, s, stream) : cudaSuccess;
 }
 
 // ---- vorticity confinement ---------------------------------------------------------------
@@ -2154,6 +2658,10 @@ cudaError_t launch_xsph(const StepConsts& c, const Geometry& G, const float4* X,
   cudaError_t e = launch_groups<kGroupsXsph>(c, s, X, V, n, stream);
   if (e != cudaSuccess) return e;
   PassArgs a = base_args(c, G, X, cs, n, s, pass);
+  // where the last position update left them: after niter - 1 swaps of xa and
+  // xb it read one and used the other
+  a.VR = (pass / 2) % 2 ? s.xb : s.xa;
+  a.S = components_of(c, s, a.VR, n);
   a.V = V;
   a.NV = NV;
   if (c.order && (e = bucket_by_cell(a, s, n, stream)) != cudaSuccess) return e;
@@ -2165,8 +2673,7 @@ cudaError_t launch_xsph(const StepConsts& c, const Geometry& G, const float4* X,
 namespace pbf {
 
 int pass_launches(const StepConsts& c, int n) {
-  const bool all = c.dense_all >= 0 ? c.dense_all != 0 : n < kDenseAllBelow;
-  return all ? 1 : 2;
+  return dense_for_all(c, n) ? 1 : 2;
 }
 
 // launch_groups: 1 launch before each lambda pass, 2 before each delta_p pass, 3 before xsph;
