@@ -103,6 +103,42 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 
+// Two floats in one register pair: packed arithmetic rounds each as the scalar
+// operation does and takes one issue slot for both.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 dist2_2(f32x2 ex, f32x2 ey, f32x2 ez) {
+  return fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
+}
+
 // W(r^2) for r^2 < h^2 (getPoly6::operator(), fluids/Simulator.cu:84-89).
 __device__ __forceinline__ float poly6_inside(const StepConsts& c, float r2) {
   float d = c.h2 - r2;

@@ -529,42 +529,6 @@ __device__ __forceinline__ void visit_window_grouped(const SceneGeom& g, const P
 
 // ---- the passes: per-candidate visit, partial-sum fields, finish ----------------------
 
-// Two floats in one register pair: packed arithmetic rounds each as the scalar
-// operation does and takes one issue slot for both.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f32x2 dist2_2(f32x2 ex, f32x2 ey, f32x2 ez) {
-  return fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
-}
-
 // rsqrtf of a normal number (bitwise the same there, without the scaling of
 // subnormal arguments; a zero gives +inf).
 __device__ __forceinline__ float rsqrt_normal(float x) {

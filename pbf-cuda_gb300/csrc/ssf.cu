@@ -2,14 +2,14 @@
 // reference's OpenGL SSFRenderer (fluids/SSFRenderer.cpp:113-358, shaders
 // fluids/shader/SSF*.glsl) as CUDA kernels over headless device images.
 //
-// One render = clear, splat (depth + thickness of every sprite fragment),
-// resolve, smooth_niter smoothing passes, normals, shading: 5 + smooth_niter
-// launches on the caller's stream.
+// One render = splat (depth + thickness of every sprite fragment), resolve,
+// smooth_niter smoothing passes, normals and shading: 3 + smooth_niter launches
+// on the caller's stream (one more when profiled).
 //
-//   k_ssf_splat   a warp takes 32 particles; each lane projects one (the vertex
-//                 shader), then the warp rasterises the 32 sprites one after the
-//                 other, its lanes spread over the sprite's pixels (the fragment
-//                 shaders).  A pixel keeps the smallest eye depth (atomicMin on
+//   k_ssf_splat   a warp takes 32 or 8 particles; each lane projects one (the
+//                 vertex shader), then the warp rasterises the sprites one after
+//                 the other, its lanes spread over the sprite's pixels (the
+//                 fragment shaders).  A pixel keeps the smallest eye depth (atomicMin on
 //                 an order-preserving integer image of the float) and the sum of
 //                 2 r z in 64-bit fixed point (2^-32 per unit): both independent
 //                 of the order fragments arrive in, so renders are deterministic.
@@ -19,14 +19,16 @@
 //                 written the same way, reproduces depth and thickness bit for
 //                 bit.  gl_PointCoord takes one reciprocal of the point size per
 //                 sprite (GL leaves its precision to the implementation).
-//   k_ssf_smooth  32 x 16 output pixels per 256-thread block, the source tile
-//                 and its kernel_r halo staged in shared memory with the spatial
-//                 weights; taps summed in the shader's order (dx outer, dy inner).
-//   k_ssf_normal  one thread per pixel, neighbours wrapping at the image edges.
-//   k_ssf_shade   one thread per pixel; trace_color's floor and sky cube map.
+//   k_ssf_smooth  32 x 16 output pixels per 128-thread block, four rows a thread,
+//                 the source tile and its kernel_r halo staged in shared memory
+//                 with the spatial weights; taps summed in the shader's order (dx
+//                 outer, dy inner).
+//   k_ssf_surface one thread per pixel: the normal (neighbours wrapping at the
+//                 image edges), then trace_color's floor and sky cube map.
 //
 // All kernels are bounded loops over in-range indices: no waits, no device
 // asserts.
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -47,12 +49,14 @@ constexpr int kMaxImageSide = 16384;
 constexpr float kClearDepth = 100.f;       // glClearTexImage(d_depth_a/b, ..., 100) (SSFRenderer.cpp:159-162)
 constexpr float kBackground = 99.f;        // smoothing skips z > 99 (SSFsmooth_depth.f.glsl:68)
 constexpr float kThickScale = 4294967296.f;  // 2^32: fixed-point units per unit of thickness
-constexpr int kSmoothTileW = 32, kSmoothTileH = 16, kSmoothThreadsY = 8;
+constexpr int kSmoothTileW = 32, kSmoothRows = 4, kSmoothThreadsY = 4;
+constexpr int kSmoothTileH = kSmoothRows * kSmoothThreadsY;
 
 struct SsfConsts {
   int W, H;
   float V[16], P[16], IV[16];
   float p_n, p_f, p_t, p_r;
+  float c_x, c_y;         // the normal's 2 / (W p_n / p_r), 2 / (H p_n / p_t)
   float r;
   int kernel_r;
   float blur_r, blur_z;
@@ -129,52 +133,84 @@ __global__ void __launch_bounds__(256) k_ssf_clear(int npix, uint32_t* __restric
   tfx[k] = 0ull;
 }
 
-__global__ void __launch_bounds__(256) k_ssf_splat(SsfConsts c, const float4* __restrict__ pos, int n,
-                                                   uint32_t* __restrict__ zkey,
-                                                   unsigned long long* __restrict__ tfx,
-                                                   unsigned long long* __restrict__ frag_count) {
+constexpr int kSplatThreads = 128;
+// Sprites of a warp: 32, or 8 where 32 would leave the SMs short of warps
+// (32,768 particles at 640 x 480: a frame 123 us with 32, 88 with 8).
+constexpr int kSplatFewBelow = 32 * 32 * 152;
+
+// Bound by the images' atomics (two for each fragment, resolved in L2) and
+// instruction issue.  A whole warp draws one sprite, so that an atomic's lanes
+// lie in few rows: eight lanes to a sprite, four sprites at a time, executes
+// less and takes 416 us.  The pixel coordinates are stepped as floats.
+// Gathering a warp's fragments in shared memory first gained nothing
+// (consecutive particles rarely overlap enough).  70M fragments of 1,048,576
+// particles at 1600 x 1200: 324 -> 301 us.
+//
+// kNarrow: a fragment's thickness fits 32 bits of fixed point.
+template <int kSprites, bool kNarrow>
+__global__ void __launch_bounds__(kSplatThreads) k_ssf_splat(SsfConsts c, const float4* __restrict__ pos, int n,
+                                                             uint32_t* __restrict__ zkey,
+                                                             unsigned long long* __restrict__ tfx,
+                                                             unsigned long long* __restrict__ frag_count) {
+  __shared__ float4 s_disc[kSplatThreads / 32][kSprites];  // xw, yw, s2, vz
+  __shared__ int4 s_box[kSplatThreads / 32][kSprites];     // x0, y0, width, pixels (0: not drawn)
   const int lane = threadIdx.x & 31;
-  const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x));
-  Sprite me = {};
-  const bool ok = i < n && make_sprite(c, pos[i], me);
+  float4* disc = s_disc[threadIdx.x >> 5];
+  int4* box = s_box[threadIdx.x >> 5];
+  const long long i = (((long long)blockIdx.x * kSplatThreads + threadIdx.x) >> 5) * kSprites + lane;
+  if (lane < kSprites) {
+    Sprite me = {};
+    if (i < n && make_sprite(c, pos[i], me)) {
+      const int w = me.x1 - me.x0 + 1;  // 1 .. W
+      disc[lane] = make_float4(me.xw, me.yw, me.s2, me.vz);
+      box[lane] = make_int4(me.x0, me.y0, w, w * (me.y1 - me.y0 + 1));  // <= W H < 2^31
+    } else {
+      box[lane] = make_int4(0, 0, 1, 0);
+    }
+  }
+  __syncwarp();
   unsigned frags = 0;
   // thickness 2 r z in fixed point: z (2 r 2^32), the same value as (2 r z) 2^32
   const float qscale = fm(fm(2.f, c.r), kThickScale);
-  unsigned todo = __ballot_sync(0xffffffffu, ok);
-  while (todo) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1u;
-    const float xw = __shfl_sync(0xffffffffu, me.xw, src), yw = __shfl_sync(0xffffffffu, me.yw, src);
-    const float s2 = __shfl_sync(0xffffffffu, me.s2, src), vz = __shfl_sync(0xffffffffu, me.vz, src);
-    const int x0 = __shfl_sync(0xffffffffu, me.x0, src), x1 = __shfl_sync(0xffffffffu, me.x1, src);
-    const int y0 = __shfl_sync(0xffffffffu, me.y0, src), y1 = __shfl_sync(0xffffffffu, me.y1, src);
-    const int w = x1 - x0 + 1;                 // 1 .. W
-    const int total = w * (y1 - y0 + 1);       // <= W H < 2^31
-    // fragment f = row * w + col, lanes strided by 32 (row, col stepped incrementally)
-    int row = lane / w, col = lane - (lane / w) * w;
-    const int drow = 32 / w, dcol = 32 - drow * w;
+  for (int src = 0; src < kSprites; ++src) {
+    const float4 d = disc[src];
+    const int4 b = box[src];
+    const int w = b.z, total = b.w;
+    // fragment f = row * w + col, lanes strided by 32; row = lane / w by a
+    // reciprocal in 16.16 (exact: lane <= 32)
+    const unsigned inv = 65536u / (unsigned)w + 1u;
+    const int row = (int)((unsigned)lane * inv >> 16), drow = (int)(32u * inv >> 16);
+    int col = lane - row * w;
+    const int dcol = 32 - drow * w;
+    // pixel centres (integer + 1/2, exact in float) and the pixel's index, stepped
+    float fx = fa((float)(b.x + col), 0.5f), fy = fa((float)(b.y + row), 0.5f);
+    const float fdx = (float)dcol, fdy = (float)drow, fw = (float)w;
+    int k = (b.y + row) * c.W + b.x + col;
+    const int dk = drow * c.W + dcol, wrap = c.W - w;
     for (int f = lane; f < total; f += 32) {
-      const int px = x0 + col, py = y0 + row;
       // the fragment shader (SSFget_depth.f.glsl:21-37) at gl_PointCoord (upper-left
       // origin): x = 2 s - 1 = (px + 1/2 - xw) 2 / size, y = 2 t - 1 = (yw - py - 1/2) 2 / size
-      const float x = fm(fs(fa((float)px, 0.5f), xw), s2);
-      const float y = fm(fs(yw, fa((float)py, 0.5f)), s2);
+      const float x = fm(fs(fx, d.x), d.z);
+      const float y = fm(fs(d.y, fy), d.z);
       const float pho = __fmaf_rn(x, x, fm(y, y));
       if (!(pho > 1.f)) {
         const float z = __fsqrt_rn(fs(1.f, pho));
-        const float depth = -__fmaf_rn(z, c.r, vz);  // -nviewPos.z, nviewPos = viewPos + (x, y, z) r
-        const size_t k = (size_t)py * c.W + px;
+        const float depth = -__fmaf_rn(z, c.r, d.w);  // -nviewPos.z, nviewPos = viewPos + (x, y, z) r
         atomicMin(zkey + k, depth_key(depth));
         // 2 r dot((x, y, z), (0, 0, 1)) (SSFget_thick.f.glsl:24-25)
-        const long long q = __float2ll_rn(fm(z, qscale));
-        if (q) atomicAdd(tfx + k, (unsigned long long)q);
+        const float q = fm(z, qscale);
+        atomicAdd(tfx + k, kNarrow ? (unsigned long long)__float2uint_rn(q) : (unsigned long long)__float2ll_rn(q));
         ++frags;
       }
       col += dcol;
-      row += drow;
+      k += dk;
+      fx = fa(fx, fdx);
+      fy = fa(fy, fdy);
       if (col >= w) {
         col -= w;
-        ++row;
+        k += wrap;
+        fx = fs(fx, fw);
+        fy = fa(fy, 1.f);
       }
     }
   }
@@ -184,38 +220,143 @@ __global__ void __launch_bounds__(256) k_ssf_splat(SsfConsts c, const float4* __
   }
 }
 
-// depth_a <- the splat's depth, depth_b <- the clear value, thickness <- the
-// fixed-point sums (SSFRenderer.cpp:159-162, 207).
-__global__ void __launch_bounds__(256) k_ssf_resolve(int npix, const uint32_t* __restrict__ zkey,
-                                                     const unsigned long long* __restrict__ tfx,
-                                                     float* __restrict__ depth_a, float* __restrict__ depth_b,
-                                                     float* __restrict__ thick) {
+template <bool kNarrow>
+void launch_splat(const SsfConsts& c, const float4* pos, int n, uint32_t* zkey, unsigned long long* tfx,
+                  unsigned long long* frags, cudaStream_t st) {
+  const auto blocks = [n](int sprites) {
+    const long long per_block = (long long)kSplatThreads / 32 * sprites;
+    return (int)((n + per_block - 1) / per_block);
+  };
+  if (n < kSplatFewBelow)
+    k_ssf_splat<8, kNarrow><<<blocks(8), kSplatThreads, 0, st>>>(c, pos, n, zkey, tfx, frags);
+  else
+    k_ssf_splat<32, kNarrow><<<blocks(32), kSplatThreads, 0, st>>>(c, pos, n, zkey, tfx, frags);
+}
+
+// depth_a <- the splat's depth, thickness <- the fixed-point sums
+// (SSFRenderer.cpp:159-162, 207), and the splat's images back to their clear
+// values for the next render.
+__global__ void __launch_bounds__(256) k_ssf_resolve(int npix, uint32_t* __restrict__ zkey,
+                                                     unsigned long long* __restrict__ tfx,
+                                                     float* __restrict__ depth_a, float* __restrict__ thick) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= npix) return;
   depth_a[k] = depth_of_key(zkey[k]);
-  depth_b[k] = kClearDepth;
   thick[k] = __double2float_rn(__ll2double_rn((long long)tfx[k]) * 0x1p-32);
+  zkey[k] = depth_key(kClearDepth);
+  tfx[k] = 0ull;
+}
+
+// 2^x; a result below the smallest normal float is 0 (as an addend of the
+// weight sums, which the centre tap makes at least 1, it changes nothing).
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Four output pixels of a column as two pairs, their sums and weight sums.
+struct Bilateral {
+  pbf::f32x2 za, zb, bz, sum_a = 0ull, sum_b = 0ull, w_a = 0ull, w_b = 0ull;
+  // g = exp(-((s - z) blur_z)^2) = 2^-((s - z) blur_z sqrt(log2 e))^2
+  __device__ __forceinline__ pbf::f32x2 weight(pbf::f32x2 w, pbf::f32x2 s, pbf::f32x2 z) const {
+    const pbf::f32x2 r = pbf::mul2(pbf::sub2(s, z), bz);
+    float lo, hi;
+    pbf::unpack2(pbf::mul2(r, r), lo, hi);
+    return pbf::mul2(w, pbf::pack2(exp2_ftz(-lo), exp2_ftz(-hi)));
+  }
+  __device__ __forceinline__ void tap(float w, pbf::f32x2 sa, pbf::f32x2 sb) {
+    const pbf::f32x2 w2 = pbf::both(w);
+    const pbf::f32x2 wa = weight(w2, sa, za), wb = weight(w2, sb, zb);
+    sum_a = pbf::fma2(sa, wa, sum_a);
+    w_a = pbf::add2(w_a, wa);
+    sum_b = pbf::fma2(sb, wb, sum_b);
+    w_b = pbf::add2(w_b, wb);
+  }
+};
+struct Gaussian {
+  pbf::f32x2 sum_a = 0ull, sum_b = 0ull, w_a = 0ull, w_b = 0ull;
+  __device__ __forceinline__ void tap(float w, pbf::f32x2 sa, pbf::f32x2 sb) {
+    const pbf::f32x2 w2 = pbf::both(w);
+    sum_a = pbf::fma2(sa, w2, sum_a);
+    sum_b = pbf::fma2(sb, w2, sum_b);
+    w_a = pbf::add2(w_a, w2);
+    w_b = w_a;
+  }
+};
+
+// The taps of four pixels in a column, in the shader's order.  The tile is
+// stored by columns, twice, the second copy one row down, so that the pair
+// (row k, row k + 1) is one aligned load for any k; the pair of the two upper
+// pixels at tap k + 2 is the lower pixels' at tap k.
+template <class F>
+__device__ __forceinline__ void smooth_taps(const float* even, const float* odd, int stride, const float* wsp, int K,
+                                            F& f) {
+  auto at = [](const float* p) { return *reinterpret_cast<const pbf::f32x2*>(p); };
+  for (int dx = 0; dx < K; ++dx, even += stride, odd += stride, wsp += K) {
+    pbf::f32x2 p0 = at(even), p1 = at(odd);
+    int k = 0;
+#pragma unroll 2
+    for (; k + 1 < K; k += 2) {
+      const pbf::f32x2 p2 = at(even + k + 2);
+      f.tap(wsp[k], p0, p2);
+      const pbf::f32x2 p3 = at(odd + k + 2);
+      f.tap(wsp[k + 1], p1, p3);
+      p0 = p2;
+      p1 = p3;
+    }
+    f.tap(wsp[k], p0, at(even + k + 2));  // K is odd
+  }
+}
+
+// Rows of a tile column, and the column stride: even, half of it odd (the lanes
+// of a load, one column apart, then hit different banks).
+__host__ __device__ constexpr int smooth_stride(int R) {
+  return kSmoothTileH + 2 * R + (((kSmoothTileH + 2 * R) / 2) & 1 ? 0 : 2);
+}
+size_t smooth_smem(int R) {
+  const int K = 2 * R + 1;
+  return sizeof(float) * (2 * (size_t)(kSmoothTileW + 2 * R) * smooth_stride(R) + (size_t)K * K);
 }
 
 // One smoothing pass (SSFsmooth_depth.f.glsl:26-75): dst keeps its content where
-// the source depth is background (> 99).  Taps in the shader's order; the
-// range weight through exp2f and fused multiply-adds (within 1e-5 of the float
-// oracle's expf and separate roundings).
+// the source depth is background (> 99); the first pass writes the clear value
+// there (dst then holds the previous render's image).  Taps in the shader's
+// order; the range weight through exp2 and fused multiply-adds (within 1e-5 of
+// the float oracle's expf and separate roundings).
+//
+// Bound by instruction issue: a tap of one pixel in scalar arithmetic cost ~14
+// instructions, here ~5 (two pixels to a packed one, one shared-memory load for
+// four pixels' taps, no subnormal handling around ex2).  1600 x 1200, kernel_r
+// 10: 133 -> 76 us a pass; 640 x 480, gaussian: 30 -> 14.
 __global__ void __launch_bounds__(kSmoothTileW * kSmoothThreadsY)
-k_ssf_smooth(SsfConsts c, const float* __restrict__ src, float* __restrict__ dst) {
-  constexpr int kTW = kSmoothTileW + 2 * kMaxKernelR, kTH = kSmoothTileH + 2 * kMaxKernelR;
-  constexpr int kK = 2 * kMaxKernelR + 1;
-  __shared__ float tile[kTW * kTH];
-  __shared__ float wsp[kK * kK];
-  const int R = c.kernel_r, K = 2 * R + 1;
-  const int tw = kSmoothTileW + 2 * R, th = kSmoothTileH + 2 * R;
-  const int gx0 = blockIdx.x * kSmoothTileW - R, gy0 = blockIdx.y * kSmoothTileH - R;
-  const int tid = threadIdx.y * kSmoothTileW + threadIdx.x;
+k_ssf_smooth(SsfConsts c, const float* __restrict__ src, float* __restrict__ dst, bool first) {
+  extern __shared__ __align__(16) float smem[];
   constexpr int kThreads = kSmoothTileW * kSmoothThreadsY;
+  const int R = c.kernel_r, K = 2 * R + 1;
+  const int tw = kSmoothTileW + 2 * R, th = kSmoothTileH + 2 * R, stride = smooth_stride(R);
+  float* even = smem;                 // [tw][stride]
+  float* odd = smem + tw * stride;    // [tw][stride]: one row down
+  float* wsp = odd + tw * stride;     // [K][K]
+  const int tid = threadIdx.y * kSmoothTileW + threadIdx.x;
+  const int px = blockIdx.x * kSmoothTileW + threadIdx.x, py = blockIdx.y * kSmoothTileH + threadIdx.y * kSmoothRows;
+  float z[kSmoothRows];
+  bool fluid = false;
+#pragma unroll
+  for (int k = 0; k < kSmoothRows; ++k) {
+    const bool in = px < c.W && py + k < c.H;
+    z[k] = in ? src[(size_t)(py + k) * c.W + px] : kClearDepth;
+    if (in && first && z[k] > kBackground) dst[(size_t)(py + k) * c.W + px] = kClearDepth;
+    fluid |= !(z[k] > kBackground);
+  }
+  if (!__syncthreads_or(fluid)) return;
+  const int gx0 = blockIdx.x * kSmoothTileW - R, gy0 = blockIdx.y * kSmoothTileH - R;
   for (int k = tid; k < tw * th; k += kThreads) {
     const int ty = k / tw, tx = k - ty * tw;
     const int gx = gx0 + tx, gy = gy0 + ty;
-    tile[k] = (gx >= 0 && gx < c.W && gy >= 0 && gy < c.H) ? src[(size_t)gy * c.W + gx] : 0.f;  // texelFetch out of range: 0
+    const float v = (gx >= 0 && gx < c.W && gy >= 0 && gy < c.H) ? src[(size_t)gy * c.W + gx] : 0.f;  // texelFetch out of range: 0
+    even[tx * stride + ty] = v;
+    if (ty > 0) odd[tx * stride + ty - 1] = v;
   }
   for (int k = tid; k < K * K; k += kThreads) {
     const int a = k / K, b = k - a * K;
@@ -224,49 +365,35 @@ k_ssf_smooth(SsfConsts c, const float* __restrict__ src, float* __restrict__ dst
     wsp[k] = expf(fm(fm((float)(-(dx * dx + dy * dy)), c.blur_r), c.blur_r));
   }
   __syncthreads();
-  const int px = blockIdx.x * kSmoothTileW + threadIdx.x;
-  for (int row = threadIdx.y; row < kSmoothTileH; row += kSmoothThreadsY) {
-    const int py = blockIdx.y * kSmoothTileH + row;
-    if (px >= c.W || py >= c.H) continue;
-    const float* center = tile + (row + R) * tw + threadIdx.x + R;
-    const float z = *center;
-    if (z > kBackground) continue;
-    float sum = 0.f, wsum = 0.f;
-    if (c.blur_option == 0) {
-      // g = exp(-((s - z) blur_z)^2) = 2^-((s - z) blur_z sqrt(log2 e))^2
-      const float bz = c.blur_z * 1.2011224087864498f;
-      for (int dx = -R; dx <= R; ++dx) {
-        const float* wrow = wsp + (dx + R) * K + R;
-        for (int dy = -R; dy <= R; ++dy) {
-          const float s = center[dy * tw + dx];
-          const float r2 = (s - z) * bz;
-          const float wg = wrow[dy] * exp2f(-r2 * r2);
-          sum = fmaf(s, wg, sum);
-          wsum += wg;
-        }
-      }
-    } else {
-      for (int dx = -R; dx <= R; ++dx) {
-        const float* wrow = wsp + (dx + R) * K + R;
-        for (int dy = -R; dy <= R; ++dy) {
-          const float w = wrow[dy];
-          sum = fmaf(center[dy * tw + dx], w, sum);
-          wsum += w;
-        }
-      }
-    }
-    if (wsum > 0.f) sum = fd(sum, wsum);
-    dst[(size_t)py * c.W + px] = sum;
+  if (!fluid) return;
+  const int at = threadIdx.x * stride + threadIdx.y * kSmoothRows;
+  float sum[kSmoothRows], wsum[kSmoothRows];
+  auto take = [&](const auto& f) {
+    pbf::unpack2(f.sum_a, sum[0], sum[1]);
+    pbf::unpack2(f.sum_b, sum[2], sum[3]);
+    pbf::unpack2(f.w_a, wsum[0], wsum[1]);
+    pbf::unpack2(f.w_b, wsum[2], wsum[3]);
+  };
+  if (c.blur_option == 0) {
+    Bilateral f;
+    f.za = pbf::pack2(z[0], z[1]), f.zb = pbf::pack2(z[2], z[3]);
+    f.bz = pbf::both(c.blur_z * 1.2011224087864498f);
+    smooth_taps(even + at, odd + at, stride, wsp, K, f);
+    take(f);
+  } else {
+    Gaussian f;
+    smooth_taps(even + at, odd + at, stride, wsp, K, f);
+    take(f);
   }
+#pragma unroll
+  for (int k = 0; k < kSmoothRows; ++k)
+    if (!(z[k] > kBackground)) dst[(size_t)(py + k) * c.W + px] = wsum[k] > 0.f ? fd(sum[k], wsum[k]) : sum[k];
 }
 
 // SSFrestore_normal.f.glsl:31-58; getZ returns -depth, neighbours wrap (REPEAT).
 // Explicitly rounded in the float oracle's order: the same depth image gives
 // the same normals bit for bit.
-__global__ void __launch_bounds__(256) k_ssf_normal(SsfConsts c, const float* __restrict__ depth,
-                                                    float4* __restrict__ normal_D) {
-  const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y;
-  if (px >= c.W || py >= c.H) return;
+__device__ __forceinline__ float4 surface_normal(const SsfConsts& c, const float* __restrict__ depth, int px, int py) {
   const int xp = px + 1 == c.W ? 0 : px + 1, xm = px == 0 ? c.W - 1 : px - 1;
   const int yp = py + 1 == c.H ? 0 : py + 1, ym = py == 0 ? c.H - 1 : py - 1;
   const size_t row = (size_t)py * c.W;
@@ -277,11 +404,10 @@ __global__ void __launch_bounds__(256) k_ssf_normal(SsfConsts c, const float* __
     if (fabsf(dzdx2) < fabsf(dzdx)) dzdx = dzdx2;
     if (fabsf(dzdy2) < fabsf(dzdy)) dzdy = dzdy2;
   }
-  const float f_x = fd(c.p_n, c.p_r), f_y = fd(c.p_n, c.p_t);
-  const float c_x = fd(2.f, fm((float)c.W, f_x)), c_y = fd(2.f, fm((float)c.H, f_y));
+  const float c_x = c.c_x, c_y = c.c_y;
   const float nx = fm(-c_y, dzdx), ny = fm(-c_x, dzdy), nz = -fm(fm(c_x, c_y), z);
   const float d = __fsqrt_rn(fa(fa(fm(nx, nx), fm(ny, ny)), fm(nz, nz)));
-  normal_D[row + px] = make_float4(fd(nx, d), fd(ny, d), fd(nz, d), d);
+  return make_float4(fd(nx, d), fd(ny, d), fd(nz, d), d);
 }
 
 // ---- shading (SSFshading.f.glsl) ------------------------------------------------------
@@ -353,17 +479,27 @@ __device__ void trace_color(const SsfConsts& c, const float p[3], const float d[
   sky_color(c, wd, out);
 }
 
-__global__ void __launch_bounds__(256) k_ssf_shade(SsfConsts c, const float* __restrict__ depth,
-                                                   const float4* __restrict__ normal_D,
-                                                   const float* __restrict__ thick, float4* __restrict__ color) {
+// kNormal: writes the pixel's normal (else reads it); kShade: and its colour.
+// Both in one pass, or one after the other when the render is profiled.
+template <bool kNormal, bool kShade>
+__global__ void __launch_bounds__(256) k_ssf_surface(SsfConsts c, const float* __restrict__ depth,
+                                                     float4* __restrict__ normal_D,
+                                                     const float* __restrict__ thick, float4* __restrict__ color) {
   const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y;
   if (px >= c.W || py >= c.H) return;
   const size_t k = (size_t)py * c.W + px;
+  float4 nd;
+  if (kNormal) {
+    nd = surface_normal(c, depth, px, py);
+    normal_D[k] = nd;
+  } else {
+    nd = normal_D[k];
+  }
+  if (!kShade) return;
   const float ze = depth[k];
   // gl_FragDepth from ze against the cleared depth buffer: drawn iff ze < far
   if (!(ze < c.p_f)) return;
   const float u = fd(fa((float)px, 0.5f), (float)c.W), v = fd(fa((float)py, 0.5f), (float)c.H);
-  const float4 nd = normal_D[k];
   const float n[3] = {nd.x, nd.y, nd.z};
   // getPos: right-handed eye position of the pixel's surface point
   const float p[3] = {fd(fm(fm(fs(fm(2.f, u), 1.f), c.p_r), ze), c.p_n),
@@ -540,6 +676,9 @@ SsfConsts consts_of(const pbf_ssf* s) {
   std::memcpy(c.P, p.proj, sizeof(c.P));
   std::memcpy(c.IV, s->iview, sizeof(c.IV));
   c.p_n = p.p_n, c.p_f = p.p_f, c.p_t = p.p_t, c.p_r = p.p_r;
+  // rounded operation by operation, as in the shader
+  const float f_x = p.p_n / p.p_r, f_y = p.p_n / p.p_t;
+  c.c_x = 2.f / ((float)c.W * f_x), c.c_y = 2.f / ((float)c.H * f_y);
   c.r = p.radius;
   c.kernel_r = p.kernel_r;
   // loadParams: blur_r = 1 / sigma_r, blur_z = 1 / sigma_z (fluids/SSFRenderer.cpp:286-287)
@@ -651,6 +790,11 @@ pbf_status pbf_ssf_create(const pbf_ssf_params* p, pbf_ssf** out) {
   if (e == cudaSuccess) e = cudaMalloc(&s->normal_D, 16 * npix);
   if (e == cudaSuccess) e = cudaMalloc(&s->frag_count, 8);
   if (e == cudaSuccess) e = cudaMemset(s->frag_count, 0, 8);
+  if (e == cudaSuccess) {  // every render leaves the splat's images clear
+    k_ssf_clear<<<(int)((npix + 255) / 256), 256>>>((int)npix, s->zkey, s->tfx);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  }
   for (int k = 0; e == cudaSuccess && k < 5; ++k) e = cudaEventCreate(&s->ev[k]);
   if (e == cudaSuccess) s->have_events = true;
   if (e != cudaSuccess) {
@@ -739,16 +883,17 @@ pbf_status pbf_ssf_render(pbf_ssf* s, const void* pos, int n, void* color, void*
     e = cudaMemsetAsync(s->frag_count, 0, 8, st);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev[0], st);
   }
-  // 1-2. depth and thickness splats, resolved into depth_a / depth_b / thick
+  // 1-2. depth and thickness splats, resolved into depth_a / thick
   if (e == cudaSuccess) {
-    k_ssf_clear<<<(npix + 255) / 256, 256, 0, st>>>(npix, s->zkey, s->tfx);
-    ++launches;
     if (n > 0) {
-      k_ssf_splat<<<(int)(((long long)n + 255) / 256), 256, 0, st>>>(c, (const float4*)pos, n, s->zkey, s->tfx,
-                                                   prof ? s->frag_count : nullptr);
+      unsigned long long* frags = prof ? s->frag_count : nullptr;
+      if (2.0 * c.r < 0.999)  // 2 r 2^32 < 2^32, with room for its rounding
+        launch_splat<true>(c, (const float4*)pos, n, s->zkey, s->tfx, frags, st);
+      else
+        launch_splat<false>(c, (const float4*)pos, n, s->zkey, s->tfx, frags, st);
       ++launches;
     }
-    k_ssf_resolve<<<(npix + 255) / 256, 256, 0, st>>>(npix, s->zkey, s->tfx, s->depth_a, s->depth_b, s->thick);
+    k_ssf_resolve<<<(npix + 255) / 256, 256, 0, st>>>(npix, s->zkey, s->tfx, s->depth_a, s->thick);
     ++launches;
     e = cudaGetLastError();
   }
@@ -762,24 +907,26 @@ pbf_status pbf_ssf_render(pbf_ssf* s, const void* pos, int n, void* color, void*
     for (int it = 1; it <= s->p.smooth_niter; ++it) {
       const float* src = (it & 1) ? s->depth_a : s->depth_b;
       float* dst = (it & 1) ? s->depth_b : s->depth_a;
-      k_ssf_smooth<<<grid, block, 0, st>>>(c, src, dst);
+      k_ssf_smooth<<<grid, block, smooth_smem(c.kernel_r), st>>>(c, src, dst, it == 1);
       ++launches;
       final_depth = dst;
     }
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && prof) e = cudaEventRecord(s->ev[2], st);
-  // 4. normals
+  // 4-5. normals and shading
   const dim3 pgrid((c.W + 255) / 256, c.H);
   if (e == cudaSuccess) {
-    k_ssf_normal<<<pgrid, 256, 0, st>>>(c, final_depth, s->normal_D);
+    if (prof || !color)
+      k_ssf_surface<true, false><<<pgrid, 256, 0, st>>>(c, final_depth, s->normal_D, s->thick, nullptr);
+    else
+      k_ssf_surface<true, true><<<pgrid, 256, 0, st>>>(c, final_depth, s->normal_D, s->thick, (float4*)color);
     ++launches;
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && prof) e = cudaEventRecord(s->ev[3], st);
-  // 5. shading
-  if (e == cudaSuccess && color) {
-    k_ssf_shade<<<pgrid, 256, 0, st>>>(c, final_depth, s->normal_D, s->thick, (float4*)color);
+  if (e == cudaSuccess && prof && color) {
+    k_ssf_surface<false, true><<<pgrid, 256, 0, st>>>(c, final_depth, s->normal_D, s->thick, (float4*)color);
     ++launches;
     e = cudaGetLastError();
   }
