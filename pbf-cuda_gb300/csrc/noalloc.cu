@@ -50,7 +50,7 @@ pbf_status validate_step_buffers(const void* pos, const void* npos, const void* 
 namespace {
 
 constexpr int kNoAllocMaxParticles = 32768;
-// every particle takes the dense kernel: no component copies, no hit lists
+// every particle takes the dense kernel: no hit lists
 static_assert(kNoAllocMaxParticles < pbf::kDenseAllBelow, "the one-thread-per-particle kernel needs its lists");
 constexpr int kNoAllocMaxCells = 131072;
 constexpr size_t kAlign = 256;
@@ -78,7 +78,10 @@ constexpr size_t kOffRho = kOffLambda + align_up(4 * kNp);
 constexpr size_t kOffFlags = kOffRho + align_up(4 * kNp);
 constexpr size_t kOffDense = kOffFlags + align_up(4 * (size_t)pbf::kFlagWords);
 constexpr size_t kOffXl = kOffDense + align_up(4 * pbf::dense_list_len(kNoAllocMaxParticles));
-constexpr size_t kOffCellFlags = kOffXl + align_up(16 * kNp);
+constexpr size_t kComponents = 3 * (size_t)pbf::particle_stride(kNoAllocMaxParticles);
+constexpr size_t kOffSa = kOffXl + align_up(16 * kNp);
+constexpr size_t kOffSb = kOffSa + align_up(4 * kComponents);
+constexpr size_t kOffCellFlags = kOffSb + align_up(4 * kComponents);
 constexpr size_t kSlots = (size_t)kNoAllocMaxParticles / pbf::kGroupCell + 1;
 constexpr size_t kEntries = kNp;
 constexpr size_t kOffGrpCell = kOffCellFlags + align_up(4 * kNc);
@@ -199,6 +202,9 @@ extern "C" pbf_status pbf_step_noalloc(const pbf_params* params, const float uli
   s.flags = (uint32_t*)(base + kOffFlags);
   s.dense = (uint32_t*)(base + kOffDense);
   s.xl = (float4*)(base + kOffXl);
+  s.sa = (float*)(base + kOffSa);
+  s.sb = (float*)(base + kOffSb);
+  s.stride = pbf::particle_stride(kNoAllocMaxParticles);
   s.cell_flags = (uint32_t*)(base + kOffCellFlags);
   s.grp_pool = kNoAllocMaxParticles;
   s.grp_cell = (int*)(base + kOffGrpCell);

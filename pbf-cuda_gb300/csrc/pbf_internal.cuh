@@ -219,11 +219,12 @@ struct SolverScratch {
   uint32_t* flags;     // [kNumFlags] per-step flags and dense-list counters, zeroed by reorder
   uint32_t* dense;     // [dense_list_len(max_particles)] work slots handed to the dense kernels
   float4* xl;          // [max_particles] (position, lambda): the delta_p passes' positions
-  // one-thread-per-particle kernels only (null where no step runs them):
   float* sa;           // [3][stride] component copies of xa and xb
   float* sb;
   int stride;          // particle_stride(max_particles)
-  uint32_t* hits;      // [kHitCap][hit_stride] the lambda pass's hit lists, by thread slot
+  // [kHitCap][hit_stride] the lambda pass's hit lists, by thread slot, or the hit
+  // masks of a step whose particles are all dense (null: none kept)
+  uint32_t* hits;
   int* hit_n;          // [hit_stride] their lengths, or a HitCode
   int hit_stride;      // list_slots(max_particles)
   uint32_t* cell_flags;         // [max_cells + 1] CellFlag bits per cell, zeroed by reorder

@@ -99,7 +99,7 @@ struct PassArgs {
   // the positions by component (x at S, y at S + stride, z at S + 2 stride):
   // the sparse kernel's candidate tests read four at a time
   const float* S;
-  float* S_out;           // delta_p: out, beside T / npos (null when no sparse kernel runs)
+  float* S_out;           // delta_p: out, beside T / npos
   int stride;             // of S
   uint32_t* hits;         // hit lists: lambda writes them, delta_p reads them
   int* hit_n;
@@ -766,7 +766,7 @@ struct DeltaPPass {
     const float4 xf = make_float4(fmaxf(fminf(xi.x + dx, g.hi[0]), g.lo[0]),
                                   fmaxf(fminf(xi.y + dy, g.hi[1]), g.lo[1]),
                                   fmaxf(fminf(xi.z + dz, g.hi[2]), g.lo[2]), 0.f);
-    if (a.S_out) put_components(a.S_out, a.stride, i, xf);
+    put_components(a.S_out, a.stride, i, xf);
     if (!kFinal) {
       a.T[i] = xf;
       return;
@@ -1148,7 +1148,7 @@ struct QueueColumn {
 
 // The hits of one particle in queue entries [0, n), one after the other; the
 // caller counts them.
-template <bool kSecond>
+template <bool kSecond, int kStride>
 struct QueuedHits {
   QueueColumn q;
   uint32_t m = 0u;
@@ -1164,8 +1164,8 @@ struct QueuedHits {
         m = e.x;
         base = (int)e.y;
       }
-      q.run += kSparseThreads;
-      q.second += kSparseThreads;
+      q.run += kStride;
+      q.second += kStride;
     }
     const int bit = __clz(m);  // the first candidate is the highest bit
     m ^= 0x80000000u >> bit;
@@ -1175,10 +1175,10 @@ struct QueuedHits {
 
 // Visits `hits` queued hits in order, two at a time, each two's loads issued
 // two ahead.  out: where the lambda pass lists them (null: nowhere).
-template <int kKind, bool kSecond, class P>
+template <int kKind, bool kSecond, int kStride, class P>
 __device__ __forceinline__ void visit_queued(const PassArgs& a, QueueColumn q, int hits, P& p, uint32_t* out) {
   if (hits == 0) return;
-  QueuedHits<kSecond> h(q);
+  QueuedHits<kSecond, kStride> h(q);
   float4 xa, xb, va = make_float4(0.f, 0.f, 0.f, 0.f), vb = va;
   // the next two hits (the second one the first again when only one is left)
   auto fetch = [&](int left) {
@@ -1252,7 +1252,7 @@ __device__ __forceinline__ void for_chunks(uint2 run, F&& f) {
 template <int kKind, bool kSecond, class P>
 __device__ __forceinline__ int finish_queued(const PassArgs& a, QueueColumn col, int n, int hits, P& p, int h) {
   const bool list = kKind == kLambda && __all_sync(__activemask(), hits <= kHitCap);
-  visit_queued<kKind, kSecond>(a, col, hits, p, list ? a.hits + h : nullptr);
+  visit_queued<kKind, kSecond, kSparseThreads>(a, col, hits, p, list ? a.hits + h : nullptr);
   if (kKind != kLambda || list) return hits;
   int chunks = 0;
   for (int k = 0; k < n; ++k) {
@@ -1587,11 +1587,84 @@ __global__ void __launch_bounds__(kSparseThreads, 8) k_sparse_pair(PassArgs a) {
 
 // kStage: the variant that stages each item's column runs (launched when
 // stage_dense > 0); the other carries no staging code.
+// A part of a window without grouped cells, entries [lo, hi) in visiting order,
+// for a particle that walk_hits would take: the sparse kernel's tests and packed
+// visits.  runs: the window's, 32 apart; q: this thread's queue column.  Where
+// saved is not null the lambda pass leaves the part's chunks with hits there (up
+// to cap of them: mask, first slot; a zero mask ends them, and a slot of ~0 there
+// says that they did not fit).
+constexpr int kPartQueue = 4;
+template <int kKind, class P>
+__device__ __forceinline__ void visit_part(const PassArgs& a, const uint2* runs, int lo, int hi, P& p, QueueColumn q,
+                                           uint32_t* saved, int cap) {
+  const HitTest test(p.xi, a.c.h2);
+  int v0 = 0, chunks = 0, n = 0, hits = 0;
+  for (int r = 0; r < 9; ++r) {
+    const uint2 run = runs[32 * r];
+    const int len = (int)(run.y - run.x);
+    const int from = max(lo - v0, 0), to = min(hi - v0, len);
+    v0 += len;
+    if (from >= to) continue;
+    for_chunks(make_uint2(run.x + from, run.x + to), [&](int base, int groups, uint32_t valid) {
+      uint32_t m = 0u;
+#pragma unroll 4
+      for (int g = 0; g < groups; ++g) m = test.four(Four(a.S, a.stride, base + 4 * g), m);
+      m = ~m << (32 - 4 * groups) & valid;
+      if (!m) return;
+      if (n == kPartQueue) {
+        visit_queued<kKind, false, kDenseThreads>(a, q, hits, p, nullptr);
+        n = hits = 0;
+      }
+      q.run[n * kDenseThreads] = make_uint2(m, (uint32_t)base);
+      ++n;
+      hits += __popc(m);
+      if (saved && chunks < cap) saved[2 * chunks] = m, saved[2 * chunks + 1] = (uint32_t)base;
+      ++chunks;
+    });
+  }
+  visit_queued<kKind, false, kDenseThreads>(a, q, hits, p, nullptr);
+  if (saved && chunks != cap) {
+    const int end = chunks > cap ? 0 : chunks;
+    saved[2 * end] = 0u, saved[2 * end + 1] = chunks > cap ? ~0u : 0u;
+  }
+}
+
+// The same hits from what the lambda pass saved; false if it did not fit.
+template <int kKind, class P>
+__device__ __forceinline__ bool visit_saved(const PassArgs& a, P& p, QueueColumn q, const uint32_t* saved, int cap) {
+  int n = 0, hits = 0;
+  for (int k = 0; k < cap; ++k) {
+    const uint2 e = __ldg(reinterpret_cast<const uint2*>(saved) + k);
+    if (e.x == 0u) {
+      if (e.y != 0u) return false;  // (only the first entry)
+      break;
+    }
+    if (n == kPartQueue) {
+      visit_queued<kKind, false, kDenseThreads>(a, q, hits, p, nullptr);
+      n = hits = 0;
+    }
+    q.run[n * kDenseThreads] = e;
+    ++n;
+    hits += __popc(e.x);
+  }
+  visit_queued<kKind, false, kDenseThreads>(a, q, hits, p, nullptr);
+  return true;
+}
+
+// Steps of few particles are bound by the latency of a pass's chain of loads,
+// not by its work, so the chain is kept short: a block's first batch is its
+// own index, the runs of the batch's windows are loaded by all its warps at once
+// and shared, a part's tests have twelve 16-byte loads in flight, and where every
+// particle is dense the delta_p passes take the hits the lambda pass saved.
+// 1,728 particles: @MEASD1@ us a pass; 65,231: @MEASD2@.
 template <int kKind, bool kStage>
 __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
   using P = typename PassOf<kKind>::type;
+  constexpr bool kDp = kKind == kDeltaP || kKind == kDeltaPFinal;
   __shared__ float part[kDenseWarps][kMaxFields][32];
   __shared__ StageState st;
+  __shared__ uint2 window[kStage ? 1 : kDenseWarps][kStage ? 1 : 9][32];
+  __shared__ uint2 queue[kStage ? 1 : kPartQueue * kDenseThreads];
   // dynamic shared memory: the hit queue (a.c.queue_dense chunks per thread),
   // then the stage (a.c.stage_dense slots, kStage only)
   extern __shared__ __align__(16) float4 dyn_smem[];
@@ -1621,15 +1694,26 @@ __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
   // no grouped cell this step: windows are walked as 9 column runs (the same
   // candidates in the same order as cell by cell, with fewer table reads)
   const bool groups = a.c.keps2 > 0.f && a.flags[kGroupCount] != 0u;
-  // batches are handed out one block-load at a time by a counter, so a block
-  // that drew light batches takes more (batches cost from a few hundred to
-  // many thousand candidates); which block computes a batch changes nothing
+  const bool flat = !kStage && !groups && !a.c.dense_interleave;
+  // a part's share of a particle's 64 words in a.hits (the sparse kernel's lists
+  // are not in use then)
+  const int words = kHitCap >> split_log2;
+  const bool saves = flat && a.dense_all && a.hits != nullptr;
+  // a block's first batches are its index's; then batches are handed out one
+  // block-load at a time by a counter, so a block that drew light batches takes
+  // more (batches cost from a few hundred to many thousand candidates); which
+  // block computes a batch changes nothing
   __shared__ uint32_t s_first;
   uint32_t phase = 0u;
-  for (;;) {
-    if (threadIdx.x == 0) s_first = atomicAdd(&a.flags[a.item_counter], (uint32_t)slots);
-    __syncthreads();  // also: every thread has read the previous s_first
-    const uint32_t first = s_first;
+  const uint32_t own = gridDim.x * (uint32_t)slots;
+  for (bool once = true;; once = false) {
+    uint32_t first = blockIdx.x * (uint32_t)slots;
+    if (!once) {
+      if (own >= count) break;  // uniform over the grid: every batch was some block's own
+      if (threadIdx.x == 0) s_first = own + atomicAdd(&a.flags[a.item_counter], (uint32_t)slots);
+      __syncthreads();  // also: every thread has read the previous s_first
+      first = s_first;
+    }
     if (first >= count) break;  // uniform over the block
     const uint32_t item = first + (uint32_t)slot;
     const uint32_t e = item * 32 + lane;
@@ -1650,25 +1734,53 @@ __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
       __syncthreads();
       staged = stage_wait(st, a, phase);
     }
+    uint32_t* saved = saves ? a.hits + (size_t)t * kHitCap + sub * words : nullptr;
+    const bool fast = flat && !exact && fast_hits(a, xi);
+    if (flat) {  // the windows' runs, each of the item's warps its share of the nine
+      if (valid)
+        for (int r = sub; r < 9; r += split) {
+          int s0 = 0, e0 = 0;
+          const int x = q.x + r / 3 - 1, y = q.y + r % 3 - 1;
+          if (x >= 0 && x < g.dims[0] && y >= 0 && y < g.dims[1]) column_run(g, a.cs, a.n, x, y, q.z, s0, e0);
+          window[kStage ? 0 : slot][kStage ? 0 : r][lane] = make_uint2((uint32_t)s0, (uint32_t)e0);
+        }
+      __syncthreads();
+    }
     if (valid) {
-      const int total = groups ? window_total_grouped(g, a, q) : window_total(g, a.cs, a.n, q);
-      const int lo = (int)(((long long)total * sub) >> split_log2);
-      const int hi = (int)(((long long)total * (sub + 1)) >> split_log2);
       P p(a, g, xi, i, exact);
-      // a staged window holds no grouped cell: its runs are walked as runs;
-      // dense_interleave: the warps take every split-th chunk instead of
-      // one contiguous part (windows without grouped cells)
-      if (kStage && staged) {
-        if (a.c.dense_interleave)
-          visit_window_strided(g, a.cs, a.n, q, FromStage{stage, st.D}, p, sub, split, hq);
-        else
-          visit_window_chunk(g, a.cs, a.n, q, FromStage{stage, st.D}, p, lo, hi, hq);
-      } else if (groups) {
-        visit_window_grouped(g, a, q, FromGlobal{a.X}, p, lo, hi, hq);
-      } else if (a.c.dense_interleave) {
-        visit_window_strided(g, a.cs, a.n, q, FromGlobal{a.X}, p, sub, split, hq);
+      const QueueColumn col{queue + (kStage ? 0 : threadIdx.x), nullptr};
+      if (kDp && fast && saves && visit_saved<kKind>(a, p, col, saved, words / 2)) {
+        // the lambda pass's hits
       } else {
-        visit_window_chunk(g, a.cs, a.n, q, FromGlobal{a.X}, p, lo, hi, hq);
+        int total = 0;
+        if (flat) {
+          for (int r = 0; r < 9; ++r) {
+            const uint2 run = window[kStage ? 0 : slot][kStage ? 0 : r][lane];
+            total += (int)(run.y - run.x);
+          }
+        } else {
+          total = groups ? window_total_grouped(g, a, q) : window_total(g, a.cs, a.n, q);
+        }
+        const int lo = (int)(((long long)total * sub) >> split_log2);
+        const int hi = (int)(((long long)total * (sub + 1)) >> split_log2);
+        // a staged window holds no grouped cell: its runs are walked as runs;
+        // dense_interleave: the warps take every split-th chunk instead of
+        // one contiguous part (windows without grouped cells)
+        if (kStage && staged) {
+          if (a.c.dense_interleave)
+            visit_window_strided(g, a.cs, a.n, q, FromStage{stage, st.D}, p, sub, split, hq);
+          else
+            visit_window_chunk(g, a.cs, a.n, q, FromStage{stage, st.D}, p, lo, hi, hq);
+        } else if (groups) {
+          visit_window_grouped(g, a, q, FromGlobal{a.X}, p, lo, hi, hq);
+        } else if (a.c.dense_interleave) {
+          visit_window_strided(g, a.cs, a.n, q, FromGlobal{a.X}, p, sub, split, hq);
+        } else if (fast) {
+          visit_part<kKind>(a, &window[kStage ? 0 : slot][0][lane], lo, hi, p, col,
+                            kKind == kLambda ? saved : nullptr, words / 2);
+        } else {
+          visit_window_chunk(g, a.cs, a.n, q, FromGlobal{a.X}, p, lo, hi, hq);
+        }
       }
       p.store(&part[warp][0][lane], 32);
     }
@@ -1717,7 +1829,7 @@ k_reorder(const uint32_t* __restrict__ perm, const float4* __restrict__ pos,
   xs[k] = x;
   const float4 xp = make_float4(fmaf(c.dt, vx, x.x), fmaf(c.dt, vy, x.y), fmaf(c.dt, vz, x.z), x.w);
   xa[k] = xp;
-  if (sa) put_components(sa, stride, k, xp);
+  put_components(sa, stride, k, xp);
   iid_s[k] = iid[p];
 }
 
@@ -2218,13 +2330,13 @@ k_follow(const int* __restrict__ follow, int n, StepConsts c, float* __restrict_
   } else if constexpr (kKind == kDeltaP) {
     const float4 t = T[r];
     T[i] = t;
-    if (S_out) put_components(S_out, stride, i, t);
+    put_components(S_out, stride, i, t);
   } else {
     // DeltaPPass<true>::finish with the group's final position
     const float4 xf = npos[r];
     const float4 x0 = xs[i];
     npos[i] = make_float4(xf.x, xf.y, xf.z, x0.w);
-    if (S_out) put_components(S_out, stride, i, xf);
+    put_components(S_out, stride, i, xf);
     const float4 v = make_float4((xf.x - x0.x) * c.inv_dt, (xf.y - x0.y) * c.inv_dt, (xf.z - x0.z) * c.inv_dt, 0.f);
     vel[i] = v;
     VR[i] = make_float4(v.x, v.y, v.z, rho[i]);
@@ -2413,22 +2525,25 @@ cudaError_t run_pass(const PassArgs& a, cudaStream_t stream) {
 }
 
 template <int kKind>
-cudaError_t allow_stage(int bytes) {
-  return cudaFuncSetAttribute(k_dense<kKind, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+cudaError_t allow_stage(int queue, int stage) {
+  cudaError_t e = cudaFuncSetAttribute(k_dense<kKind, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, queue);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_dense<kKind, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, queue + stage);
+  return e;
 }
 
 }  // namespace
 
-// Lets the staged dense kernels take their largest hit queue and up to
+// Lets the dense kernels take their largest hit queue, and the staged ones up to
 // kStageMax staged slots of dynamic shared memory (the current device; call
 // before any capture).
 cudaError_t set_pass_kernel_attributes() {
   const int queue = 8 * kMaxQueueDense * kDenseThreads;
-  const int bytes = (int)sizeof(float4) * kStageMax + queue;
-  cudaError_t e = allow_stage<kLambda>(bytes);
-  if (e == cudaSuccess) e = allow_stage<kDeltaP>(bytes);
-  if (e == cudaSuccess) e = allow_stage<kDeltaPFinal>(bytes);
-  if (e == cudaSuccess) e = allow_stage<kXsph>(bytes);
+  const int stage = (int)sizeof(float4) * kStageMax;
+  cudaError_t e = allow_stage<kLambda>(queue, stage);
+  if (e == cudaSuccess) e = allow_stage<kDeltaP>(queue, stage);
+  if (e == cudaSuccess) e = allow_stage<kDeltaPFinal>(queue, stage);
+  if (e == cudaSuccess) e = allow_stage<kXsph>(queue, stage);
   return e;
 }
 
@@ -2438,7 +2553,7 @@ cudaError_t reorder(const StepConsts& c, const uint32_t* perm, const float4* pos
   if (e == cudaSuccess) e = cudaMemsetAsync(s.flags, 0, sizeof(uint32_t) * kNumFlags, stream);
   if (e != cudaSuccess) return e;
   k_reorder<<<(n + 255) / 256, 256, 0, stream>>>(perm, pos, vel, iid, n, c, s.xs, s.xa,
-                                                  dense_for_all(c, n) ? nullptr : s.sa, s.stride, s.iid_s, s.flags, s.keys_sorted, s.cell_start, s.cell_flags,
+                                                  s.sa, s.stride, s.iid_s, s.flags, s.keys_sorted, s.cell_start, s.cell_flags,
                                                   s.grp_cell, s.grp_off, s.grp_item_off, s.grp_item_slot);
   return cudaGetLastError();
 }
@@ -2467,10 +2582,8 @@ cudaError_t launch_follow(const PassArgs& a, const SolverScratch& s, cudaStream_
   return cudaGetLastError();
 }
 
-// The component copy of position buffer X (null: no sparse kernel reads it).
-float* components_of(const StepConsts& c, const SolverScratch& s, const float4* X, int n) {
-  return dense_for_all(c, n) ? nullptr : (X == s.xa ? s.sa : s.sb);
-}
+// The component copy of position buffer X.
+float* components_of(const SolverScratch& s, const float4* X) { return X == s.xa ? s.sa : s.sb; }
 
 }  // namespace
 
@@ -2481,7 +2594,7 @@ cudaError_t launch_lambda(const StepConsts& c, const Geometry& G, const float4* 
   const bool wl = use_work_list(c, n);
   if (wl && (e = launch_work_list(s, n, stream)) != cudaSuccess) return e;
   PassArgs a = base_args(c, G, X, cs, n, s, pass);
-  a.S = components_of(c, s, X, n);
+  a.S = components_of(s, X);
   if (wl) a.list = s.work_list;
   if (c.order && (e = bucket_by_cell(a, s, n, stream)) != cudaSuccess) return e;
   if ((e = run_pass<kLambda>(a, stream)) != cudaSuccess) return e;
@@ -2494,8 +2607,8 @@ cudaError_t launch_delta_p(const StepConsts& c, const Geometry& G, const float4*
   if (e != cudaSuccess) return e;
   const bool wl = use_work_list(c, n);
   PassArgs a = base_args(c, G, s.xl, cs, n, s, pass);  // X with its lambda
-  a.S = components_of(c, s, X, n);
-  a.S_out = components_of(c, s, T, n);
+  a.S = components_of(s, X);
+  a.S_out = components_of(s, T);
   a.T = T;
   if (wl) a.list = s.work_list;
   if (c.order) use_buckets(a, s);
@@ -2510,9 +2623,9 @@ cudaError_t launch_delta_p_final(const StepConsts& c, const Geometry& G, const f
   if (e != cudaSuccess) return e;
   const bool wl = use_work_list(c, n);
   PassArgs a = base_args(c, G, s.xl, cs, n, s, pass);
-  a.S = components_of(c, s, X, n);
+  a.S = components_of(s, X);
   a.VR = X == s.xa ? s.xb : s.xa;  // the positions go to npos: T's buffers are free
-  a.S_out = components_of(c, s, a.VR, n);
+  a.S_out = components_of(s, a.VR);
   a.xs = s.xs;
   a.iid_s = s.iid_s;
   a.npos = npos;
@@ -2625,7 +2738,7 @@ cudaError_t launch_xsph(const StepConsts& c, const Geometry& G, const float4* X,
   // where the last position update left them: after niter - 1 swaps of xa and
   // xb it read one and used the other
   a.VR = (pass / 2) % 2 ? s.xb : s.xa;
-  a.S = components_of(c, s, a.VR, n);
+  a.S = components_of(s, a.VR);
   a.V = V;
   a.NV = NV;
   if (c.order && (e = bucket_by_cell(a, s, n, stream)) != cudaSuccess) return e;
