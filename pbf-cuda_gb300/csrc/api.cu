@@ -191,6 +191,8 @@ pbf_status check_device_word(uint32_t* word, cudaStream_t stream, const char* wh
   if (bits & pbf::kErrStageTimeout)
     return fail(PBF_ERR_TIMEOUT, "%s: a shared-memory staging copy did not complete in time (the pass read "
                                  "global memory instead)", what);
+  if (bits & pbf::kErrBarrierTimeout)
+    return fail(PBF_ERR_TIMEOUT, "%s: a block of a grid barrier did not arrive in time (the step is not complete)", what);
   return fail(PBF_ERR_CUDA, "%s: device error bits 0x%x", what, bits);
 }
 
@@ -667,8 +669,9 @@ pbf_status enqueue_step(const StepPlan& P, void* pos, void* npos, void* vel, voi
   PBF_EV(P.ev[kEvStart]);
   // advect + buildGridHash (fluids/Simulator.cpp:46-53)
   const uint32_t* perm = nullptr;
+  const pbf::ClearList clear = pbf::step_clears(c, *P.sol);
   PBF_CUDA(pbf::build_grid(c, G, (const float4*)pos, (const float4*)vel, nullptr, n, *P.grid, &perm,
-                           nullptr, st_),
+                           nullptr, st_, &clear),
            "pbf_step: grid");
   PBF_EV(P.ev[kEvGrid]);
   if (P.perm_out) *P.perm_out = perm;
@@ -710,8 +713,8 @@ pbf_status enqueue_step(const StepPlan& P, void* pos, void* npos, void* vel, voi
   }
   // correctVelocity: XSPH (fluids/Simulator.cpp:68-71)
   PBF_EV(P.ev[kEvXsphStart]);
-  PBF_CUDA(pbf::launch_xsph(c, G, (const float4*)npos, (const float4*)vel, cs, n, sol, 2 * niter,
-                            (float4*)nvel, st_),
+  PBF_CUDA(pbf::launch_xsph(c, G, (const float4*)npos, (const float4*)vel, cs, n, sol, 2 * niter, (float4*)pos,
+                            (float4*)npos, (float4*)vel, iid, (float4*)nvel, st_),
            "pbf_step: xsph");
   if (c.vort_eps > 0.f)
     PBF_CUDA(pbf::launch_vorticity(c, G, (const float4*)npos, cs, n, sol, (float4*)nvel, st_),
@@ -862,7 +865,7 @@ pbf_status pbf_step(pbf_solver* s, void* pos, void* npos, void* vel, void* nvel,
   const int niter = s->params.niter;
   s->last_grid_launches = pbf::grid_launches(c, n);
   s->last_launches = s->last_grid_launches + 1 + pbf::pass_launches(c, n) * (2 * niter + 1) +
-                     pbf::group_launches(c, n, niter) + pbf::bucket_launches(c, niter) +
+                     pbf::group_launches(c, n, niter) + pbf::bucket_launches(c, n, niter) +
                      (c.vort_eps > 0.f ? pbf::kVorticityLaunches : 0);
   if (prof) s->prof_iters = niter < kMaxProfiledIters ? niter : kMaxProfiledIters;
   s->last_n = n;

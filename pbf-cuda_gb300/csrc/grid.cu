@@ -121,6 +121,27 @@ k_scan_down(const uint32_t* in, int len, const uint32_t* __restrict__ partials, 
   }
 }
 
+// The whole scan in one block, for arrays of up to kScanOne entries: each
+// thread a contiguous share (read twice; the second time from L1).  The three
+// launches of the general scan cost 7 us at 4,001 entries, this one 2.5.
+constexpr int kScanOne = 32768;
+__global__ void __launch_bounds__(kTopThreads)
+k_scan_one(const uint32_t* in, int len, uint32_t* out, const uint32_t* __restrict__ groups) {
+  // in and out may alias: a thread touches its own share only
+  __shared__ uint32_t smem[kTopThreads / 32 + 1];
+  const bool apart = groups && *groups != 0u;
+  const int items = (len + kTopThreads - 1) / kTopThreads;
+  const int from = min(threadIdx.x * items, len), to = min(from + items, len);
+  uint32_t sum = 0;
+  for (int k = from; k < to; ++k) sum += groups ? pair_slots(in[k], apart) : in[k];
+  uint32_t total;
+  uint32_t run = block_exclusive_scan<kTopThreads>(sum, smem, &total);
+  for (int k = from; k < to; ++k) {
+    const uint32_t v = groups ? pair_slots(in[k], apart) : in[k];
+    out[k] = run;
+    run += v;
+  }
+}
 
 }  // namespace
 
@@ -128,6 +149,10 @@ cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t*
                            const uint32_t* groups) {
   const int tiles = (len + kScanTile - 1) / kScanTile;
   if (tiles > kMaxScanPartials) return cudaErrorInvalidValue;
+  if (len <= kScanOne) {
+    k_scan_one<<<1, kTopThreads, 0, stream>>>(in, len, out, groups);
+    return cudaGetLastError();
+  }
   k_scan_reduce<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, groups);
   k_scan_top<<<1, kTopThreads, 0, stream>>>(partials, tiles);
   k_scan_down<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, out, groups);
@@ -135,6 +160,14 @@ cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t*
 }
 
 namespace {
+
+// Up to three arrays set to zero in one launch.
+__global__ void __launch_bounds__(256) k_clear(ClearList c) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    if (k < c.len[a]) c.words[a][k] = 0u;
+}
 
 // ---- predict + hash ---------------------------------------------------------------
 
@@ -248,6 +281,84 @@ k_radix_downsweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restri
   }
 }
 
+// The whole sort in one block, for steps of up to kSortOne particles: keys and
+// indices stay in registers (thread: 8 of its warp's 256 consecutive items) and
+// go through shared memory once per 7-bit digit.  1,728 particles, 10 key bits:
+// 6.4 us, against 24 in the two passes of five launches.
+constexpr int kSortOneThreads = 1024, kSortOneItems = 8, kSortOne = kSortOneThreads * kSortOneItems;
+constexpr int kSortOneBits = 7, kSortOneDigits = 1 << kSortOneBits;
+__global__ void __launch_bounds__(kSortOneThreads)
+k_sort_one(const uint32_t* __restrict__ keys_in, int n, int passes, uint32_t* __restrict__ keys_out,
+           uint32_t* __restrict__ vals_out) {
+  constexpr int kWarps = kSortOneThreads / 32;
+  __shared__ uint32_t exchange[kSortOne];
+  __shared__ uint16_t whist[kWarps][kSortOneDigits];
+  __shared__ uint32_t first[kSortOneDigits];  // where a digit's items start
+  __shared__ uint32_t smem[kWarps + 1];
+  const int warp = threadIdx.x >> 5;
+  const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1;
+  const int base = warp * (32 * kSortOneItems) + (int)lane;
+  uint32_t key[kSortOneItems], val[kSortOneItems];
+#pragma unroll
+  for (int k = 0; k < kSortOneItems; ++k) {
+    const int idx = base + 32 * k;
+    key[k] = idx < n ? keys_in[idx] : 0xffffffffu;  // the filling sorts behind every particle
+    val[k] = (uint32_t)idx;
+  }
+  for (int pass = 0; pass < passes; ++pass) {
+    const int shift = pass * kSortOneBits;
+    for (int k = threadIdx.x; k < kWarps * kSortOneDigits; k += kSortOneThreads) (&whist[0][0])[k] = 0;
+    __syncthreads();
+    uint32_t at[kSortOneItems];
+#pragma unroll
+    for (int k = 0; k < kSortOneItems; ++k) {
+      const uint32_t d = (key[k] >> shift) & (kSortOneDigits - 1);
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t b = whist[warp][d];
+      __syncwarp();
+      if ((peers & lt) == 0u) whist[warp][d] = (uint16_t)(b + __popc(peers));
+      __syncwarp();
+      at[k] = b + __popc(peers & lt);
+    }
+    __syncthreads();
+    uint32_t count = 0;
+    if (threadIdx.x < kSortOneDigits)
+      for (int w = 0; w < kWarps; ++w) {
+        const uint32_t t = whist[w][threadIdx.x];
+        whist[w][threadIdx.x] = (uint16_t)count;
+        count += t;
+      }
+    uint32_t total;
+    const uint32_t start = block_exclusive_scan<kSortOneThreads>(count, smem, &total);
+    if (threadIdx.x < kSortOneDigits) first[threadIdx.x] = start;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSortOneItems; ++k) {
+      const uint32_t d = (key[k] >> shift) & (kSortOneDigits - 1);
+      at[k] += first[d] + whist[warp][d];
+      exchange[at[k]] = key[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSortOneItems; ++k) key[k] = exchange[base + 32 * k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSortOneItems; ++k) exchange[at[k]] = val[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSortOneItems; ++k) val[k] = exchange[base + 32 * k];
+    __syncthreads();
+  }
+#pragma unroll
+  for (int k = 0; k < kSortOneItems; ++k) {
+    const int idx = base + 32 * k;
+    if (idx < n) {
+      keys_out[idx] = key[k];
+      vals_out[idx] = val[k];
+    }
+  }
+}
+
 __global__ void k_export_ranges(const uint32_t* __restrict__ cs, int cells,
                                 uint32_t* __restrict__ start, uint32_t* __restrict__ end) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -265,11 +376,14 @@ int key_bits(int cells) {
 
 }  // namespace
 
+int scan_launches(int len) { return len <= kScanOne ? 1 : 3; }
+
 int grid_launches(const StepConsts& c, int n) {
-  (void)n;
   const int bits = key_bits(c.cells);
   const int passes = bits > 0 ? (bits + kRadixBits - 1) / kRadixBits : 1;
-  return 1 + 3 + passes * (1 + 3 + 1);  // hash, cell scan, passes x (upsweep, scan, downsweep)
+  // clear, hash, cell scan, then the sort: one launch, or passes x (upsweep, scan, downsweep)
+  return 2 + scan_launches(c.cells + 1) +
+         (n <= kSortOne ? 1 : passes * (2 + scan_launches(kRadix * sort_tiles(n))));
 }
 
 int sort_tiles(int n) { return (n + kSortTile - 1) / kSortTile; }
@@ -280,11 +394,15 @@ size_t radix_counts_len(int max_particles) {
 
 cudaError_t build_grid(const StepConsts& c, const Geometry& G, const float4* pos, const float4* vel,
                        const float4* xstar, int n, GridScratch& s, const uint32_t** perm_out,
-                       uint32_t* keys_copy, cudaStream_t stream) {
+                       uint32_t* keys_copy, cudaStream_t stream, const ClearList* clear) {
   cudaError_t err;
   const int cells1 = c.cells + 1;
-  if ((err = cudaMemsetAsync(s.cell_count, 0, sizeof(uint32_t) * cells1, stream)) != cudaSuccess)
-    return err;
+  ClearList cl = {};
+  if (clear) cl = *clear;
+  cl.words[2] = s.cell_count;
+  cl.len[2] = cells1;
+  const int longest = max(max(cl.len[0], cl.len[1]), cl.len[2]);
+  k_clear<<<(longest + 255) / 256, 256, 0, stream>>>(cl);
   const int blocks = (n + 255) / 256;
   if (xstar)
     k_hash<false><<<blocks, 256, 0, stream>>>(xstar, nullptr, n, c, G, s.keys_a, s.cell_count);
@@ -301,6 +419,13 @@ cudaError_t build_grid(const StepConsts& c, const Geometry& G, const float4* pos
 
   // LSD passes over the key bits; at least one pass so perm is always written.
   const int bits = key_bits(c.cells);
+  if (n <= kSortOne) {
+    const int digits = bits > 0 ? (bits + kSortOneBits - 1) / kSortOneBits : 1;
+    k_sort_one<<<1, kSortOneThreads, 0, stream>>>(s.keys_a, n, digits, s.keys_b, s.vals_a);
+    s.keys_sorted = s.keys_b;
+    *perm_out = s.vals_a;
+    return cudaGetLastError();
+  }
   const int passes = bits > 0 ? (bits + kRadixBits - 1) / kRadixBits : 1;
   const int ntiles = sort_tiles(n);
   const int clen = kRadix * ntiles;

@@ -243,10 +243,11 @@ extern "C" pbf_status pbf_step_noalloc(const pbf_params* params, const float uli
       (e = cudaMemsetAsync(base + kOffGrpListN, 0, kOffGrpZero - kOffGrpListN, strm)) != cudaSuccess)
     return pbf::set_cuda_error(e, "pbf_step_noalloc: clear");
   const uint32_t* perm = nullptr;
-  // build_grid clears the per-cell counters itself (cudaMemsetAsync, no allocation)
+  // build_grid clears the per-cell counters itself (a kernel, no allocation)
   const pbf::Geometry G{nullptr, nullptr};
-  if ((e = pbf::build_grid(c, G, (const float4*)pos, (const float4*)vel, nullptr, n, g, &perm, nullptr,
-                           strm)) != cudaSuccess)
+  const pbf::ClearList clear = pbf::step_clears(c, s);
+  if ((e = pbf::build_grid(c, G, (const float4*)pos, (const float4*)vel, nullptr, n, g, &perm, nullptr, strm,
+                           &clear)) != cudaSuccess)
     return pbf::set_cuda_error(e, "pbf_step_noalloc: grid");
   s.keys_sorted = g.keys_sorted;
   s.cell_start = g.cell_start;
@@ -270,7 +271,7 @@ extern "C" pbf_status pbf_step_noalloc(const pbf_params* params, const float uli
     }
   }
   if ((e = pbf::launch_xsph(c, G, (const float4*)npos, (const float4*)vel, g.cell_start, n, s, 2 * niter,
-                            (float4*)nvel, strm)) != cudaSuccess)
+                            (float4*)pos, (float4*)npos, (float4*)vel, iid, (float4*)nvel, strm)) != cudaSuccess)
     return pbf::set_cuda_error(e, "pbf_step_noalloc: xsph");
   if (c.vort_eps > 0.f &&
       (e = pbf::launch_vorticity(c, G, (const float4*)npos, g.cell_start, n, s, (float4*)nvel, strm)) != cudaSuccess)

@@ -193,6 +193,12 @@ constexpr int kSortTile = 2048;
 int sort_tiles(int n);
 size_t radix_counts_len(int max_particles);
 
+// Two arrays of words that a step starts from zero, cleared with the grid's own.
+struct ClearList {
+  uint32_t* words[3];
+  int len[3];
+};
+
 // Hash (optionally predicting x* = x + dt (v + dt g) first), count cells,
 // stable radix sort by cell id, exclusive prefix of counts.
 //   pos/vel != null: predict from them;  xstar != null: hash xstar directly.
@@ -201,7 +207,7 @@ size_t radix_counts_len(int max_particles);
 // keys_copy (optional, n entries) receives the unsorted cell ids.
 cudaError_t build_grid(const StepConsts& c, const Geometry& G, const float4* pos, const float4* vel,
                        const float4* xstar, int n, GridScratch& s, const uint32_t** perm_out,
-                       uint32_t* keys_copy, cudaStream_t stream);
+                       uint32_t* keys_copy, cudaStream_t stream, const ClearList* clear = nullptr);
 
 // start/end per cell in the reference's format (0/0 for empty cells).
 cudaError_t export_ranges(const StepConsts& c, const uint32_t* cell_start, uint32_t* start,
@@ -216,7 +222,7 @@ struct SolverScratch {
   uint32_t* iid_s;     // sorted iid
   float* lambda;
   float* rho;
-  uint32_t* flags;     // [kNumFlags] per-step flags and dense-list counters, zeroed by reorder
+  uint32_t* flags;     // [kNumFlags] per-step flags and dense-list counters, zero when a step starts (step_clears)
   uint32_t* dense;     // [dense_list_len(max_particles)] work slots handed to the dense kernels
   float4* xl;          // [max_particles] (position, lambda): the delta_p passes' positions
   float* sa;           // [3][stride] component copies of xa and xb
@@ -227,7 +233,7 @@ struct SolverScratch {
   uint32_t* hits;
   int* hit_n;          // [hit_stride] their lengths, or a HitCode
   int hit_stride;      // list_slots(max_particles)
-  uint32_t* cell_flags;         // [max_cells + 1] CellFlag bits per cell, zeroed by reorder
+  uint32_t* cell_flags;         // [max_cells + 1] CellFlag bits per cell, zero when a step starts (step_clears)
   const uint32_t* keys_sorted;  // the grid's sorted cell ids (set before the passes)
   const uint32_t* cell_start;   // the grid's cell prefix (set before the passes)
   // group tables of the cells holding >= kGroupCell particles (one slot each);
@@ -352,7 +358,12 @@ enum StepFlag {
   kBucketCount = 10,         // particles in the current buckets
   kItemCount0 = 11,          // dense-kernel batches handed out, by pass parity (work queue)
   kItemCount1 = 12,
-  kNumFlags = 13
+  kMoved0 = 13,              // small steps: particles outside their grid cell, by iteration parity
+  kMoved1 = 14,
+  kBucketIdentity = 15,      // 1: the current buckets are every particle, in order
+  kBarrierCount = 16,        // grid_barrier
+  kBarrierGen = 17,
+  kNumFlags = 18
 };
 
 // One more word after the step flags, cleared only when the host reads it:
@@ -361,6 +372,7 @@ constexpr int kErrorWord = kNumFlags;
 constexpr int kFlagWords = kNumFlags + 1;
 enum ErrorBit : uint32_t {
   kErrStageTimeout = 1u,     // a shared-memory staging copy did not complete in time
+  kErrBarrierTimeout = 2u,   // a block of a small step's grid barrier did not arrive in time
 };
 
 // Largest stage (slots, 16 bytes each) a dense-kernel block may ask for; the
@@ -372,6 +384,8 @@ cudaError_t set_pass_kernel_attributes();
 // Entries of the dense list: one per particle.
 constexpr size_t dense_list_len(int max_particles) { return (size_t)max_particles + 1; }
 
+// What reorder and the passes expect at zero when a step starts (build_grid's clear).
+ClearList step_clears(const StepConsts& c, const SolverScratch& s);
 // Gather pos/vel/iid into cell order and recompute x* (bit-identical to the hash).
 cudaError_t reorder(const StepConsts& c, const uint32_t* perm, const float4* pos, const float4* vel,
                     const uint32_t* iid, int n, SolverScratch& s, cudaStream_t stream);
@@ -392,8 +406,10 @@ cudaError_t launch_delta_p_final(const StepConsts& c, const Geometry& G, const f
                                  const SolverScratch& s, int pass, float4* pos, float4* npos,
                                  float4* vel, uint32_t* iid, cudaStream_t stream);
 // XSPH: nvel = vel + c sum_j 2 (v_j - v_i) W / (rho_i + rho_j).
+// pos, npos, vel, iid: as launch_delta_p_final had them.
 cudaError_t launch_xsph(const StepConsts& c, const Geometry& G, const float4* X, const float4* V, const uint32_t* cs,
-                        int n, const SolverScratch& s, int pass, float4* NV, cudaStream_t stream);
+                        int n, const SolverScratch& s, int pass, float4* pos, float4* npos, float4* vel,
+                        uint32_t* iid, float4* NV, cudaStream_t stream);
 
 // Candidates above which a warp takes the dense kernel, and the particle
 // count below which every warp does (defaults; pbf_autotune can override).
@@ -513,16 +529,20 @@ cudaError_t backward(const BackwardArgs& args, const BackwardTape& tape, const u
                      const void* g_npos, const void* g_nvel, void* g_pos, void* g_vel, float* g_lim,
                      cudaStream_t stream);
 
-// Exclusive prefix of in[0, len) into out (may alias in): 3 launches,
-// partials holds kMaxScanPartials entries.  groups: of pair_slots of the values,
+// Exclusive prefix of in[0, len) into out (may alias in): one launch for short
+// arrays or three (scan_launches); partials holds kMaxScanPartials entries.  groups: of pair_slots of the values,
 // apart where *groups (device) is not zero.
 cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t* partials, cudaStream_t stream,
                            const uint32_t* groups = nullptr);
 
-// Launches (and memset nodes) of one bucketing by current cell; an ordered
+int scan_launches(int len);
+
+// Launches (and memset nodes) of a step's bucketings by current cell; an ordered
 // step buckets before every lambda pass and before XSPH.
-constexpr int kBucketLaunches = 6;
-inline int bucket_launches(const StepConsts& c, int niter) { return c.order ? kBucketLaunches * (niter + 1) : 0; }
+bool is_small(const StepConsts& c, int n);  // see solver.cu
+inline int bucket_launches(const StepConsts& c, int n, int niter) {
+  return c.order && !is_small(c, n) ? (3 + scan_launches(c.cells + 1)) * (niter + 1) : 0;
+}
 
 // Kernel launches of one build_grid call with n particles and c.cells cells.
 int grid_launches(const StepConsts& c, int n);

@@ -137,6 +137,7 @@ struct PassArgs {
   // empty slot holds -1): the sparse kernel of the lambda and xsph passes takes
   // the two slots of a pair in one thread
   int paired;
+  int moved_word;         // delta_p: a flag counting the particles that left their grid cell (-1: none)
 };
 
 // The particle that thread slot t of a pass computes (t < work_count(a)).
@@ -767,6 +768,12 @@ struct DeltaPPass {
                                   fmaxf(fminf(xi.y + dy, g.hi[1]), g.lo[1]),
                                   fmaxf(fminf(xi.z + dz, g.hi[2]), g.lo[2]), 0.f);
     put_components(a.S_out, a.stride, i, xf);
+    if (a.moved_word >= 0) {  // how many leave their grid cell
+      const int3 q = cell_of(c, g, xf);
+      const bool moved = (uint32_t)cell_index(g, q.x, q.y, q.z) != a.skeys[i];
+      const unsigned act = __activemask(), left = __ballot_sync(act, moved);
+      if (left && (threadIdx.x & 31) == __ffs(act) - 1) atomicAdd(&a.flags[a.moved_word], (uint32_t)__popc(left));
+    }
     if (!kFinal) {
       a.T[i] = xf;
       return;
@@ -1656,7 +1663,8 @@ __device__ __forceinline__ bool visit_saved(const PassArgs& a, P& p, QueueColumn
 // own index, the runs of the batch's windows are loaded by all its warps at once
 // and shared, a part's tests have twelve 16-byte loads in flight, and where every
 // particle is dense the delta_p passes take the hits the lambda pass saved.
-// 1,728 particles: @MEASD1@ us a pass; 65,231: @MEASD2@.
+// 1,728 particles: lambda 13.1 -> 9.0 us, delta_p 15.7 -> 7.2;
+// 65,231: 36 -> 36 and 43 -> 26.
 template <int kKind, bool kStage>
 __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
   using P = typename PassOf<kKind>::type;
@@ -1992,7 +2000,7 @@ __device__ __forceinline__ bool last_item(const GroupArgs& a, const Item& it, in
 // writes rep, cnt, pos (and for xsph aux = the first particle's velocity and
 // sum.w = its density), h_rank, ng, and clears the claimed entries.
 template <int kWhat>
-__global__ void __launch_bounds__(kGroupThreads) k_group_insert(GroupArgs a) {
+__device__ __forceinline__ void group_insert(const GroupArgs& a) {
   __shared__ int sh[80];
   __shared__ int s_last;
   __shared__ int s_buf[2 * kGroupList];
@@ -2131,7 +2139,7 @@ __device__ __forceinline__ float group_dev(const GroupArgs& a, const Item& it, i
 }
 
 // Fixed-point sums over each group of (value - the group's first particle's
-// value), two kernels.  k_group_devmax: the largest |deviation| per group
+// value), two kernels.  group_devmax: the largest |deviation| per group
 // (atomicMax on the float bits; +inf marks a non-finite deviation); the last
 // block of a slot sets ng = -1 on a non-finite one and zero[slot] when every
 // deviation is 0.  k_group_devsum: each deviation scaled by 2^sh, sh from the
@@ -2139,7 +2147,7 @@ __device__ __forceinline__ float group_dev(const GroupArgs& a, const Item& it, i
 // free, exact to 2^-62 of the bound); the last block writes the sums
 // (lambda: sum = (lambda_rep, sum dev); xsph: sum.xyz) and clears gmax / acc.
 template <int kWhat>
-__global__ void __launch_bounds__(kGroupThreads) k_group_devmax(GroupArgs a) {
+__device__ __forceinline__ void group_devmax(const GroupArgs& a) {
   constexpr int C = kWhat == kGroupsLambda ? 1 : 3;
   __shared__ int s_last, s_flag;
   const int items = (int)a.flags[kGroupItems];
@@ -2183,7 +2191,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_devmax(GroupArgs a) {
 }
 
 template <int kWhat>
-__global__ void __launch_bounds__(kGroupThreads) k_group_devsum(GroupArgs a) {
+__device__ __forceinline__ void group_devsum(const GroupArgs& a) {
   constexpr int C = kWhat == kGroupsLambda ? 1 : 3;
   __shared__ int s_last;
   const int items = (int)a.flags[kGroupItems];
@@ -2234,6 +2242,19 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_devsum(GroupArgs a) {
   }
 }
 
+template <int kWhat>
+__global__ void __launch_bounds__(kGroupThreads) k_group_insert(GroupArgs a) {
+  group_insert<kWhat>(a);
+}
+template <int kWhat>
+__global__ void __launch_bounds__(kGroupThreads) k_group_devmax(GroupArgs a) {
+  group_devmax<kWhat>(a);
+}
+template <int kWhat>
+__global__ void __launch_bounds__(kGroupThreads) k_group_devsum(GroupArgs a) {
+  group_devsum<kWhat>(a);
+}
+
 // ---- work lists: one computing particle per position group -----------------------------
 
 static_assert(kWorkThreads == kGroupThreads, "the work-list kernels use the group kernels' block scan");
@@ -2243,11 +2264,25 @@ static_assert(kWorkThreads == kGroupThreads, "the work-list kernels use the grou
 // particle when particle i of a grouped cell is not that particle, else -1;
 // blocks[b] = the computing particles of block b.  The block that finishes
 // last turns blocks[] into exclusive offsets (so the list is in cell order).
-__global__ void __launch_bounds__(kWorkThreads)
-k_work_mark(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ cell_flags,
-            const int* __restrict__ grp_n, const int* __restrict__ grp_off, const int* __restrict__ grp_id,
-            const int* __restrict__ grp_hash, const int* __restrict__ grp_rep, int np, int n,
-            int* __restrict__ follow, int* __restrict__ blocks, uint32_t* __restrict__ flags) {
+struct WorkArgs {
+  const uint32_t* skeys;
+  const uint32_t* cell_flags;
+  const int* grp_n;
+  const int* grp_off;
+  const int* grp_id;
+  const int* grp_hash;
+  const int* grp_rep;
+  int np, n;
+  int* follow;
+  int* blocks;
+  int* list;
+  uint32_t* flags;
+};
+
+__device__ __forceinline__ void work_mark(const WorkArgs& w) {
+  uint32_t* flags = w.flags;
+  int* blocks = w.blocks;
+  const int n = w.n, np = w.np;
   __shared__ int sh[80];
   __shared__ int s_last;
   if (flags[kGroupCount] == 0u) {  // no grouped cell this step: every particle computes, in order
@@ -2260,18 +2295,18 @@ k_work_mark(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ cel
   const int i = blockIdx.x * kWorkThreads + threadIdx.x;
   int r = -1;
   if (i < n) {
-    const uint32_t sl = cell_flags[skeys[i]] >> kCellSlotShift;
+    const uint32_t sl = w.cell_flags[w.skeys[i]] >> kCellSlotShift;
     if (sl) {
       const int slot = (int)sl - 1;
-      if (grp_n[slot] > 0) {
+      if (w.grp_n[slot] > 0) {
         // the particle's hash entry -> its group's rank -> the group's first particle
-        const int t0 = grp_off[slot];
-        const int rank = grp_hash[2 * t0 + 6 * np + grp_id[i]];
-        const int rep = grp_rep[t0 + rank];
+        const int t0 = w.grp_off[slot];
+        const int rank = w.grp_hash[2 * t0 + 6 * np + w.grp_id[i]];
+        const int rep = w.grp_rep[t0 + rank];
         if (rep != i) r = rep;
       }
     }
-    follow[i] = r;
+    w.follow[i] = r;
   }
   const int cnt = __syncthreads_count(i < n && r < 0);
   if (threadIdx.x == 0) blocks[blockIdx.x] = cnt;
@@ -2298,55 +2333,55 @@ k_work_mark(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ cel
 }
 
 // list[blocks[b] + rank] = i for the computing particles of block b, in order.
-__global__ void __launch_bounds__(kWorkThreads)
-k_work_list(const int* __restrict__ follow, const int* __restrict__ blocks, int n, int* __restrict__ list,
-            const uint32_t* __restrict__ flags) {
+__device__ __forceinline__ void work_list(const WorkArgs& w) {
   __shared__ int sh[80];
-  if (flags[kWorkIdentity]) return;
+  if (w.flags[kWorkIdentity]) return;
   const int i = blockIdx.x * kWorkThreads + threadIdx.x;
-  const bool keep = i < n && follow[i] < 0;
+  const bool keep = i < w.n && w.follow[i] < 0;
   int total;
   const int rank = block_scan(keep, sh, total);
-  if (keep) list[blocks[blockIdx.x] + rank] = i;
+  if (keep) w.list[w.blocks[blockIdx.x] + rank] = i;
 }
+
+__global__ void __launch_bounds__(kWorkThreads) k_work_mark(WorkArgs w) { work_mark(w); }
+__global__ void __launch_bounds__(kWorkThreads) k_work_list(WorkArgs w) { work_list(w); }
 
 // The followers take their group's results.
 template <int kKind>
-__global__ void __launch_bounds__(256)
-k_follow(const int* __restrict__ follow, int n, StepConsts c, float* __restrict__ lambda, float4* __restrict__ XL,
-         float* __restrict__ rho, float4* __restrict__ T, float* __restrict__ S_out, int stride,
-         float4* __restrict__ VR, const float4* __restrict__ xs,
-         const uint32_t* __restrict__ iid_s, float4* __restrict__ npos, float4* __restrict__ vel,
-         float4* __restrict__ pos, uint32_t* __restrict__ iid, const uint32_t* __restrict__ skeys,
-         uint32_t* __restrict__ cell_flags, uint32_t* __restrict__ flags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || flags[kWorkIdentity]) return;
+__device__ __forceinline__ void follow_group(const PassArgs& a, const int* follow, int i) {
+  if (i >= a.n || a.flags[kWorkIdentity]) return;
   const int r = follow[i];
   if (r < 0) return;
   if constexpr (kKind == kLambda) {
-    lambda[i] = lambda[r];
-    rho[i] = rho[r];
-    XL[i] = XL[r];  // the same position
+    a.lambda[i] = a.lambda[r];
+    a.rho[i] = a.rho[r];
+    a.XL[i] = a.XL[r];  // the same position
   } else if constexpr (kKind == kDeltaP) {
-    const float4 t = T[r];
-    T[i] = t;
-    put_components(S_out, stride, i, t);
+    const float4 t = a.T[r];
+    a.T[i] = t;
+    put_components(a.S_out, a.stride, i, t);
   } else {
     // DeltaPPass<true>::finish with the group's final position
-    const float4 xf = npos[r];
-    const float4 x0 = xs[i];
-    npos[i] = make_float4(xf.x, xf.y, xf.z, x0.w);
-    put_components(S_out, stride, i, xf);
-    const float4 v = make_float4((xf.x - x0.x) * c.inv_dt, (xf.y - x0.y) * c.inv_dt, (xf.z - x0.z) * c.inv_dt, 0.f);
-    vel[i] = v;
-    VR[i] = make_float4(v.x, v.y, v.z, rho[i]);
+    const float4 xf = a.npos[r];
+    const float4 x0 = a.xs[i];
+    a.npos[i] = make_float4(xf.x, xf.y, xf.z, x0.w);
+    put_components(a.S_out, a.stride, i, xf);
+    const float4 v = make_float4((xf.x - x0.x) * a.c.inv_dt, (xf.y - x0.y) * a.c.inv_dt,
+                                 (xf.z - x0.z) * a.c.inv_dt, 0.f);
+    a.vel[i] = v;
+    a.VR[i] = make_float4(v.x, v.y, v.z, a.rho[i]);
     if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z)) {
-      atomicOr(&cell_flags[skeys[i]], (uint32_t)kCellVelNonFinite);
-      atomicOr(&flags[kFlagXsphExact], 1u);
+      atomicOr(&a.cell_flags[a.skeys[i]], (uint32_t)kCellVelNonFinite);
+      atomicOr(&a.flags[kFlagXsphExact], 1u);
     }
-    pos[i] = x0;
-    iid[i] = iid_s[i];
+    a.pos[i] = x0;
+    a.iid[i] = a.iid_s[i];
   }
+}
+
+template <int kKind>
+__global__ void __launch_bounds__(256) k_follow(PassArgs a, const int* __restrict__ follow) {
+  follow_group<kKind>(a, follow, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // ---- current-cell order ---------------------------------------------------------------
@@ -2358,11 +2393,8 @@ k_follow(const int* __restrict__ follow, int n, StepConsts c, float* __restrict_
 // load the same candidates and run similar loops.  A particle's result does
 // not depend on its place in the list (sparse / dense routing is per
 // particle), so the arbitrary ranks leave results bitwise reproducible.
-__global__ void __launch_bounds__(256) k_bucket_count(PassArgs a, uint32_t* __restrict__ bcnt,
-                                                      uint2* __restrict__ bent) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= work_count(a)) return;
-  const int i = work_particle(a, t);
+// t: a slot of the pass's list (its particle i), or any beyond it (i unused).
+__device__ __forceinline__ void bucket_count(const PassArgs& a, int t, int i, uint32_t* bcnt, uint2* bent) {
   const SceneGeom g = geom_of(a.c, a.G, i);
   const int3 q = cell_of(a.c, g, a.X[i]);
   const uint32_t cell = (uint32_t)cell_index(g, q.x, q.y, q.z);
@@ -2374,6 +2406,12 @@ __global__ void __launch_bounds__(256) k_bucket_count(PassArgs a, uint32_t* __re
   if (lane == leader) base = atomicAdd(&bcnt[cell], (uint32_t)__popc(same));
   base = __shfl_sync(same, base, leader);
   bent[t] = make_uint2(cell, base + (uint32_t)__popc(same & ((1u << lane) - 1u)));
+}
+
+__global__ void __launch_bounds__(256) k_bucket_count(PassArgs a, uint32_t* __restrict__ bcnt,
+                                                      uint2* __restrict__ bent) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < work_count(a)) bucket_count(a, t, work_particle(a, t), bcnt, bent);
 }
 
 // bstart: the prefix of the counts, or where a.paired of pair_slots of them (the
@@ -2420,6 +2458,238 @@ GroupArgs group_args(const SolverScratch& s, const float4* X, const float4* V, i
   a.acc = s.grp_acc;
   a.zero = s.grp_zero;
   return a;
+}
+
+// Whether the lambda / delta_p passes run on work lists (groups exist only
+// from kGroupCell particles on, and the zero gradient of co-located particles
+// needs kernel_eps > 0).
+bool use_work_list(const StepConsts& c, int n) { return n >= kGroupCell && c.keps2 > 0.f; }
+
+WorkArgs work_args(const SolverScratch& s, int n) {
+  return WorkArgs{s.keys_sorted, s.cell_flags, s.grp_n, s.grp_off, s.grp_id,      s.grp_hash,    s.grp_rep,
+                  s.grp_pool,    n,            s.work_follow, s.work_blocks, s.work_list, s.flags};
+}
+
+// ---- small steps: the work around a pass in one launch -----------------------------------
+//
+// A step of a few thousand particles spends its time in launches (2 us each,
+// whatever they do): group tables, work list, followers and buckets took 13 of
+// the 15 launches of an iteration.  In a small step (is_small: every particle
+// dense, one 1,024-thread block per 1,024 particles fits on the chip at once)
+// everything between two passes is one cooperative launch, its phases separated
+// by grid barriers and skipped where the step has no grouped cells:
+//   k_small_before   (lambda, xsph)  the followers of the last delta_p pass, the
+//                    position (xsph: position and density) groups, the work list,
+//                    the buckets
+//   k_small_between  (delta_p)       the lambda pass's followers, the sums of
+//                    lambda
+// The buckets are built only where they matter: with groups, or when more than
+// one particle in kMovedShare has left its grid cell (the delta_p passes count
+// them); else the passes take the particles in grid order, which is then nearly
+// the current cells' (the order changes no result).
+// A step: 209 -> 99 us (1,728 particles), 214 -> 113 (8,000).
+
+constexpr int kMovedShare = 8;
+constexpr int kBarrierSpins = 1 << 21;
+
+// Every block of the (cooperative) grid arrives before any goes on; writes
+// before it are visible after it.  Bounded: a block that waited kBarrierSpins
+// polls records kErrBarrierTimeout and returns false (its caller returns).
+__device__ __forceinline__ bool grid_barrier(uint32_t* flags) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    volatile uint32_t* gen = &flags[kBarrierGen];
+    const uint32_t g = *gen;
+    int ok = 1;
+    __threadfence();
+    if (atomicAdd(&flags[kBarrierCount], 1u) == gridDim.x - 1) {
+      flags[kBarrierCount] = 0u;
+      __threadfence();
+      atomicAdd(&flags[kBarrierGen], 1u);
+    } else {
+      int k = 0;
+      while (*gen == g && ++k < kBarrierSpins) {
+      }
+      if (k >= kBarrierSpins) {
+        ok = 0;
+        atomicOr(&flags[kErrorWord], (uint32_t)kErrBarrierTimeout);
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+struct SmallArgs {
+  PassArgs p;        // the pass that follows
+  GroupArgs g;
+  WorkArgs w;
+  uint32_t* bcnt;
+  uint32_t* bstart;
+  uint2* bent;
+  int* bucket;
+  uint32_t* bpart;
+  int iteration;     // of the pass (xsph: niter)
+  int groups;        // the step may have grouped cells
+  int buckets;       // current-cell order is on
+};
+
+// kLast: the delta_p pass whose followers come first (kDeltaPFinal: xsph follows).
+template <int kLast>
+__global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
+  constexpr bool kXsphNext = kLast == kDeltaPFinal;
+  uint32_t* flags = a.p.flags;
+  const int i = blockIdx.x * kWorkThreads + threadIdx.x;
+  const bool groups = a.groups && flags[kGroupCount] != 0u;
+  if (groups) {
+    if (a.iteration > 0) {
+      follow_group<kLast>(a.p, a.w.follow, i);
+      if (!grid_barrier(flags)) return;
+    }
+    if constexpr (kXsphNext) {
+      group_insert<kGroupsXsph>(a.g);
+      if (!grid_barrier(flags)) return;
+      group_devmax<kGroupsXsph>(a.g);
+      if (!grid_barrier(flags)) return;
+      group_devsum<kGroupsXsph>(a.g);
+    } else {
+      group_insert<kGroupsPos>(a.g);
+      if (!grid_barrier(flags)) return;
+      work_mark(a.w);
+      if (!grid_barrier(flags)) return;
+      work_list(a.w);
+      if (!grid_barrier(flags)) return;
+    }
+  } else if (!kXsphNext && i == 0) {
+    flags[kWorkCount] = (uint32_t)a.p.n;
+    flags[kWorkIdentity] = 1u;
+  }
+  if (!a.buckets) return;
+  // the count this iteration's delta_p pass adds to (the last one's is read here)
+  if (i == 0) flags[kMoved0 + (a.iteration & 1)] = 0u;
+  const uint32_t moved = a.iteration > 0 ? flags[kMoved0 + ((a.iteration + 1) & 1)] : 0u;
+  if (!groups && moved <= (uint32_t)a.p.n / kMovedShare) {  // uniform over the grid
+    if (i == 0) {
+      flags[kBucketIdentity] = 1u;
+      flags[kBucketCount] = (uint32_t)a.p.n;
+    }
+    return;
+  }
+  // count, exclusive scan over the cells (every block a share), scatter
+  const int cells1 = a.p.c.cells + 1, threads = gridDim.x * kWorkThreads;
+  for (int k = i; k < cells1; k += threads) a.bcnt[k] = 0u;
+  if (!grid_barrier(flags)) return;
+  // the list: the work list of a step with groups (lambda), else every particle
+  const bool listed = groups && !kXsphNext;
+  const int count = listed ? (int)flags[kWorkCount] : a.p.n;
+  const int j = i < count ? (listed && !flags[kWorkIdentity] ? a.w.list[i] : i) : 0;
+  if (i < count) bucket_count(a.p, i, j, a.bcnt, a.bent);
+  if (!grid_barrier(flags)) return;
+  __shared__ int sh[80];
+  const int per_block = (cells1 + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int per_thread = (per_block + kWorkThreads - 1) / kWorkThreads;
+  const int end = min((int)(blockIdx.x + 1) * per_block, cells1);
+  const int from = min((int)blockIdx.x * per_block + (int)threadIdx.x * per_thread, end);
+  const int to = min(from + per_thread, end);
+  int sum = 0;
+  for (int k = from; k < to; ++k) sum += (int)a.bcnt[k];
+  int total;
+  int run = block_scan_value(sum, sh, total);
+  if (threadIdx.x == 0) a.bpart[blockIdx.x] = (uint32_t)total;
+  if (!grid_barrier(flags)) return;
+  int before;  // the sum of the blocks before this one
+  block_scan_value(threadIdx.x < blockIdx.x ? (int)a.bpart[threadIdx.x] : 0, sh, before);
+  run += before;
+  for (int k = from; k < to; ++k) {
+    a.bstart[k] = (uint32_t)run;
+    run += (int)a.bcnt[k];
+  }
+  if (!grid_barrier(flags)) return;
+  if (i == 0) {
+    flags[kBucketIdentity] = 0u;
+    flags[kBucketCount] = (uint32_t)count;
+  }
+  if (i < count) {
+    const uint2 e = a.bent[i];
+    a.bucket[a.bstart[e.x] + e.y] = j;
+  }
+}
+
+__global__ void __launch_bounds__(kWorkThreads, 1) k_small_between(SmallArgs a) {
+  if (a.p.flags[kGroupCount] == 0u) return;
+  follow_group<kLambda>(a.p, a.w.follow, blockIdx.x * kWorkThreads + threadIdx.x);
+  if (!grid_barrier(a.p.flags)) return;
+  group_devmax<kGroupsLambda>(a.g);
+  if (!grid_barrier(a.p.flags)) return;
+  group_devsum<kGroupsLambda>(a.g);
+}
+
+// Points a small step's pass at its particles: the buckets, or the work list.
+void small_list(PassArgs& a, const SolverScratch& s, bool xsph) {
+  a.paired = 0;
+  if (a.c.order) {
+    a.list = s.bucket;
+    a.count_word = kBucketCount;
+    a.identity_word = kBucketIdentity;
+  } else if (!xsph && use_work_list(a.c, a.n)) {
+    a.list = s.work_list;  // with its own count and identity
+  }
+}
+
+SmallArgs small_args(const PassArgs& p, const SolverScratch& s, const float4* X, int pass) {
+  SmallArgs a;
+  a.p = p;
+  a.g = group_args(s, X, p.V, p.n);
+  a.w = work_args(s, p.n);
+  a.bcnt = s.bcnt, a.bstart = s.bstart, a.bent = s.bent, a.bucket = s.bucket, a.bpart = s.bpart;
+  a.iteration = pass / 2;
+  a.groups = p.n >= kGroupCell && p.c.keps2 > 0.f;
+  a.buckets = p.c.order;
+  return a;
+}
+
+template <class Kernel>
+cudaError_t launch_cooperative(Kernel kernel, const SmallArgs& a, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((a.p.n + kWorkThreads - 1) / kWorkThreads);
+  cfg.blockDim = dim3(kWorkThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+// Before a lambda pass (kLast = kDeltaP) or the xsph pass (kDeltaPFinal): see
+// k_small_before.  The first lambda pass has no followers and its particles are
+// in their grid cells, so without groups there is nothing to launch but the
+// identity's flags, which a step clears to "no identity".
+template <int kLast>
+cudaError_t small_before(PassArgs& a, const SolverScratch& s, int pass, cudaStream_t stream) {
+  constexpr bool kXsphNext = kLast == kDeltaPFinal;
+  SmallArgs args = small_args(a, s, a.X, pass);
+  if constexpr (!kXsphNext) {
+    // the delta_p pass before wrote X (its T) and its component copy
+    args.p.T = const_cast<float4*>(a.X);
+    args.p.S_out = const_cast<float*>(a.S);
+  }
+  const bool first = args.iteration == 0;
+  if (!args.groups && (first || !args.buckets)) return cudaSuccess;  // every particle, in order (a.list is null)
+  small_list(a, s, kXsphNext);
+  return launch_cooperative(k_small_before<kLast>, args, stream);
+}
+
+cudaError_t small_between(PassArgs& a, const SolverScratch& s, int pass, cudaStream_t stream) {
+  const SmallArgs args = small_args(a, s, nullptr, pass);
+  const bool first = args.iteration == 0;
+  if (args.groups || !(first || !args.buckets)) small_list(a, s, false);  // as its lambda pass
+  if (args.buckets) a.moved_word = kMoved0 + (args.iteration & 1);
+  return args.groups ? launch_cooperative(k_small_between, args, stream) : cudaSuccess;
 }
 
 // kGroupsPos: the lambda pass's groups.  kGroupsLambda: their lambda sums for
@@ -2472,6 +2742,7 @@ PassArgs base_args(const StepConsts& c, const Geometry& G, const float4* X, cons
   a.grp_aux = s.grp_aux;
   a.count_word = kWorkCount;
   a.identity_word = kWorkIdentity;
+  a.moved_word = -1;
   return a;
 }
 
@@ -2508,8 +2779,8 @@ cudaError_t run_pass(const PassArgs& a, cudaStream_t stream) {
   const size_t dense_smem = sizeof(float4) * (size_t)max(a.c.stage_dense, 0);
   const long long slots = a.paired ? 2ll * a.n : a.n;  // of the pass's list, at most
   constexpr bool kPairs = kKind == kLambda || kKind == kXsph;
-  const int per_block = kPairs && a.paired ? 2 * kSparseThreads : kSparseThreads;
-  const int sparse_blocks = (int)((slots + per_block - 1) / per_block);
+  const int per_sparse = kPairs && a.paired ? 2 * kSparseThreads : kSparseThreads;
+  const int sparse_blocks = (int)((slots + per_sparse - 1) / per_sparse);
   if (a.dense_all) {
     // the sparse kernel has nothing to do
   } else if (kPairs && a.paired) {
@@ -2517,10 +2788,13 @@ cudaError_t run_pass(const PassArgs& a, cudaStream_t stream) {
   } else {
     k_sparse<kKind><<<sparse_blocks, kSparseThreads, 0, stream>>>(a);
   }
+  // no more blocks than batches where their number is known
+  const int per_block = dense_smem ? 1 : kDenseWarps / a.c.dense_split;
+  const int grid = a.dense_all ? min(a.c.dense_grid, ((a.n + 31) / 32 + per_block - 1) / per_block) : a.c.dense_grid;
   if (dense_smem)
-    k_dense<kKind, true><<<a.c.dense_grid, kDenseThreads, dense_queue + dense_smem, stream>>>(a);
+    k_dense<kKind, true><<<grid, kDenseThreads, dense_queue + dense_smem, stream>>>(a);
   else
-    k_dense<kKind, false><<<a.c.dense_grid, kDenseThreads, dense_queue, stream>>>(a);
+    k_dense<kKind, false><<<grid, kDenseThreads, dense_queue, stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -2547,11 +2821,12 @@ cudaError_t set_pass_kernel_attributes() {
   return e;
 }
 
+ClearList step_clears(const StepConsts& c, const SolverScratch& s) {
+  return ClearList{{s.cell_flags, s.flags, nullptr}, {c.cells + 1, kNumFlags, 0}};
+}
+
 cudaError_t reorder(const StepConsts& c, const uint32_t* perm, const float4* pos, const float4* vel,
                     const uint32_t* iid, int n, SolverScratch& s, cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(s.cell_flags, 0, sizeof(uint32_t) * (c.cells + 1), stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(s.flags, 0, sizeof(uint32_t) * kNumFlags, stream);
-  if (e != cudaSuccess) return e;
   k_reorder<<<(n + 255) / 256, 256, 0, stream>>>(perm, pos, vel, iid, n, c, s.xs, s.xa,
                                                   s.sa, s.stride, s.iid_s, s.flags, s.keys_sorted, s.cell_start, s.cell_flags,
                                                   s.grp_cell, s.grp_off, s.grp_item_off, s.grp_item_slot);
@@ -2560,25 +2835,17 @@ cudaError_t reorder(const StepConsts& c, const uint32_t* perm, const float4* pos
 
 namespace {
 
-// Whether the lambda / delta_p passes run on work lists (groups exist only
-// from kGroupCell particles on, and the zero gradient of co-located particles
-// needs kernel_eps > 0).
-bool use_work_list(const StepConsts& c, int n) { return n >= kGroupCell && c.keps2 > 0.f; }
-
 cudaError_t launch_work_list(const SolverScratch& s, int n, cudaStream_t stream) {
   const int blocks = (n + kWorkThreads - 1) / kWorkThreads;
-  k_work_mark<<<blocks, kWorkThreads, 0, stream>>>(s.keys_sorted, s.cell_flags, s.grp_n, s.grp_off, s.grp_id,
-                                                   s.grp_hash, s.grp_rep, s.grp_pool, n, s.work_follow,
-                                                   s.work_blocks, s.flags);
-  k_work_list<<<blocks, kWorkThreads, 0, stream>>>(s.work_follow, s.work_blocks, n, s.work_list, s.flags);
+  const WorkArgs w = work_args(s, n);
+  k_work_mark<<<blocks, kWorkThreads, 0, stream>>>(w);
+  k_work_list<<<blocks, kWorkThreads, 0, stream>>>(w);
   return cudaGetLastError();
 }
 
 template <int kKind>
 cudaError_t launch_follow(const PassArgs& a, const SolverScratch& s, cudaStream_t stream) {
-  k_follow<kKind><<<(a.n + 255) / 256, 256, 0, stream>>>(s.work_follow, a.n, a.c, s.lambda, s.xl, s.rho, a.T, a.S_out,
-                                                         a.stride, a.VR, s.xs, s.iid_s, a.npos, a.vel, a.pos, a.iid,
-                                                         s.keys_sorted, s.cell_flags, s.flags);
+  k_follow<kKind><<<(a.n + 255) / 256, 256, 0, stream>>>(a, s.work_follow);
   return cudaGetLastError();
 }
 
@@ -2587,8 +2854,22 @@ float* components_of(const SolverScratch& s, const float4* X) { return X == s.xa
 
 }  // namespace
 
+// A step whose work around the passes runs in cooperative launches
+// (k_small_before): every particle dense and one block per kWorkThreads
+// particles on an SM of its own.
+bool is_small(const StepConsts& c, int n) {
+  return dense_for_all(c, n) && n < kDenseAllBelow &&
+         (n + kWorkThreads - 1) / kWorkThreads <= c.dense_grid / kDenseBlocksPerSm;
+}
+
 cudaError_t launch_lambda(const StepConsts& c, const Geometry& G, const float4* X, const uint32_t* cs, int n,
                           const SolverScratch& s, int pass, cudaStream_t stream) {
+  if (is_small(c, n)) {
+    PassArgs a = base_args(c, G, X, cs, n, s, pass);
+    a.S = components_of(s, X);
+    const cudaError_t e = small_before<kDeltaP>(a, s, pass, stream);
+    return e == cudaSuccess ? run_pass<kLambda>(a, stream) : e;
+  }
   cudaError_t e = launch_groups<kGroupsPos>(c, s, X, nullptr, n, stream);
   if (e != cudaSuccess) return e;
   const bool wl = use_work_list(c, n);
@@ -2603,13 +2884,17 @@ cudaError_t launch_lambda(const StepConsts& c, const Geometry& G, const float4* 
 
 cudaError_t launch_delta_p(const StepConsts& c, const Geometry& G, const float4* X, const uint32_t* cs, int n,
                            const SolverScratch& s, int pass, float4* T, cudaStream_t stream) {
-  cudaError_t e = launch_groups<kGroupsLambda>(c, s, X, nullptr, n, stream);
-  if (e != cudaSuccess) return e;
-  const bool wl = use_work_list(c, n);
   PassArgs a = base_args(c, G, s.xl, cs, n, s, pass);  // X with its lambda
   a.S = components_of(s, X);
   a.S_out = components_of(s, T);
   a.T = T;
+  if (is_small(c, n)) {
+    const cudaError_t e = small_between(a, s, pass, stream);
+    return e == cudaSuccess ? run_pass<kDeltaP>(a, stream) : e;
+  }
+  cudaError_t e = launch_groups<kGroupsLambda>(c, s, X, nullptr, n, stream);
+  if (e != cudaSuccess) return e;
+  const bool wl = use_work_list(c, n);
   if (wl) a.list = s.work_list;
   if (c.order) use_buckets(a, s);
   if ((e = run_pass<kDeltaP>(a, stream)) != cudaSuccess) return e;
@@ -2619,9 +2904,6 @@ cudaError_t launch_delta_p(const StepConsts& c, const Geometry& G, const float4*
 cudaError_t launch_delta_p_final(const StepConsts& c, const Geometry& G, const float4* X, const uint32_t* cs, int n,
                                  const SolverScratch& s, int pass, float4* pos, float4* npos,
                                  float4* vel, uint32_t* iid, cudaStream_t stream) {
-  cudaError_t e = launch_groups<kGroupsLambda>(c, s, X, nullptr, n, stream);
-  if (e != cudaSuccess) return e;
-  const bool wl = use_work_list(c, n);
   PassArgs a = base_args(c, G, s.xl, cs, n, s, pass);
   a.S = components_of(s, X);
   a.VR = X == s.xa ? s.xb : s.xa;  // the positions go to npos: T's buffers are free
@@ -2632,6 +2914,13 @@ cudaError_t launch_delta_p_final(const StepConsts& c, const Geometry& G, const f
   a.vel = vel;
   a.pos = pos;
   a.iid = iid;
+  if (is_small(c, n)) {
+    const cudaError_t e = small_between(a, s, pass, stream);
+    return e == cudaSuccess ? run_pass<kDeltaPFinal>(a, stream) : e;
+  }
+  cudaError_t e = launch_groups<kGroupsLambda>(c, s, X, nullptr, n, stream);
+  if (e != cudaSuccess) return e;
+  const bool wl = use_work_list(c, n);
   if (wl) a.list = s.work_list;
   if (c.order) use_buckets(a, s);
   if ((e = run_pass<kDeltaPFinal>(a, stream)) != cudaSuccess) return e;
@@ -2731,9 +3020,8 @@ cudaError_t launch_vorticity(const StepConsts& c, const Geometry& G, const float
 }
 
 cudaError_t launch_xsph(const StepConsts& c, const Geometry& G, const float4* X, const float4* V, const uint32_t* cs,
-                        int n, const SolverScratch& s, int pass, float4* NV, cudaStream_t stream) {
-  cudaError_t e = launch_groups<kGroupsXsph>(c, s, X, V, n, stream);
-  if (e != cudaSuccess) return e;
+                        int n, const SolverScratch& s, int pass, float4* pos, float4* npos, float4* vel,
+                        uint32_t* iid, float4* NV, cudaStream_t stream) {
   PassArgs a = base_args(c, G, X, cs, n, s, pass);
   // where the last position update left them: after niter - 1 swaps of xa and
   // xb it read one and used the other
@@ -2741,6 +3029,15 @@ cudaError_t launch_xsph(const StepConsts& c, const Geometry& G, const float4* X,
   a.S = components_of(s, a.VR);
   a.V = V;
   a.NV = NV;
+  if (is_small(c, n)) {
+    // the last position update's followers, as launch_delta_p_final has it
+    a.xs = s.xs, a.iid_s = s.iid_s, a.npos = npos, a.vel = vel, a.pos = pos, a.iid = iid;
+    a.S_out = components_of(s, a.VR);
+    const cudaError_t e = small_before<kDeltaPFinal>(a, s, pass, stream);
+    return e == cudaSuccess ? run_pass<kXsph>(a, stream) : e;
+  }
+  cudaError_t e = launch_groups<kGroupsXsph>(c, s, X, V, n, stream);
+  if (e != cudaSuccess) return e;
   if (c.order && (e = bucket_by_cell(a, s, n, stream)) != cudaSuccess) return e;
   return run_pass<kXsph>(a, stream);
 }
@@ -2757,6 +3054,9 @@ int pass_launches(const StepConsts& c, int n) {
 // with work lists 2 more before each lambda pass and one follower launch after
 // each lambda and delta_p pass.
 int group_launches(const StepConsts& c, int n, int niter) {
+  // a small step: one launch before every pass (none before a lambda or xsph pass
+  // with neither groups nor buckets, none before a delta_p pass without groups)
+  if (is_small(c, n)) return n < kGroupCell ? (c.order ? niter : 0) : 2 * niter + 1;
   if (n < kGroupCell) return 0;
   return 3 * niter + 3 + (use_work_list(c, n) ? 4 * niter : 0);
 }
