@@ -121,25 +121,68 @@ k_scan_down(const uint32_t* in, int len, const uint32_t* __restrict__ partials, 
   }
 }
 
-// The whole scan in one block, for arrays of up to kScanOne entries: each
-// thread a contiguous share (read twice; the second time from L1).  The three
-// launches of the general scan cost 7 us at 4,001 entries, this one 2.5.
-constexpr int kScanOne = 32768;
+// The whole scan in one block, for arrays of up to kScanOne entries: each warp a
+// contiguous share, four entries a lane and round, every round's load in flight
+// before the first is used.  The three launches of the general scan cost 7 us at
+// 4,001 entries, this one 3.9; at 32,001 entries 8.5 and 6.2 (a thread's own
+// contiguous share instead, uncoalesced: 55).
+constexpr int kScanOneRounds = 8;
+constexpr int kScanOne = kTopThreads * 4 * kScanOneRounds;
 __global__ void __launch_bounds__(kTopThreads)
 k_scan_one(const uint32_t* in, int len, uint32_t* out, const uint32_t* __restrict__ groups) {
-  // in and out may alias: a thread touches its own share only
+  // in and out (16-byte aligned) may alias: a thread touches its own entries only
   __shared__ uint32_t smem[kTopThreads / 32 + 1];
   const bool apart = groups && *groups != 0u;
-  const int items = (len + kTopThreads - 1) / kTopThreads;
-  const int from = min(threadIdx.x * items, len), to = min(from + items, len);
-  uint32_t sum = 0;
-  for (int k = from; k < to; ++k) sum += groups ? pair_slots(in[k], apart) : in[k];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rounds = (len + 4 * kTopThreads - 1) / (4 * kTopThreads);
+  const int base = (warp * rounds * 32 + lane) * 4;
+  uint4 v[kScanOneRounds];
+#pragma unroll
+  for (int k = 0; k < kScanOneRounds; ++k) {
+    const int at = base + 128 * k;
+    if (k >= rounds || at >= len) {
+      v[k] = make_uint4(0u, 0u, 0u, 0u);
+    } else if (at + 3 < len) {
+      v[k] = *reinterpret_cast<const uint4*>(in + at);
+    } else {
+      v[k] = make_uint4(in[at], at + 1 < len ? in[at + 1] : 0u, at + 2 < len ? in[at + 2] : 0u, 0u);
+    }
+  }
+  uint32_t carry = 0u, before[kScanOneRounds];  // entries of the warp's share before this lane's, by round
+#pragma unroll
+  for (int k = 0; k < kScanOneRounds; ++k) {
+    if (groups)
+      v[k] = make_uint4(pair_slots(v[k].x, apart), pair_slots(v[k].y, apart), pair_slots(v[k].z, apart),
+                        pair_slots(v[k].w, apart));
+    const uint32_t own = v[k].x + v[k].y + v[k].z + v[k].w;
+    uint32_t x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    before[k] = carry + x - own;
+    carry += __shfl_sync(0xffffffffu, x, 31);
+  }
   uint32_t total;
-  uint32_t run = block_exclusive_scan<kTopThreads>(sum, smem, &total);
-  for (int k = from; k < to; ++k) {
-    const uint32_t v = groups ? pair_slots(in[k], apart) : in[k];
-    out[k] = run;
-    run += v;
+  const uint32_t start = block_exclusive_scan<kTopThreads>(lane == 0 ? carry : 0u, smem, &total);
+  const uint32_t first = __shfl_sync(0xffffffffu, start, 0);
+#pragma unroll
+  for (int k = 0; k < kScanOneRounds; ++k) {
+    const int at = base + 128 * k;
+    if (k >= rounds || at >= len) continue;
+    uint4 w;
+    w.x = first + before[k];
+    w.y = w.x + v[k].x;
+    w.z = w.y + v[k].y;
+    w.w = w.z + v[k].z;
+    if (at + 3 < len) {
+      *reinterpret_cast<uint4*>(out + at) = w;
+    } else {
+      out[at] = w.x;
+      if (at + 1 < len) out[at + 1] = w.y;
+      if (at + 2 < len) out[at + 2] = w.z;
+    }
   }
 }
 

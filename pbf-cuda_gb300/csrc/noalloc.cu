@@ -96,7 +96,7 @@ constexpr size_t kOffGrpId = kOffGrpAux + align_up(16 * kEntries);
 constexpr size_t kOffGrpHash = kOffGrpId + align_up(4 * kNp);
 constexpr size_t kOffGrpMax = kOffGrpHash + align_up(4 * 8 * kNp);
 constexpr size_t kOffGrpAcc = kOffGrpMax + align_up(4 * kNp);
-constexpr size_t kItems = kNp / pbf::kGroupChunk + kSlots + 1;
+constexpr size_t kItems = kNp / pbf::kGroupChunkMin + kSlots + 1;
 constexpr size_t kOffGrpList = kOffGrpAcc + align_up(8 * 3 * kNp);
 constexpr size_t kOffGrpListN = kOffGrpList + align_up(4 * kNp);
 constexpr size_t kOffGrpDone = kOffGrpListN + align_up(4 * kSlots);

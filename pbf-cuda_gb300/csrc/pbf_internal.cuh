@@ -310,15 +310,16 @@ constexpr int kCellSlotShift = 8;
 // reference's sum with its terms grouped: results differ from it by
 // rounding only.
 constexpr int kGroupCell = 512;
-// PBF_GROUP_CHUNK (a build-time tuning macro): particles of a grouped cell per
-// work item of the group-table kernels.
-#ifndef PBF_GROUP_CHUNK
-#define PBF_GROUP_CHUNK 8192
-#endif
-constexpr int kGroupChunk = PBF_GROUP_CHUNK;
+// Particles of a grouped cell per work item of the group-table kernels, between
+// these: about one item per SM when every particle is in a grouped cell (fewer,
+// larger items keep the last item's finishing step short of blocks; 126,976
+// particles, three quarters of them on six points: a step 747 us in items of
+// 8,192, 706 in items of 1,024).
+constexpr int kGroupChunkMin = 1024, kGroupChunkMax = 8192;
+inline int group_chunk(const StepConsts& c, int n);
 inline size_t group_slots(int max_particles) { return (size_t)max_particles / kGroupCell + 1; }
 inline size_t group_items(int max_particles) {
-  return (size_t)max_particles / kGroupChunk + group_slots(max_particles) + 1;
+  return (size_t)max_particles / kGroupChunkMin + group_slots(max_particles) + 1;
 }
 
 // Hits a particle keeps between the lambda and delta_p passes of one
@@ -419,6 +420,11 @@ constexpr int kDefaultDenseWindow = 512;
 #define PBF_DENSE_BLOCKS_PER_SM 4
 #endif
 constexpr int kDenseBlocksPerSm = PBF_DENSE_BLOCKS_PER_SM;
+inline int group_chunk(const StepConsts& c, int n) {
+  const int sms = c.dense_grid / kDenseBlocksPerSm;
+  const int share = (n / (sms > 0 ? sms : 1) + kGroupChunkMin - 1) / kGroupChunkMin * kGroupChunkMin;
+  return share < kGroupChunkMin ? kGroupChunkMin : (share > kGroupChunkMax ? kGroupChunkMax : share);
+}
 constexpr int kDenseAllBelow = 131072;
 // Slots a block of the dense pass kernel stages in shared memory (0: no
 // staging; pbf_autotune can override, up to kStageMax).  The tuning's

@@ -1811,7 +1811,7 @@ k_reorder(const uint32_t* __restrict__ perm, const float4* __restrict__ pos,
           float4* __restrict__ xs, float4* __restrict__ xa, float* __restrict__ sa, int stride,
           uint32_t* __restrict__ iid_s, uint32_t* __restrict__ flags, const uint32_t* __restrict__ skeys,
           const uint32_t* __restrict__ cs, uint32_t* __restrict__ cell_flags, int* __restrict__ grp_cell,
-          int* __restrict__ grp_off, int* __restrict__ grp_item_off, int* __restrict__ grp_item_slot) {
+          int* __restrict__ grp_off, int* __restrict__ grp_item_off, int* __restrict__ grp_item_slot, int chunk) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t key = skeys[k];
@@ -1822,8 +1822,8 @@ k_reorder(const uint32_t* __restrict__ perm, const float4* __restrict__ pos,
     const uint32_t slot = atomicAdd(&flags[kGroupCount], 1u);
     grp_cell[slot] = (int)key;
     grp_off[slot] = (int)atomicAdd(&flags[kGroupPool], pop);
-    // work items of kGroupChunk particles (< n / kGroupChunk + slots of them)
-    const int items = (int)((pop + kGroupChunk - 1) / kGroupChunk);
+    // work items of `chunk` particles (< n / chunk + slots of them)
+    const int items = (int)((pop + chunk - 1) / chunk);
     const int i0 = (int)atomicAdd(&flags[kGroupItems], (uint32_t)items);
     grp_item_off[slot] = i0;
     for (int t = 0; t < items; ++t) grp_item_slot[i0 + t] = (int)slot;
@@ -1858,6 +1858,7 @@ struct GroupArgs {
   const uint32_t* flags;  // flags[kGroupCount]: slots, flags[kGroupItems]: work items
   int n;
   int np;                 // pool entries
+  int chunk;              // particles of a work item
   const int* cell;
   const int* off;
   const int* item_off;    // first work item of each slot
@@ -1959,7 +1960,7 @@ __device__ __forceinline__ int block_scan_value(int v, int* sh, int& total) {
   return sh[32 + warp] + x - v;
 }
 
-// A grouped cell's particles in work items of kGroupChunk; a kernel takes
+// A grouped cell's particles in work items of a.chunk; a kernel takes
 // items grid-stride and the block that finishes a slot's last item (counted
 // in done[slot], made visible by a fence) runs the slot's finishing step and
 // sets the counter back to 0.
@@ -1973,8 +1974,8 @@ __device__ __forceinline__ Item item_of(const GroupArgs& a, int item) {
   const int cell = a.cell[it.slot];
   it.b = (int)a.cs[cell];
   it.m = max(min((int)a.cs[cell + 1], a.n) - it.b, 0);
-  it.k0 = (item - a.item_off[it.slot]) * kGroupChunk;
-  it.k1 = min(it.k0 + kGroupChunk, it.m);
+  it.k0 = (item - a.item_off[it.slot]) * a.chunk;
+  it.k1 = min(it.k0 + a.chunk, it.m);
   it.t0 = a.off[it.slot];
   return it;
 }
@@ -1984,7 +1985,7 @@ __device__ __forceinline__ bool last_item(const GroupArgs& a, const Item& it, in
   __threadfence();  // this block's writes, before the count that may let another block read them
   __syncthreads();
   if (threadIdx.x == 0) {
-    const int items = (it.m + kGroupChunk - 1) / kGroupChunk;
+    const int items = (it.m + a.chunk - 1) / a.chunk;
     *s_last = atomicAdd(&a.done[it.slot], 1) == items - 1;
   }
   __syncthreads();
@@ -2279,7 +2280,8 @@ struct WorkArgs {
   uint32_t* flags;
 };
 
-__device__ __forceinline__ void work_mark(const WorkArgs& w) {
+// Returns whether the thread's particle computes (with groups).
+__device__ __forceinline__ bool work_mark(const WorkArgs& w) {
   uint32_t* flags = w.flags;
   int* blocks = w.blocks;
   const int n = w.n, np = w.np;
@@ -2290,7 +2292,7 @@ __device__ __forceinline__ void work_mark(const WorkArgs& w) {
       flags[kWorkCount] = (uint32_t)n;
       flags[kWorkIdentity] = 1u;
     }
-    return;
+    return false;
   }
   const int i = blockIdx.x * kWorkThreads + threadIdx.x;
   int r = -1;
@@ -2314,7 +2316,7 @@ __device__ __forceinline__ void work_mark(const WorkArgs& w) {
   __syncthreads();
   if (threadIdx.x == 0) s_last = atomicAdd(&flags[kWorkDone], 1u) == gridDim.x - 1;
   __syncthreads();
-  if (!s_last) return;
+  if (!s_last) return i < n && r < 0;
   __threadfence();
   // the last block: exclusive offsets of every block, in chunks of kWorkThreads
   int carry = 0;
@@ -2330,6 +2332,7 @@ __device__ __forceinline__ void work_mark(const WorkArgs& w) {
     flags[kWorkCount] = (uint32_t)carry;
     flags[kWorkDone] = 0u;
   }
+  return i < n && r < 0;
 }
 
 // list[blocks[b] + rank] = i for the computing particles of block b, in order.
@@ -2429,8 +2432,9 @@ __global__ void __launch_bounds__(256) k_bucket_scatter(PassArgs a, const uint32
   if (a.paired && (apart || ((e.y & 1u) == 0u && e.y + 1u == bcnt[e.x]))) bucket[slot + 1u] = -1;
 }
 
-GroupArgs group_args(const SolverScratch& s, const float4* X, const float4* V, int n) {
+GroupArgs group_args(const StepConsts& c, const SolverScratch& s, const float4* X, const float4* V, int n) {
   GroupArgs a;
+  a.chunk = group_chunk(c, n);
   a.X = X;
   a.V = V;
   a.rho = s.rho;
@@ -2483,11 +2487,13 @@ WorkArgs work_args(const SolverScratch& s, int n) {
 //                    the buckets
 //   k_small_between  (delta_p)       the lambda pass's followers, the sums of
 //                    lambda
-// The buckets are built only where they matter: with groups, or when more than
-// one particle in kMovedShare has left its grid cell (the delta_p passes count
-// them); else the passes take the particles in grid order, which is then nearly
-// the current cells' (the order changes no result).
-// A step: 209 -> 99 us (1,728 particles), 214 -> 113 (8,000).
+// The buckets are built only where they matter: when more than one computing
+// particle in kMovedShare has left its grid cell (the delta_p passes count
+// them); else the passes take the particles (with groups, the work list) in grid
+// order, which is then nearly the current cells' (the order changes no result).
+// A step: 253 -> 99 us (1,728 particles), 268 -> 113 (8,000), 717 -> 706 (126,976,
+// three quarters of them on six points; 737 with a barrier after each of the
+// phases and every list bucketed).
 
 constexpr int kMovedShare = 8;
 constexpr int kBarrierSpins = 1 << 21;
@@ -2543,7 +2549,14 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
   constexpr bool kXsphNext = kLast == kDeltaPFinal;
   uint32_t* flags = a.p.flags;
   const int i = blockIdx.x * kWorkThreads + threadIdx.x;
+  const int n = a.p.n;
   const bool groups = a.groups && flags[kGroupCount] != 0u;
+  const uint32_t moved = a.buckets && a.iteration > 0 ? flags[kMoved0 + ((a.iteration + 1) & 1)] : 0u;
+  const bool buckets = a.buckets && moved > (uint32_t)n / kMovedShare;  // uniform over the grid
+  const int cells1 = a.p.c.cells + 1;
+  if (buckets)
+    for (int k = i; k < cells1; k += gridDim.x * kWorkThreads) a.bcnt[k] = 0u;
+  bool computes = i < n;
   if (groups) {
     if (a.iteration > 0) {
       follow_group<kLast>(a.p, a.w.follow, i);
@@ -2558,35 +2571,31 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
     } else {
       group_insert<kGroupsPos>(a.g);
       if (!grid_barrier(flags)) return;
-      work_mark(a.w);
-      if (!grid_barrier(flags)) return;
-      work_list(a.w);
-      if (!grid_barrier(flags)) return;
+      computes = work_mark(a.w);
+      if (!buckets) {
+        if (!grid_barrier(flags)) return;
+        work_list(a.w);
+      }
     }
-  } else if (!kXsphNext && i == 0) {
-    flags[kWorkCount] = (uint32_t)a.p.n;
-    flags[kWorkIdentity] = 1u;
+  } else {
+    if (!kXsphNext && i == 0) {
+      flags[kWorkCount] = (uint32_t)n;
+      flags[kWorkIdentity] = 1u;
+    }
+    if (buckets && !grid_barrier(flags)) return;
   }
   if (!a.buckets) return;
-  // the count this iteration's delta_p pass adds to (the last one's is read here)
-  if (i == 0) flags[kMoved0 + (a.iteration & 1)] = 0u;
-  const uint32_t moved = a.iteration > 0 ? flags[kMoved0 + ((a.iteration + 1) & 1)] : 0u;
-  if (!groups && moved <= (uint32_t)a.p.n / kMovedShare) {  // uniform over the grid
-    if (i == 0) {
-      flags[kBucketIdentity] = 1u;
-      flags[kBucketCount] = (uint32_t)a.p.n;
-    }
-    return;
-  }
-  // count, exclusive scan over the cells (every block a share), scatter
-  const int cells1 = a.p.c.cells + 1, threads = gridDim.x * kWorkThreads;
-  for (int k = i; k < cells1; k += threads) a.bcnt[k] = 0u;
-  if (!grid_barrier(flags)) return;
-  // the list: the work list of a step with groups (lambda), else every particle
   const bool listed = groups && !kXsphNext;
-  const int count = listed ? (int)flags[kWorkCount] : a.p.n;
-  const int j = i < count ? (listed && !flags[kWorkIdentity] ? a.w.list[i] : i) : 0;
-  if (i < count) bucket_count(a.p, i, j, a.bcnt, a.bent);
+  // the count this iteration's delta_p pass adds to (the last one's was read above)
+  if (i == 0) {
+    flags[kMoved0 + (a.iteration & 1)] = 0u;
+    flags[kBucketIdentity] = !buckets && !listed;
+    if (!listed) flags[kBucketCount] = (uint32_t)n;
+    else if (!buckets) flags[kBucketCount] = flags[kWorkCount];  // (complete since the barrier)
+  }
+  if (!buckets) return;
+  // count, exclusive scan over the cells (every block a share), scatter
+  if (computes) bucket_count(a.p, i, i, a.bcnt, a.bent);
   if (!grid_barrier(flags)) return;
   __shared__ int sh[80];
   const int per_block = (cells1 + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -2608,13 +2617,10 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
     run += (int)a.bcnt[k];
   }
   if (!grid_barrier(flags)) return;
-  if (i == 0) {
-    flags[kBucketIdentity] = 0u;
-    flags[kBucketCount] = (uint32_t)count;
-  }
-  if (i < count) {
+  if (listed && i == 0) flags[kBucketCount] = flags[kWorkCount];
+  if (computes) {
     const uint2 e = a.bent[i];
-    a.bucket[a.bstart[e.x] + e.y] = j;
+    a.bucket[a.bstart[e.x] + e.y] = i;
   }
 }
 
@@ -2642,8 +2648,9 @@ void small_list(PassArgs& a, const SolverScratch& s, bool xsph) {
 SmallArgs small_args(const PassArgs& p, const SolverScratch& s, const float4* X, int pass) {
   SmallArgs a;
   a.p = p;
-  a.g = group_args(s, X, p.V, p.n);
+  a.g = group_args(p.c, s, X, p.V, p.n);
   a.w = work_args(s, p.n);
+  if (p.c.order) a.w.list = s.bucket;  // where the passes look
   a.bcnt = s.bcnt, a.bstart = s.bstart, a.bent = s.bent, a.bucket = s.bucket, a.bpart = s.bpart;
   a.iteration = pass / 2;
   a.groups = p.n >= kGroupCell && p.c.keps2 > 0.f;
@@ -2698,7 +2705,7 @@ template <int kWhat>
 cudaError_t launch_groups(const StepConsts& c, const SolverScratch& s, const float4* X, const float4* V, int n,
                           cudaStream_t stream) {
   if (n < kGroupCell) return cudaSuccess;  // no cell can hold kGroupCell particles
-  const GroupArgs a = group_args(s, X, V, n);
+  const GroupArgs a = group_args(c, s, X, V, n);
   const int grid = c.dense_grid;
   if constexpr (kWhat != kGroupsLambda) k_group_insert<kWhat><<<grid, kGroupThreads, 0, stream>>>(a);
   if constexpr (kWhat != kGroupsPos) {
@@ -2829,7 +2836,8 @@ cudaError_t reorder(const StepConsts& c, const uint32_t* perm, const float4* pos
                     const uint32_t* iid, int n, SolverScratch& s, cudaStream_t stream) {
   k_reorder<<<(n + 255) / 256, 256, 0, stream>>>(perm, pos, vel, iid, n, c, s.xs, s.xa,
                                                   s.sa, s.stride, s.iid_s, s.flags, s.keys_sorted, s.cell_start, s.cell_flags,
-                                                  s.grp_cell, s.grp_off, s.grp_item_off, s.grp_item_slot);
+                                                  s.grp_cell, s.grp_off, s.grp_item_off, s.grp_item_slot,
+                                                  group_chunk(c, n));
   return cudaGetLastError();
 }
 
