@@ -18,7 +18,9 @@
 //   F(r) = phi(s) r,  phi = b (h - s)^2 / s,  s = |r|        (spiky gradient)
 //   J(r) = dF/dr = phi I + (phi'(s) / s) r r^T,  phi' = -b (h - s)(h + s) / s^2
 // Per iteration k (last to first), with X = X_k, lambda = lambda_k and the
-// adjoint of X_{k+1}:
+// adjoint of X_{k+1} (k_bwd_window: delta_p 1, G_i and D_i of lambda 1, and the
+// neighbour lists; k_bwd_delta_p: delta_p 2; k_bwd_fix_lambda: the rest of
+// lambda 1; k_bwd_lambda: lambda 2):
 //   delta_p 1: u = X + clamp(P / pho0), X_{k+1} = box(u): the clamps pass the
 //              adjoint through where inactive, the wall takes it where active;
 //              Pbar = ubar masked by the MAX_DP clamp / pho0
@@ -44,7 +46,15 @@ namespace pbf {
 namespace {
 
 constexpr int kThreads = 128;
-// Below this many particles a warp shares each particle (see lane_sum).
+// Blocks, per block of the dense passes' grid, that take the particles without a
+// list of a one-lane step: 8 per SM, what their registers allow (4 per SM: a
+// crowded scene of 262,144 particles 30.5 ms, 8: 26.0, 20: 25.5, but 2% of a
+// step without such particles).
+constexpr int kLongBlocks = 2;
+// Below this many particles a warp shares each particle (see lane_sum).  From
+// 41,000 particles on one lane each is as fast or faster at rest (125,000: a
+// gradient 1,333 us against 1,860), but loses where particles pile up (110,592,
+// an eighth of them on 40 points: a reverse pass 4.5 ms against 2.0).
 constexpr int kWarpPerParticleBelow = 131072;
 // Lanes that split one particle's window in the reverse kernels of steps
 // under kWarpPerParticleBelow particles: BackwardArgs::lanes (8, 16 or 32;
@@ -97,11 +107,13 @@ __device__ __forceinline__ unsigned long long pack_cell(int3 q) {
 }
 
 // True when the cells differ by at most one along every axis, i.e. when a
-// window centred on one contains the other.
+// window centred on one contains the other.  All axes at once: 1 + a - b is 0, 1
+// or 2 in every field, and the lowest field that is not shows it (no borrow
+// reached it from below).
 __device__ __forceinline__ bool near_cell(unsigned long long a, unsigned long long b) {
-  const int ax = (int)(a >> 42), ay = (int)((a >> 21) & 0x1FFFFF), az = (int)(a & 0x1FFFFF);
-  const int bx = (int)(b >> 42), by = (int)((b >> 21) & 0x1FFFFF), bz = (int)(b & 0x1FFFFF);
-  return abs(ax - bx) <= 1 && abs(ay - by) <= 1 && abs(az - bz) <= 1;
+  constexpr unsigned long long kOnes = (1ull << 42) | (1ull << 21) | 1ull;
+  const unsigned long long d = a + kOnes - b;
+  return ((d & ~(3ull * kOnes)) | (d & (d >> 1) & kOnes)) == 0ull;
 }
 
 __device__ __forceinline__ void atomic_add3(float4* p, float x, float y, float z) {
@@ -146,7 +158,7 @@ __device__ __forceinline__ void note_term(const BackwardArgs& a, int comp, int j
 // lambda / rho adjoint w) or kind 1 (fixv: velocity adjoints xyz).
 __device__ __forceinline__ void scatter_term(const BackwardArgs& a, int kind, int j, float x, float y, float z,
                                              float w) {
-  const unsigned slot = atomicAdd(&a.sc_ctr[0], 1u);
+  const unsigned slot = atomicAdd(&a.sc_ctr[a.sc_list], 1u);
   if (slot >= (unsigned)a.sc_cap) {
     atomicAdd(&a.sc_ctr[1], 1u);
     float4* f = kind == 0 ? a.fix : a.fixv;
@@ -164,10 +176,44 @@ __device__ __forceinline__ void scatter_term(const BackwardArgs& a, int kind, in
   if (kind == 0) note_term(a, 3, j, w);
 }
 
-// Adds every listed term into its target's fixed-point sums (grid-stride).
-__global__ void __launch_bounds__(256) k_bwd_acc(BackwardArgs a) {
-  const unsigned listed = min(a.sc_ctr[0], (unsigned)a.sc_cap);
-  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < listed; e += gridDim.x * blockDim.x) {
+// Sums the wall adjoints of `blocks` blocks into g_lim[6] (accumulating) in a
+// fixed order: thread t adds the parts of blocks t, t + kWallThreads, ... in
+// turn, then the threads' sums are added pairwise in a fixed tree.
+constexpr int kWallThreads = 256;
+__device__ __forceinline__ void sum_walls(const float* __restrict__ part, int blocks, float* __restrict__ g_lim) {
+  __shared__ float s[6][kWallThreads];
+  float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int b = threadIdx.x; b < blocks; b += kWallThreads)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc[k] += part[b * 6 + k];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) s[k][threadIdx.x] = acc[k];
+  __syncthreads();
+  for (int w = kWallThreads / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w)
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s[k][threadIdx.x] += s[k][threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x < 6) g_lim[threadIdx.x] += s[threadIdx.x][0];
+}
+
+// Adds every listed term into its target's fixed-point sums (grid-stride), and
+// empties the other list (the last one folded: two lists take turns, so no
+// kernel reads a length that another block resets).  wall_blocks > 0: the last
+// block sums that many blocks' wall adjoints instead.
+__global__ void __launch_bounds__(kWallThreads) k_bwd_acc(BackwardArgs a, int wall_blocks, float* __restrict__ g_lim) {
+  unsigned workers = gridDim.x;
+  if (wall_blocks > 0) {
+    if (blockIdx.x == --workers) {
+      sum_walls(a.wall_part, wall_blocks, g_lim);
+      return;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.sc_ctr[a.sc_list ^ 2] = 0u;
+  const unsigned listed = min(a.sc_ctr[a.sc_list], (unsigned)a.sc_cap);
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < listed; e += workers * blockDim.x) {
     const int2 key = a.sc_key[e];
     const float4 v = a.sc_val[e];
     const int j = key.x, kind = key.y, base = kind == 0 ? 0 : 4, comps = kind == 0 ? 4 : 3;
@@ -197,29 +243,36 @@ __device__ __forceinline__ float take_sum(const BackwardArgs& a, int comp, int j
     return (bits & 2u) ? __int_as_float(0x7f800000) : __int_as_float((int)0xff800000);
   }
   if (cnt == 0u || acc == 0ull) return 0.f;
-  return (float)ldexp((double)(long long)acc, -scale_shift(mx, cnt));
+  return ldexpf(__ll2float_rn((long long)acc), -scale_shift(mx, cnt));  // (one rounding; no FP64 units)
 }
 
 // Target i's scattered sums of `kind` (xyz, and w for fix), its scratch
-// cleared, plus what overflowed into fix / fixv (also cleared).
-__device__ __forceinline__ float4 take_scattered(const BackwardArgs& a, int kind, int i) {
+// cleared, plus what overflowed into fix / fixv (also cleared).  `listed`: the
+// terms listed for all targets (0: nothing to read); false when none are i's.
+__device__ __forceinline__ bool take_scattered(const BackwardArgs& a, int kind, int i, unsigned listed, float4& s) {
+  s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (listed == 0u) return false;
   const unsigned cnt = a.sc_cnt[kind * a.sc_stride + i];
-  a.sc_cnt[kind * a.sc_stride + i] = 0u;
-  const unsigned nonfin = a.sc_nonfin[i];
-  float4* f = kind == 0 ? a.fix : a.fixv;
-  const float4 o = f[i];
-  f[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int base = kind == 0 ? 0 : 4;
-  float4 s;
-  s.x = take_sum(a, base, i, cnt, nonfin) + o.x;
-  s.y = take_sum(a, base + 1, i, cnt, nonfin) + o.y;
-  s.z = take_sum(a, base + 2, i, cnt, nonfin) + o.z;
-  s.w = kind == 0 ? take_sum(a, 3, i, cnt, nonfin) + o.w : 0.f;
-  return s;
+  if (cnt != 0u) {
+    a.sc_cnt[kind * a.sc_stride + i] = 0u;
+    const unsigned nonfin = a.sc_nonfin[i];
+    const int base = kind == 0 ? 0 : 4;
+    s.x = take_sum(a, base, i, cnt, nonfin);
+    s.y = take_sum(a, base + 1, i, cnt, nonfin);
+    s.z = take_sum(a, base + 2, i, cnt, nonfin);
+    if (kind == 0) s.w = take_sum(a, 3, i, cnt, nonfin);
+  }
+  if (listed > (unsigned)a.sc_cap) {
+    float4* f = kind == 0 ? a.fix : a.fixv;
+    const float4 o = f[i];
+    f[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    s = make_float4(s.x + o.x, s.y + o.y, s.z + o.z, kind == 0 ? s.w + o.w : 0.f);
+    return true;
+  }
+  return cnt != 0u;
 }
 
-// After a fold: the list is empty again, and each target's non-finite bits
-// of the folded kind are clear.
+// After a fold: the target's non-finite bits of the folded kind are clear.
 __device__ __forceinline__ void clear_nonfin(const BackwardArgs& a, int i, unsigned mask) {
   const unsigned nf = a.sc_nonfin[i];
   if (nf & mask) a.sc_nonfin[i] = nf & ~mask;
@@ -246,104 +299,311 @@ __device__ __forceinline__ Vec lane_sum(Vec v) {
   return {lane_sum<L>(v.x), lane_sum<L>(v.y), lane_sum<L>(v.z)};
 }
 
-// phi(s) and phi'(s) / s of the spiky gradient F = phi r (|r| = s).
-__device__ __forceinline__ void spiky_parts(const StepConsts& c, float s, float& phi, float& k) {
+// phi(s) and phi'(s) / s of the spiky gradient F = phi r (|r| = s, q = s^2).
+__device__ __forceinline__ void spiky_parts(const StepConsts& c, float q, float& phi, float& k) {
+  const float is = __frsqrt_rn(q), s = q * is;
   const float d = c.h - s;
-  phi = c.spiky_coef * d * d / s;
-  k = -c.spiky_coef * d * (c.h + s) / (s * s * s);
+  phi = c.spiky_coef * d * d * is;
+  k = -c.spiky_coef * d * (c.h + s) * is * is * is;
 }
 
-// J v = phi v + k r (r . v)
-__device__ __forceinline__ Vec jac(float phi, float k, Vec r, Vec v) {
-  const float rv = vdot(r, v);
-  return {phi * v.x + k * r.x * rv, phi * v.y + k * r.y * rv, phi * v.z + k * r.z * rv};
+// ---- neighbour lists -------------------------------------------------------------------
+//
+// The window of a particle holds 216 candidates on average at rest and 33
+// neighbours.  One kernel per iteration tests the candidates and lists the
+// neighbours (the test the same as the lambda sums'), and all four sums of the
+// iteration run over the list: lanes then stay together, and a sum gathers only
+// what it needs.  A particle with more than kHitCap neighbours has no list
+// (length -1): its sums walk the window, as every sum of every particle did
+// before (with one lane per particle, a warp each: a crowded scene of 262,144
+// particles 31.9 -> 26.0 ms).  Reverse pass of 262,144 particles at rest, 4
+// iterations: 2,906 -> 1,060 us; of 15,625 (32 lanes per particle): 559 -> 231.
+// Bounds: k_bwd_window (109 us of 262,144 particles) issues instructions (64% of
+// the slots: 85 million, three quarters of them tests and list entries), the
+// sums over the lists wait for their gathers (47% of the slots).
+
+// Entry k of particle i: one thread per particle interleaves the particles'
+// lists (a warp reads entry k of its particles in one line), lanes of one
+// particle read its list along.
+template <int L>
+__device__ __forceinline__ uint32_t* hit_list(const BackwardArgs& a, int i) {
+  return a.hits + (L == 1 ? (size_t)i : (size_t)i * kHitCap);
+}
+template <int L>
+__device__ __forceinline__ size_t hit_step(const BackwardArgs& a) {
+  return L == 1 ? (size_t)a.hit_stride : 1;
 }
 
-// Packed cells of positions X (the grid's, or the current ones).
+constexpr uint32_t kOneSided = 0x80000000u;  // list entry: j cannot gather i's terms
+
+// The lanes of particle i's group (all of a group's lanes run together).
+template <int L>
+__device__ __forceinline__ unsigned group_mask() {
+  const unsigned lane = threadIdx.x & 31u;
+  return L == 32 ? 0xffffffffu : ((1u << L) - 1u) << (lane & ~(unsigned)(L - 1));
+}
+
+// Lists the candidates of particle i's window that lie within h of xi (or whose
+// distance is NaN), itself among them, and returns their number, or -1 when they
+// do not fit.
+template <int L>
+__device__ __forceinline__ int list_hits(const BackwardArgs& a, const float4* __restrict__ X, float4 xi, int i,
+                                         int lane) {
+  const StepConsts& c = a.c;
+  const SceneGeom g = geom_of(c, a.G, i);
+  const int3 q = cell_of(c, g, xi);
+  uint32_t* list = hit_list<L>(a, i);
+  int cnt = 0;
+  const auto is_hit = [&](float4 xj) {
+    const float r2 = dist2(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
+    return !(r2 >= c.h2);
+  };
+  if constexpr (L == 1) {
+    // four candidates' loads in flight at a time, and room for four more entries
+    // looked at once for them (so that a list holds kHitCap - 3 at least)
+    const size_t step = hit_step<L>(a);
+    for (int dx = -1; dx <= 1; ++dx) {
+      const int x = q.x + dx;
+      if (x < 0 || x >= g.dims[0]) continue;
+      for (int dy = -1; dy <= 1; ++dy) {
+        const int y = q.y + dy;
+        if (y < 0 || y >= g.dims[1]) continue;
+        int s, e;
+        column_run(g, a.cs, a.n, x, y, q.z, s, e);
+        for (int j = s; j < e; j += 4) {
+          float4 xj[4];
+          if (j + 4 <= a.n) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xj[u] = ld4(X + j, u);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xj[u] = ld4(X, min(j + u, a.n - 1));
+          }
+          if (cnt > kHitCap - 4) return -1;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (j + u < e && is_hit(xj[u])) {
+              *list = (uint32_t)(j + u);
+              list += step;
+              ++cnt;
+            }
+          }
+        }
+      }
+    }
+  } else {
+    // the lanes look up the nine columns side by side, and every column's first
+    // L candidates are in flight before the first test
+    constexpr int kPer = (9 + L - 1) / L;
+    const unsigned mask = group_mask<L>(), below = mask & ((1u << (threadIdx.x & 31u)) - 1u);
+    int s[kPer], e[kPer];
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int col = lane + p * L, x = q.x + col / 3 - 1, y = q.y + col % 3 - 1;
+      s[p] = e[p] = 0;
+      if (col < 9 && x >= 0 && x < g.dims[0] && y >= 0 && y < g.dims[1])
+        column_run(g, a.cs, a.n, x, y, q.z, s[p], e[p]);
+    }
+    const auto append = [&](int j, bool hit) {
+      const unsigned b = __ballot_sync(mask, hit);
+      const int at = cnt + __popc(b & below);
+      if (hit && at < kHitCap) list[at] = (uint32_t)j;
+      cnt += __popc(b & mask);
+    };
+    float4 first[9];
+#pragma unroll
+    for (int col = 0; col < 9; ++col) {
+      const int j = __shfl_sync(mask, s[col / L], col % L, L) + lane;
+      if (j < __shfl_sync(mask, e[col / L], col % L, L)) first[col] = ld4(X, j);
+      else first[col] = xi;
+    }
+#pragma unroll
+    for (int col = 0; col < 9; ++col) {
+      const int from = __shfl_sync(mask, s[col / L], col % L, L), to = __shfl_sync(mask, e[col / L], col % L, L);
+      if (from >= to) continue;
+      append(from + lane, from + lane < to && is_hit(first[col]));
+      for (int j = from + lane + L; j - lane < to; j += L) append(j, j < to && is_hit(ld4(X, min(j, to - 1))));
+    }
+    __syncwarp(mask);  // the lanes read each other's entries
+  }
+  return cnt <= kHitCap ? cnt : -1;
+}
+
+template <int N>
+struct Sums {
+  float v[N];
+};
+
+// visit(own(i), sums, j, one-sided, load(j), null) for lane `lane` of `stride`'s
+// share of the candidates of particle i's window that list_hits would list.
+template <int N, class Own, class Load, class Visit>
+__device__ __forceinline__ void walk_window(const BackwardArgs& a, const float4* __restrict__ X, int i, int lane,
+                                            int stride, Sums<N>& sums, Own&& own, Load&& load, Visit&& visit) {
+  const auto self = own(i);
+  const float4 x = ld4(X, i);
+  const SceneGeom g = geom_of(a.c, a.G, i);
+  const unsigned long long cell = a.gcell[i];
+  for_window(g, a.cs, a.n, cell_of(a.c, g, x), [&](int j) {
+    const float4 xj = ld4(X, j);
+    if (dist2(x.x - xj.x, x.y - xj.y, x.z - xj.z) >= a.c.h2) return;
+    visit(self, sums, j, !near_cell(cell, a.kcell[j]), load(j), (uint32_t*)nullptr);
+  }, lane, stride);
+}
+
+// finish(i, sums) in one lane for every particle i, sums over its neighbours
+// what visit(own(i), sums, j, one-sided, load(j), list entry) adds: those of its
+// list (the next one's loads in flight).  cnt: the list's length, or negative
+// without one; with several lanes per particle they then walk the window, with
+// one a warp of finish_long's does.
+template <int L, int N, class Own, class Load, class Visit, class Finish>
+__device__ __forceinline__ void finish_listed(const BackwardArgs& a, const float4* __restrict__ X, int i, int lane,
+                                              int cnt, Own&& own, Load&& load, Visit&& visit, Finish&& finish) {
+  if (L == 1 && cnt < 0) return;
+  Sums<N> acc = {};
+  if (lane < cnt) {
+    const auto self = own(i);
+    uint32_t* list = hit_list<L>(a, i);
+    const size_t step = hit_step<L>(a);
+    uint32_t e = list[lane * step];
+    auto d = load((int)(e & ~kOneSided));
+    for (int k = lane; k < cnt; k += L) {
+      uint32_t en = e;
+      auto dn = d;
+      if (k + L < cnt) {
+        en = list[(size_t)(k + L) * step];
+        dn = load((int)(en & ~kOneSided));
+      }
+      visit(self, acc, (int)(e & ~kOneSided), (e & kOneSided) != 0u, d, list + (size_t)k * step);
+      e = en;
+      d = dn;
+    }
+  }
+  if constexpr (L > 1) {
+    if (cnt < 0) walk_window(a, X, i, lane, L, acc, own, load, visit);
+#pragma unroll
+    for (int k = 0; k < N; ++k) acc.v[k] = lane_sum<L>(acc.v[k]);
+  }
+  if (lane == 0) finish(i, acc);
+}
+
+// The same for the particles without a list of a one-lane step, a warp each.
+// They come in runs (a crowded cell's particles), so warp w of W takes particles
+// w, w + W, ...
+template <int N, class Own, class Load, class Visit, class Finish>
+__device__ __forceinline__ void finish_long(const BackwardArgs& a, const float4* __restrict__ X, int blocks,
+                                            Own&& own, Load&& load, Visit&& visit, Finish&& finish) {
+  const int lane = threadIdx.x & 31;
+  const int W = blocks * (kThreads / 32), w = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  for (long long base = w; base < a.n; base += 32ll * W) {
+    const long long i = base + (long long)lane * W;
+    for (unsigned m = __ballot_sync(0xffffffffu, i < a.n && a.hit_n[i] < 0); m != 0u; m &= m - 1u) {
+      const int of = (int)(base + (long long)(__ffs(m) - 1) * W);
+      Sums<N> acc = {};
+      walk_window(a, X, of, lane, 32, acc, own, load, visit);
+#pragma unroll
+      for (int k = 0; k < N; ++k) acc.v[k] = lane_sum<32>(acc.v[k]);
+      if (lane == 0) finish(of, acc);
+    }
+  }
+}
+
+struct Two {
+  float4 x, b;
+};
+
+// The packed cells of the grid's positions and of the final ones, the velocities
+// v = (X_K - X0) / dt with rho, and empty lists of scattered terms.
 __global__ void __launch_bounds__(256)
-k_bwd_cells(BackwardArgs a, const float4* __restrict__ X, unsigned long long* __restrict__ out) {
+k_bwd_start(BackwardArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 2) a.sc_ctr[2 * i] = 0u;
   if (i >= a.n) return;
-  out[i] = pack_cell(cell_of(a.c, geom_of(a.c, a.G, i), ld4(X, i)));
+  const SceneGeom g = geom_of(a.c, a.G, i);
+  const float4 x = ld4(a.XK, i), x0 = ld4(a.xs, i);
+  a.gcell[i] = pack_cell(cell_of(a.c, g, ld4(a.X0, i)));
+  a.kcell[i] = pack_cell(cell_of(a.c, g, x));
+  a.pbar[i] = make_float4((x.x - x0.x) * a.c.inv_dt, (x.y - x0.y) * a.c.inv_dt, (x.z - x0.z) * a.c.inv_dt, a.rho[i]);
 }
 
 // ---- XSPH and the velocity update --------------------------------------------------
 
-template <int L>
+// kLong: the particles without a list of a one-lane step (after the others).
+template <int L, bool kLong>
 __global__ void __launch_bounds__(kThreads)
 k_bwd_xsph(BackwardArgs a) {
   const StepConsts& c = a.c;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = t / L, lane = t % L;
-  if (i >= a.n) return;
-  const float4 xi = ld4(a.XK, i), x0i = ld4(a.xs, i), gi = ld4(a.g_nvel, i);
-  const float4 vi = make_float4((xi.x - x0i.x) * c.inv_dt, (xi.y - x0i.y) * c.inv_dt,
-                                (xi.z - x0i.z) * c.inv_dt, 0.f);
-  const float ri = a.rho[i];
-  const unsigned long long gci = a.gcell[i];
-  const SceneGeom g = geom_of(c, a.G, i);
-  Vec vb = {0.f, 0.f, 0.f}, xb = {0.f, 0.f, 0.f};
-  float rb = 0.f;
-  for_window(g, a.cs, a.n, cell_of(c, g, xi), [&](int j) {
-    if (j == i) return;
-    const float4 xj = ld4(a.XK, j);
-    const Vec r = vsub(xi, xj);
+  struct Own {
+    float4 x, v, g;
+    unsigned long long cell;
+    int i;
+  };
+  const auto own = [&](int k) { return Own{ld4(a.XK, k), ld4(a.pbar, k), ld4(a.g_nvel, k), a.gcell[k], k}; };
+  const auto load = [&](int j) { return Two{ld4(a.XK, j), ld4(a.pbar, j)}; };
+  const auto visit = [&](const Own& o, Sums<7>& s, int j, bool, const Two& t, uint32_t*) {
+    const Vec r = vsub(o.x, t.x);
     const float q = vdot(r, r);
-    if (!(q < c.h2)) return;
-    const float4 x0j = ld4(a.xs, j);
-    const Vec dv = {(xj.x - x0j.x) * c.inv_dt - vi.x, (xj.y - x0j.y) * c.inv_dt - vi.y,
-                    (xj.z - x0j.z) * c.inv_dt - vi.z};
-    const float den = ri + a.rho[j];
-    const float W = poly6_inside(c, q);
-    const float w = 2.f * W / den;
-    const float dq = 2.f * dpoly6(c, q) / den * 2.f;  // d w / d x_i per unit of r
-    const float dr = -2.f * W / (den * den);           // d w / d rho
-    // nv_i's term c w (v_j - v_i): its adjoint on i's inputs
-    const float own = c.c_xsph * (gi.x * dv.x + gi.y * dv.y + gi.z * dv.z);
-    vb.x -= c.c_xsph * w * gi.x;
-    vb.y -= c.c_xsph * w * gi.y;
-    vb.z -= c.c_xsph * w * gi.z;
-    xb.x += own * dq * r.x;
-    xb.y += own * dq * r.y;
-    xb.z += own * dq * r.z;
-    rb += own * dr;
-    if (near_cell(gci, a.kcell[j])) {
-      // i is in j's window: nv_j's term c w (v_i - v_j) on i's inputs
-      const float4 gj = ld4(a.g_nvel, j);
-      const float tr = -c.c_xsph * (gj.x * dv.x + gj.y * dv.y + gj.z * dv.z);
-      vb.x += c.c_xsph * w * gj.x;
-      vb.y += c.c_xsph * w * gj.y;
-      vb.z += c.c_xsph * w * gj.z;
-      xb.x += tr * dq * r.x;
-      xb.y += tr * dq * r.y;
-      xb.z += tr * dq * r.z;
-      rb += tr * dr;
-    } else {
+    if (!(q < c.h2) || j == o.i) return;
+    const Vec dv = vsub(t.b, o.v);
+    const float inv = 1.f / (o.v.w + t.b.w);  // 1 / (rho_i + rho_j)
+    const float w = 2.f * poly6_inside(c, q) * inv;
+    const float dq = 4.f * dpoly6(c, q) * inv;  // d w / d x_i per unit of r
+    const float dr = -w * inv;                  // d w / d rho
+    // nv_i's term c w (v_j - v_i) and, when i is in j's window, nv_j's
+    // c w (v_i - v_j): their adjoints on i's inputs, from nvbar_i - nvbar_j
+    const bool both = near_cell(o.cell, a.kcell[j]);
+    Vec gd = {o.g.x, o.g.y, o.g.z};
+    if (both) gd = vsub(o.g, ld4(a.g_nvel, j));
+    const float gv = c.c_xsph * vdot(gd, dv);
+    const float cw = c.c_xsph * w;
+    s.v[0] -= cw * gd.x;
+    s.v[1] -= cw * gd.y;
+    s.v[2] -= cw * gd.z;
+    s.v[3] += gv * dq * r.x;
+    s.v[4] += gv * dq * r.y;
+    s.v[5] += gv * dq * r.z;
+    s.v[6] += gv * dr;
+    if (!both) {
       // j cannot gather nv_i's term: scatter its adjoint on j's inputs
-      scatter_term(a, 1, j, c.c_xsph * w * gi.x, c.c_xsph * w * gi.y, c.c_xsph * w * gi.z, 0.f);
-      scatter_term(a, 0, j, -own * dq * r.x, -own * dq * r.y, -own * dq * r.z, own * dr);
+      scatter_term(a, 1, j, cw * gd.x, cw * gd.y, cw * gd.z, 0.f);
+      scatter_term(a, 0, j, -gv * dq * r.x, -gv * dq * r.y, -gv * dq * r.z, gv * dr);
     }
-  }, lane, L);
-  vb = lane_sum<L>(vb);
-  xb = lane_sum<L>(xb);
-  rb = lane_sum<L>(rb);
-  if (lane != 0) return;
-  vb = {gi.x + vb.x, gi.y + vb.y, gi.z + vb.z};  // nv_i = v_i + ...: the identity part
-  // v = (X_K - X0) / dt: the position adjoint of the step's output plus XSPH's
-  const float4 gp = ld4(a.g_npos, i);
-  a.gx[i] = make_float4(gp.x + xb.x + vb.x * c.inv_dt, gp.y + xb.y + vb.y * c.inv_dt,
-                        gp.z + xb.z + vb.z * c.inv_dt, 0.f);
-  a.gx0[i] = make_float4(-vb.x * c.inv_dt, -vb.y * c.inv_dt, -vb.z * c.inv_dt, 0.f);
-  a.grho[i] = rb;
+  };
+  const auto finish = [&](int i, const Sums<7>& s) {
+    const float4 gi = ld4(a.g_nvel, i), gp = ld4(a.g_npos, i);
+    const Vec vb = {gi.x + s.v[0], gi.y + s.v[1], gi.z + s.v[2]};  // nv_i = v_i + ...: the identity part
+    // v = (X_K - X0) / dt: the position adjoint of the step's output plus XSPH's
+    a.gx[i] = make_float4(gp.x + s.v[3] + vb.x * c.inv_dt, gp.y + s.v[4] + vb.y * c.inv_dt,
+                          gp.z + s.v[5] + vb.z * c.inv_dt, 0.f);
+    a.gx0[i] = make_float4(-vb.x * c.inv_dt, -vb.y * c.inv_dt, -vb.z * c.inv_dt, 0.f);
+    a.grho[i] = s.v[6];
+  };
+  if constexpr (kLong) {
+    finish_long<7>(a, a.XK, gridDim.x, own, load, visit, finish);
+  } else {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t / L, lane = t % L;
+    if (i >= a.n) return;
+    const int cnt = list_hits<L>(a, a.XK, ld4(a.XK, i), i, lane);
+    if (lane == 0) a.hit_n[i] = cnt;
+    finish_listed<L, 7>(a, a.XK, i, lane, cnt, own, load, visit, finish);
+  }
+}
+
+// The packed cells of the positions the next iteration's kernels work on (null: none follow).
+__device__ __forceinline__ void next_cells(const BackwardArgs& a, const float4* __restrict__ X, int i) {
+  if (X) a.kcell[i] = pack_cell(cell_of(a.c, geom_of(a.c, a.G, i), ld4(X, i)));
 }
 
 // Folds the scattered XSPH adjoints in and clears their scratch.
 __global__ void __launch_bounds__(256)
-k_bwd_fix_xsph(BackwardArgs a) {
+k_bwd_fix_xsph(BackwardArgs a, const float4* __restrict__ next) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) a.sc_ctr[0] = 0u;  // every listed term has been added (k_bwd_acc)
   if (i >= a.n) return;
-  const float4 f = take_scattered(a, 0, i), v = take_scattered(a, 1, i);
+  next_cells(a, next, i);
+  const unsigned listed = a.sc_ctr[a.sc_list];
+  float4 f, v;
+  const bool any = take_scattered(a, 0, i, listed, f), anyv = take_scattered(a, 1, i, listed, v);
+  if (!any && !anyv) return;
   clear_nonfin(a, i, 0x1fffffu);
   const float4 g = a.gx[i], g0 = a.gx0[i];
   const float t = a.c.inv_dt;
@@ -352,251 +612,245 @@ k_bwd_fix_xsph(BackwardArgs a) {
   a.grho[i] += f.w;
 }
 
-// Folds scattered position adjoints into gx_next (and, with kLambda, the w
-// part into lambdabar) and clears their scratch.
-template <bool kLambda>
+// Folds the lambda sums' scattered position adjoints into gx_next and clears
+// their scratch.
 __global__ void __launch_bounds__(256)
-k_bwd_fix(BackwardArgs a) {
+k_bwd_fix(BackwardArgs a, const float4* __restrict__ next) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) a.sc_ctr[0] = 0u;
   if (i >= a.n) return;
-  const float4 f = take_scattered(a, 0, i);
+  next_cells(a, next, i);
+  float4 f;
+  if (!take_scattered(a, 0, i, a.sc_ctr[a.sc_list], f)) return;
   clear_nonfin(a, i, 0xfffu);
   const float4 g = a.gx_next[i];
   a.gx_next[i] = make_float4(g.x + f.x, g.y + f.y, g.z + f.z, 0.f);
-  if (kLambda) a.lbar[i] += f.w;
 }
 
 // ---- delta_p -----------------------------------------------------------------------
 
-// Recomputes P_i (the forward's sum), applies the clamps' transposes.  Writes
-// Pbar, starts the X_k adjoint with ubar, and adds this block's wall
-// adjoints to wall_part[block][6] (ulim xyz, llim xyz).
-template <int L>
+// Lists every particle's neighbours, recomputes P_i (the forward's sum) and the
+// lambda sums (G_i and D_i), applies the clamps' transposes.  Writes Pbar,
+// starts the X_k adjoint with ubar, and leaves this block's wall adjoints in
+// wall_part[block][6] (ulim xyz, llim xyz).  kLong: as k_bwd_xsph's.
+template <int L, bool kLong>
 __global__ void __launch_bounds__(kThreads)
-k_bwd_dp1(BackwardArgs a, const float4* __restrict__ X, const float* __restrict__ lam) {
+k_bwd_window(BackwardArgs a, const float4* __restrict__ X, const float* __restrict__ lam, float* __restrict__ wall_part) {
   const StepConsts& c = a.c;
-  __shared__ float wall[6][kThreads];
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / L, lane = tid % L;
+  __shared__ float wall[6][kThreads / 32];
+  struct Own {
+    float4 x;
+    float lam;
+    unsigned long long cell;
+    int i;
+  };
+  struct Pair {
+    float4 x;
+    float lam;
+    unsigned long long cell;
+  };
+  const auto own = [&](int k) { return Own{ld4(X, k), __ldg(lam + k), a.gcell[k], k}; };
+  const auto load = [&](int j) { return Pair{ld4(X, j), __ldg(lam + j), a.kcell[j]}; };
+  // P (0-2), G (3-5), sum of |g_ij|^2 (6)
+  const auto visit = [&](const Own& o, Sums<7>& s, int j, bool, const Pair& t, uint32_t* entry) {
+    if (entry && !near_cell(o.cell, t.cell)) *entry = (uint32_t)j | kOneSided;
+    const float ex = o.x.x - t.x.x, ey = o.x.y - t.x.y, ez = o.x.z - t.x.z;
+    const float r2 = dist2(ex, ey, ez);
+    if (r2 >= c.h2 || r2 < c.keps2) return;
+    const float ir = rsqrtf(r2);
+    const float d = c.h - r2 * ir;
+    const float sc = c.spiky_coef_rho0 * d * d * ir;
+    s.v[3] += sc * ex;
+    s.v[4] += sc * ey;
+    s.v[5] += sc * ez;
+    if (j != o.i) {
+      const float corr = c.coef_corr * pow_corr(c, poly6_inside(c, r2));
+      const float f = (o.lam + t.lam + corr) * (c.spiky_coef * d * d * ir);
+      s.v[0] = fmaf(f, ex, s.v[0]);
+      s.v[1] = fmaf(f, ey, s.v[1]);
+      s.v[2] = fmaf(f, ez, s.v[2]);
+      s.v[6] += dist2(sc * ex, sc * ey, sc * ez);
+    }
+  };
   float w6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  float Px = 0.f, Py = 0.f, Pz = 0.f;
-  if (i < a.n) {
-    const float4 xi = ld4(X, i);
-    const float li = lam[i];
+  const auto finish = [&](int i, const Sums<7>& s) {
     const SceneGeom g = geom_of(c, a.G, i);
-    for_window(g, a.cs, a.n, cell_of(c, g, xi), [&](int j) {
-      const float4 xj = ld4(X, j);
-      const float ex = xi.x - xj.x, ey = xi.y - xj.y, ez = xi.z - xj.z;
-      const float r2 = dist2(ex, ey, ez);
-      if (!(r2 >= c.h2) && !(r2 < c.keps2) && j != i) {
-        const float corr = c.coef_corr * pow_corr(c, poly6_inside(c, r2));
-        const float ir = rsqrtf(r2);
-        const float t = c.h - r2 * ir;
-        const float f = (li + __ldg(lam + j) + corr) * (c.spiky_coef * t * t * ir);
-        Px = fmaf(f, ex, Px);
-        Py = fmaf(f, ey, Py);
-        Pz = fmaf(f, ez, Pz);
-      }
-    }, lane, L);
-    Px = lane_sum<L>(Px);
-    Py = lane_sum<L>(Py);
-    Pz = lane_sum<L>(Pz);
-  }
-  if (i < a.n && lane == 0) {
-    const float4 xi = ld4(X, i);
-    const SceneGeom g = geom_of(c, a.G, i);
-    const float4 gn = ld4(a.gx, i);  // adjoint of X_{k+1}
-    const float P[3] = {Px, Py, Pz}, x[3] = {xi.x, xi.y, xi.z}, gin[3] = {gn.x, gn.y, gn.z};
+    const float4 xi = ld4(X, i), gn = ld4(a.gx, i);  // gx: the adjoint of X_{k+1}
+    const float x[3] = {xi.x, xi.y, xi.z}, gin[3] = {gn.x, gn.y, gn.z};
     float ub[3], pb[3];
+#pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-      const float dpa = P[ax] / c.pho0;
+      const float dpa = s.v[ax] / c.pho0;
       const float u = x[ax] + fmaxf(fminf(dpa, c.max_dp), -c.max_dp);
       ub[ax] = gin[ax];
       if (u > g.hi[ax]) {
-        w6[ax] = gin[ax];
+        w6[ax] += gin[ax];
         ub[ax] = 0.f;
       } else if (u < g.lo[ax]) {
-        w6[3 + ax] = gin[ax];
+        w6[3 + ax] += gin[ax];
         ub[ax] = 0.f;
       }
       pb[ax] = (dpa < c.max_dp && dpa > -c.max_dp) ? ub[ax] / c.pho0 : 0.f;
     }
-    a.pbar[i] = make_float4(pb[0], pb[1], pb[2], 0.f);
+    a.pbar[i] = make_float4(pb[0], pb[1], pb[2], lam[i]);
     a.gx_next[i] = make_float4(ub[0], ub[1], ub[2], 0.f);
-    a.kcell[i] = pack_cell(cell_of(c, g, xi));
+    a.gs[i] = make_float4(s.v[3], s.v[4], s.v[5], s.v[6] + dist2(s.v[3], s.v[4], s.v[5]) + c.lambda_eps);
+  };
+  if constexpr (kLong) {
+    finish_long<7>(a, X, gridDim.x, own, load, visit, finish);
+  } else {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = tid / L, lane = tid % L;
+    if (i < a.n) {
+      const int cnt = list_hits<L>(a, X, ld4(X, i), i, lane);
+      if (lane == 0) a.hit_n[i] = cnt;
+      finish_listed<L, 7>(a, X, i, lane, cnt, own, load, visit, finish);
+    }
   }
-  // this block's wall adjoints, summed in thread order
-  for (int k = 0; k < 6; ++k) wall[k][threadIdx.x] = w6[k];
-  __syncthreads();
+  // this block's wall adjoints, added in a fixed tree (mostly all zero)
+  const bool some = w6[0] != 0.f || w6[1] != 0.f || w6[2] != 0.f || w6[3] != 0.f || w6[4] != 0.f || w6[5] != 0.f;
+  const bool any = __syncthreads_or(some) != 0;
+  if (any) {
+    for (int k = 0; k < 6; ++k) {
+      float v = w6[k];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if ((threadIdx.x & 31) == 0) wall[k][threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+  }
   if (threadIdx.x < 6) {
     float sum = 0.f;
-    for (int k = 0; k < kThreads; ++k) sum += wall[threadIdx.x][k];
-    a.wall_part[blockIdx.x * 6 + threadIdx.x] = sum;
+    if (any)
+      for (int k = 0; k < kThreads / 32; ++k) sum += wall[threadIdx.x][k];
+    wall_part[blockIdx.x * 6 + threadIdx.x] = sum;
   }
 }
 
+// long_blocks: with one lane per particle, the first blocks take the particles
+// without a list.
 template <int L>
 __global__ void __launch_bounds__(kThreads)
-k_bwd_dp2(BackwardArgs a, const float4* __restrict__ X, const float* __restrict__ lam) {
+k_bwd_delta_p(BackwardArgs a, const float4* __restrict__ X, int long_blocks) {
   const StepConsts& c = a.c;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / L, lane = tid % L;
-  if (i >= a.n) return;
-  const float4 xi = ld4(X, i), pbi4 = ld4(a.pbar, i);
-  const Vec pbi = {pbi4.x, pbi4.y, pbi4.z};
-  const float li = lam[i];
-  const unsigned long long gci = a.gcell[i];
-  const SceneGeom g = geom_of(c, a.G, i);
-  Vec xb = {0.f, 0.f, 0.f};
-  float lb = 0.f;
-  for_window(g, a.cs, a.n, cell_of(c, g, xi), [&](int j) {
-    if (j == i) return;
-    const float4 xj = ld4(X, j);
-    const Vec r = vsub(xi, xj);
+  struct Own {
+    float4 x, p;
+    int i;
+  };
+  const auto own = [&](int k) { return Own{ld4(X, k), ld4(a.pbar, k), k}; };
+  const auto load = [&](int j) { return Two{ld4(X, j), ld4(a.pbar, j)}; };
+  const auto visit = [&](const Own& o, Sums<4>& s, int j, bool one_sided, const Two& t, uint32_t*) {
+    const Vec r = vsub(o.x, t.x);
     const float q = vdot(r, r);
-    if (!(q < c.h2) || q < c.keps2) return;
+    if (!(q < c.h2) || q < c.keps2 || j == o.i) return;
     float phi, k;
-    spiky_parts(c, sqrtf(q), phi, k);
-    const Vec F = {phi * r.x, phi * r.y, phi * r.z};
+    spiky_parts(c, q, phi, k);
     const float wq = poly6_inside(c, q);
-    const float lsum = li + __ldg(lam + j) + c.coef_corr * pow_corr(c, wq);
+    const float lsum = o.p.w + t.b.w + c.coef_corr * pow_corr(c, wq);
     const float dsdq = c.npow == 4 ? 4.f * c.coef_corr * wq * wq * wq * dpoly6(c, q)
                                    : c.coef_corr * c.n_corr * powf(wq, c.n_corr - 1.f) * dpoly6(c, q);
-    // P_i's term (lambda_i + lambda_j + s_ij) F(r_ij): its adjoint on lambda_i and x_i
-    const float fi = vdot(F, pbi);
-    const Vec Ji = jac(phi, k, r, pbi);
-    const Vec oi = {lsum * Ji.x + 2.f * dsdq * r.x * fi, lsum * Ji.y + 2.f * dsdq * r.y * fi,
-                    lsum * Ji.z + 2.f * dsdq * r.z * fi};
-    lb += fi;
-    xb.x += oi.x;
-    xb.y += oi.y;
-    xb.z += oi.z;
-    if (near_cell(gci, a.kcell[j])) {
-      // P_j's term on lambda_i and x_i (F and r change sign, J does not)
-      const float4 pbj4 = ld4(a.pbar, j);
-      const Vec pbj = {pbj4.x, pbj4.y, pbj4.z};
-      const float fj = vdot(F, pbj);
-      const Vec Jj = jac(phi, k, r, pbj);
-      lb -= fj;
-      xb.x -= lsum * Jj.x + 2.f * dsdq * r.x * fj;
-      xb.y -= lsum * Jj.y + 2.f * dsdq * r.y * fj;
-      xb.z -= lsum * Jj.z + 2.f * dsdq * r.z * fj;
-    } else {
-      // j cannot gather P_i's term: scatter its adjoint on lambda_j and x_j
-      scatter_term(a, 0, j, -oi.x, -oi.y, -oi.z, fi);
-    }
-  }, lane, L);
-  xb = lane_sum<L>(xb);
-  lb = lane_sum<L>(lb);
-  if (lane != 0) return;
-  const float4 u = ld4(a.gx_next, i);
-  a.gx_next[i] = make_float4(u.x + xb.x, u.y + xb.y, u.z + xb.z, 0.f);
-  a.lbar[i] = lb;
+    // P_i's term (lambda_i + lambda_j + s_ij) F(r_ij) and, when i is in j's
+    // window, P_j's (F and r change sign, J does not): their adjoints on
+    // lambda_i and x_i, from d = Pbar_i - Pbar_j
+    Vec d = {o.p.x, o.p.y, o.p.z};
+    if (!one_sided) d = vsub(o.p, t.b);
+    const float rd = vdot(r, d), fd = phi * rd;
+    const float u = lsum * phi, v = lsum * k * rd + 2.f * dsdq * fd;
+    const Vec x = {u * d.x + v * r.x, u * d.y + v * r.y, u * d.z + v * r.z};
+    s.v[0] += x.x;
+    s.v[1] += x.y;
+    s.v[2] += x.z;
+    s.v[3] += fd;
+    // j cannot gather P_i's term: scatter its adjoint on lambda_j and x_j
+    if (one_sided) scatter_term(a, 0, j, -x.x, -x.y, -x.z, fd);
+  };
+  const auto finish = [&](int i, const Sums<4>& s) {
+    const float4 u = ld4(a.gx_next, i);
+    a.gx_next[i] = make_float4(u.x + s.v[0], u.y + s.v[1], u.z + s.v[2], 0.f);
+    a.lbar[i] = s.v[3];
+  };
+  if (L == 1 && (int)blockIdx.x < long_blocks) {
+    finish_long<4>(a, X, long_blocks, own, load, visit, finish);
+    return;
+  }
+  const int tid = ((int)blockIdx.x - long_blocks) * kThreads + threadIdx.x;
+  const int i = tid / L, lane = tid % L;
+  if (i < a.n) finish_listed<L, 4>(a, X, i, lane, a.hit_n[i], own, load, visit, finish);
 }
 
 // ---- lambda ------------------------------------------------------------------------
 
-template <int L>
-__global__ void __launch_bounds__(kThreads)
-k_bwd_lam1(BackwardArgs a, const float4* __restrict__ X, const float* __restrict__ lam, int last) {
-  const StepConsts& c = a.c;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / L, lane = tid % L;
+// Folds the delta_p sums' scattered adjoints in and clears their scratch; then
+// the constraint's adjoints: Sbar_i beside 2 Sbar_i G_i, rho's beside X_i.
+__global__ void __launch_bounds__(256)
+k_bwd_fix_lambda(BackwardArgs a, const float4* __restrict__ X, const float* __restrict__ lam, int last) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
-  const float4 xi = ld4(X, i);
-  const SceneGeom g = geom_of(c, a.G, i);
-  float gx = 0.f, gy = 0.f, gz = 0.f, gl2 = 0.f;
-  for_window(g, a.cs, a.n, cell_of(c, g, xi), [&](int j) {
-    const float4 xj = ld4(X, j);
-    const float ex = xi.x - xj.x, ey = xi.y - xj.y, ez = xi.z - xj.z;
-    const float r2 = dist2(ex, ey, ez);
-    if (!(r2 >= c.h2) && !(r2 < c.keps2)) {
-      const float ir = rsqrtf(r2);
-      const float t = c.h - r2 * ir;
-      const float sc = c.spiky_coef_rho0 * t * t * ir;
-      gx += sc * ex;
-      gy += sc * ey;
-      gz += sc * ez;
-      if (j != i) gl2 += dist2(sc * ex, sc * ey, sc * ez);
-    }
-  }, lane, L);
-  gx = lane_sum<L>(gx);
-  gy = lane_sum<L>(gy);
-  gz = lane_sum<L>(gz);
-  gl2 = lane_sum<L>(gl2);
-  if (lane != 0) return;
-  const float D = gl2 + dist2(gx, gy, gz) + c.lambda_eps;
-  const float lb = a.lbar[i];
-  const float cbar = -lb / D;
-  const float sbar = -lb * lam[i] / D;
-  a.gs[i] = make_float4(gx, gy, gz, sbar);
-  a.rtot[i] = (last ? a.grho[i] : 0.f) + cbar / c.pho0;
+  float lb = a.lbar[i];
+  float4 f;
+  if (take_scattered(a, 0, i, a.sc_ctr[a.sc_list], f)) {
+    clear_nonfin(a, i, 0xfffu);
+    const float4 g = a.gx_next[i];
+    a.gx_next[i] = make_float4(g.x + f.x, g.y + f.y, g.z + f.z, 0.f);
+    lb += f.w;
+  }
+  const float4 g = a.gs[i], x = ld4(X, i);
+  const float cbar = -lb / g.w;
+  const float sbar = -lb * lam[i] / g.w;
+  const float s2 = 2.f * sbar;
+  a.gs[i] = make_float4(s2 * g.x, s2 * g.y, s2 * g.z, s2);
+  a.pbar[i] = make_float4(x.x, x.y, x.z, (last ? a.grho[i] : 0.f) + cbar / a.c.pho0);
 }
 
 template <int L>
 __global__ void __launch_bounds__(kThreads)
-k_bwd_lam2(BackwardArgs a, const float4* __restrict__ X) {
+k_bwd_lambda(BackwardArgs a, int long_blocks) {
   const StepConsts& c = a.c;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = tid / L, lane = tid % L;
-  if (i >= a.n) return;
-  const float4 xi = ld4(X, i), gsi = ld4(a.gs, i);
-  const float rti = a.rtot[i];
-  const unsigned long long gci = a.gcell[i];
-  const SceneGeom g = geom_of(c, a.G, i);
-  Vec xb = {0.f, 0.f, 0.f};
-  for_window(g, a.cs, a.n, cell_of(c, g, xi), [&](int j) {
-    if (j == i) return;
-    const float4 xj = ld4(X, j);
-    const Vec r = vsub(xi, xj);
+  struct Own {
+    float4 x, g;
+    int i;
+  };
+  const auto own = [&](int k) { return Own{ld4(a.pbar, k), ld4(a.gs, k), k}; };
+  const auto load = [&](int j) { return Two{ld4(a.pbar, j), ld4(a.gs, j)}; };
+  const auto visit = [&](const Own& o, Sums<3>& s, int j, bool one_sided, const Two& t, uint32_t*) {
+    const Vec r = vsub(o.x, t.x);
     const float q = vdot(r, r);
-    if (!(q < c.h2)) return;
-    const bool recip = near_cell(gci, a.kcell[j]);
-    // rho_i's term W(q): 2 W'(q) r rhobar_i on x_i; rho_j's the same with rhobar_j
-    const float dw = 2.f * dpoly6(c, q);
-    float wt = dw * rti;
-    if (recip) wt += dw * a.rtot[j];
-    xb.x += wt * r.x;
-    xb.y += wt * r.y;
-    xb.z += wt * r.z;
-    // what j cannot gather: rho_i's (and below S_i's) terms on x_j
-    float sx = recip ? 0.f : -dw * rti * r.x, sy = recip ? 0.f : -dw * rti * r.y,
-          sz = recip ? 0.f : -dw * rti * r.z;
+    if (!(q < c.h2) || j == o.i) return;
+    // rho_i's term W(q) and, when i is in j's window, rho_j's: 2 W'(q) r times
+    // the adjoints of rho on x_i, minus that on x_j
+    const float wt = 2.f * dpoly6(c, q) * (one_sided ? o.x.w : o.x.w + t.x.w);
+    Vec x = {wt * r.x, wt * r.y, wt * r.z};
     if (!(q < c.keps2)) {
       // S_i's terms |g_ij|^2 + the g_ij part of |G_i|^2, g_ij = F / pho0:
-      // a_ij = 2 Sbar_i (g_ij + G_i); J a_ij / pho0 on x_i, minus that on x_j
+      // a_ij = 2 Sbar_i (g_ij + G_i); S_j's a_ji = 2 Sbar_j (-g_ij + G_j):
+      // J (a_ij - a_ji) / pho0 on x_i, minus that on x_j
       float phi, k;
-      spiky_parts(c, sqrtf(q), phi, k);
-      const float si = gsi.w;
-      const Vec ai = {2.f * si * (phi * r.x * c.inv_pho0 + gsi.x), 2.f * si * (phi * r.y * c.inv_pho0 + gsi.y),
-                      2.f * si * (phi * r.z * c.inv_pho0 + gsi.z)};
-      const Vec Ji = jac(phi, k, r, ai);
-      xb.x += Ji.x * c.inv_pho0;
-      xb.y += Ji.y * c.inv_pho0;
-      xb.z += Ji.z * c.inv_pho0;
-      if (recip) {
-        // S_j's: a_ji = 2 Sbar_j (-g_ij + G_j); -J a_ji / pho0 on x_i
-        const float4 gsj = ld4(a.gs, j);
-        const float sj = gsj.w;
-        const Vec aj = {2.f * sj * (-phi * r.x * c.inv_pho0 + gsj.x), 2.f * sj * (-phi * r.y * c.inv_pho0 + gsj.y),
-                        2.f * sj * (-phi * r.z * c.inv_pho0 + gsj.z)};
-        const Vec Jj = jac(phi, k, r, aj);
-        xb.x -= Jj.x * c.inv_pho0;
-        xb.y -= Jj.y * c.inv_pho0;
-        xb.z -= Jj.z * c.inv_pho0;
-      } else {
-        sx -= Ji.x * c.inv_pho0;
-        sy -= Ji.y * c.inv_pho0;
-        sz -= Ji.z * c.inv_pho0;
+      spiky_parts(c, q, phi, k);
+      Vec v = {o.g.x, o.g.y, o.g.z};
+      float s2 = o.g.w;
+      if (!one_sided) {
+        v = vsub(o.g, t.b);
+        s2 += t.b.w;
       }
+      const float m = phi * c.inv_pho0, sp = s2 * m;
+      v = {v.x + sp * r.x, v.y + sp * r.y, v.z + sp * r.z};
+      const float n = k * vdot(r, v) * c.inv_pho0;
+      x = {x.x + (m * v.x + n * r.x), x.y + (m * v.y + n * r.y), x.z + (m * v.z + n * r.z)};
     }
-    if (!recip) scatter_term(a, 0, j, sx, sy, sz, 0.f);
-  }, lane, L);
-  xb = lane_sum<L>(xb);
-  if (lane != 0) return;
-  const float4 u = ld4(a.gx_next, i);
-  a.gx_next[i] = make_float4(u.x + xb.x, u.y + xb.y, u.z + xb.z, 0.f);
+    s.v[0] += x.x;
+    s.v[1] += x.y;
+    s.v[2] += x.z;
+    if (one_sided) scatter_term(a, 0, j, -x.x, -x.y, -x.z, 0.f);
+  };
+  const auto finish = [&](int i, const Sums<3>& s) {
+    const float4 u = ld4(a.gx_next, i);
+    a.gx_next[i] = make_float4(u.x + s.v[0], u.y + s.v[1], u.z + s.v[2], 0.f);
+  };
+  if (L == 1 && (int)blockIdx.x < long_blocks) {
+    finish_long<3>(a, a.pbar, long_blocks, own, load, visit, finish);
+    return;
+  }
+  const int tid = ((int)blockIdx.x - long_blocks) * kThreads + threadIdx.x;
+  const int i = tid / L, lane = tid % L;
+  if (i < a.n) finish_listed<L, 3>(a, a.pbar, i, lane, a.hit_n[i], own, load, visit, finish);
 }
 
 // ---- advection and the permutation ---------------------------------------------------
@@ -607,34 +861,12 @@ __global__ void __launch_bounds__(256)
 k_bwd_out(BackwardArgs a, const uint32_t* __restrict__ perm, float4* __restrict__ g_pos,
           float4* __restrict__ g_vel) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < 2) a.sc_ctr[2 * k] = 0u;  // both lists, for the next call
   if (k >= a.n) return;
   const float4 gs = ld4(a.gx, k), g0 = ld4(a.gx0, k);
   const uint32_t p = min(perm[k], (uint32_t)(a.n - 1));
   g_pos[p] = make_float4(gs.x + g0.x, gs.y + g0.y, gs.z + g0.z, 0.f);
   g_vel[p] = make_float4(a.c.dt * gs.x, a.c.dt * gs.y, a.c.dt * gs.z, 0.f);
-}
-
-// Sums the blocks' wall adjoints into g_lim[6] (accumulating) in a fixed
-// order: thread t of one block adds the parts of blocks t, t + kWallThreads,
-// ... in turn, then the threads' sums are added pairwise in a fixed tree.
-constexpr int kWallThreads = 256;
-__global__ void __launch_bounds__(kWallThreads)
-k_bwd_wall(const float* __restrict__ part, int blocks, float* __restrict__ g_lim) {
-  __shared__ float s[6][kWallThreads];
-  float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int b = threadIdx.x; b < blocks; b += kWallThreads)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) acc[k] += part[b * 6 + k];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) s[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int w = kWallThreads / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-#pragma unroll
-      for (int k = 0; k < 6; ++k) s[k][threadIdx.x] += s[k][threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x < 6) g_lim[threadIdx.x] += s[threadIdx.x][0];
 }
 
 // ---- density grid ---------------------------------------------------------------------
@@ -856,21 +1088,26 @@ cudaError_t run_backward(BackwardArgs a, const BackwardTape& t, const uint32_t* 
   const int blocks = (int)(((long long)a.n * L + kThreads - 1) / kThreads);
   const int blocks256 = (a.n + 255) / 256;
   const int acc_blocks = a.c.dense_grid;
-  k_bwd_xsph<L><<<blocks, kThreads, 0, stream>>>(a);
-  k_bwd_acc<<<acc_blocks, 256, 0, stream>>>(a);
-  k_bwd_fix_xsph<<<blocks256, 256, 0, stream>>>(a);
-  for (int k = t.niter - 1; k >= 0; --k) {
+  const int K = t.niter;
+  const int longs = L == 1 ? kLongBlocks * acc_blocks : 0;  // blocks for the particles without a list
+  k_bwd_xsph<L, false><<<blocks, kThreads, 0, stream>>>(a);
+  if constexpr (L == 1) k_bwd_xsph<1, true><<<longs, kThreads, 0, stream>>>(a);
+  k_bwd_acc<<<acc_blocks, kWallThreads, 0, stream>>>(a, 0, g_lim);
+  k_bwd_fix_xsph<<<blocks256, 256, 0, stream>>>(a, K > 0 ? t.X[K - 1] : nullptr);
+  a.sc_list ^= 2;
+  for (int k = K - 1; k >= 0; --k) {
     const float4* X = t.X[k];
     const float* lam = t.lambda[k];
-    k_bwd_dp1<L><<<blocks, kThreads, 0, stream>>>(a, X, lam);  // also the packed cells of X_k
-    k_bwd_wall<<<1, kWallThreads, 0, stream>>>(a.wall_part, blocks, g_lim);
-    k_bwd_dp2<L><<<blocks, kThreads, 0, stream>>>(a, X, lam);
-    k_bwd_acc<<<acc_blocks, 256, 0, stream>>>(a);
-    k_bwd_fix<true><<<blocks256, 256, 0, stream>>>(a);
-    k_bwd_lam1<L><<<blocks, kThreads, 0, stream>>>(a, X, lam, k == t.niter - 1);
-    k_bwd_lam2<L><<<blocks, kThreads, 0, stream>>>(a, X);
-    k_bwd_acc<<<acc_blocks, 256, 0, stream>>>(a);
-    k_bwd_fix<false><<<blocks256, 256, 0, stream>>>(a);
+    k_bwd_window<L, false><<<blocks, kThreads, 0, stream>>>(a, X, lam, a.wall_part);
+    if constexpr (L == 1) k_bwd_window<1, true><<<longs, kThreads, 0, stream>>>(a, X, lam, a.wall_part + 6 * blocks);
+    k_bwd_delta_p<L><<<longs + blocks, kThreads, 0, stream>>>(a, X, longs);
+    k_bwd_acc<<<acc_blocks + 1, kWallThreads, 0, stream>>>(a, blocks + longs, g_lim);
+    k_bwd_fix_lambda<<<blocks256, 256, 0, stream>>>(a, X, lam, k == K - 1);
+    a.sc_list ^= 2;
+    k_bwd_lambda<L><<<longs + blocks, kThreads, 0, stream>>>(a, longs);
+    k_bwd_acc<<<acc_blocks, kWallThreads, 0, stream>>>(a, 0, g_lim);
+    k_bwd_fix<<<blocks256, 256, 0, stream>>>(a, k > 0 ? t.X[k - 1] : nullptr);
+    a.sc_list ^= 2;
     // the adjoint of X_k becomes the input of the next (earlier) iteration
     float4* tmp = a.gx;
     a.gx = a.gx_next;
@@ -879,7 +1116,6 @@ cudaError_t run_backward(BackwardArgs a, const BackwardTape& t, const uint32_t* 
   k_bwd_out<<<(a.n + 255) / 256, 256, 0, stream>>>(a, perm, (float4*)g_pos, (float4*)g_vel);
   return cudaGetLastError();
 }
-
 
 cudaError_t backward(const BackwardArgs& args, const BackwardTape& t, const uint32_t* perm,
                      const void* g_npos, const void* g_nvel, void* g_pos, void* g_vel,
@@ -892,8 +1128,7 @@ cudaError_t backward(const BackwardArgs& args, const BackwardTape& t, const uint
   a.XK = t.X[t.niter];
   a.X0 = t.X[0];
   const int blocks256 = (a.n + 255) / 256;
-  k_bwd_cells<<<blocks256, 256, 0, stream>>>(a, a.X0, a.gcell);
-  k_bwd_cells<<<blocks256, 256, 0, stream>>>(a, a.XK, a.kcell);
+  k_bwd_start<<<blocks256, 256, 0, stream>>>(a);
   if (a.n < kWarpPerParticleBelow) {
     if (a.lanes == 8) return run_backward<8>(a, t, perm, g_pos, g_vel, g_lim, stream);
     if (a.lanes == 16) return run_backward<16>(a, t, perm, g_pos, g_vel, g_lim, stream);

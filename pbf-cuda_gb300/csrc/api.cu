@@ -139,7 +139,8 @@ struct pbf_solver {
   } tape_meta[kMaxTapeDepth];
   float4* bw4;               // 7 * max_particles: gx, gx_next, gx0, pbar, gs, fix, fixv
   unsigned char* bw_sc;      // the reverse pass's exact-scatter scratch (scatter_bytes)
-  float* bw1;                // 4 * max_particles: grho, lbar, rtot (+ spare)
+  float* bw1;                // 3 * max_particles: grho, lbar, the lists' lengths (int)
+  uint32_t* bw_hits;         // kHitCap * max_particles: the reverse pass's neighbour lists
   unsigned long long* bw8;   // 2 * max_particles: packed grid cells, packed current cells
   float* wall_part;          // 6 * blocks
   const uint32_t* last_perm;
@@ -437,7 +438,7 @@ void free_all(pbf_solver* s) {
   s->cache.clear();
   s->bw_cache.clear();
   if (s->cap_stream) cudaStreamDestroy(s->cap_stream);
-  void* tape[] = {s->tape_mem, s->bw4, s->bw1, s->bw8, s->wall_part, s->bw_sc};
+  void* tape[] = {s->tape_mem, s->bw4, s->bw1, s->bw8, s->wall_part, s->bw_sc, s->bw_hits};
   for (void* p : tape)
     if (p) cudaFree(p);
 }
@@ -893,7 +894,8 @@ pbf_status pbf_tape_enable(pbf_solver* s, int depth) {
   if (!s->bw4) {
     const size_t blocks = (np * 32 + 127) / 128;  // the reverse kernels' blocks at 32 lanes per particle
     cudaError_t e = alloc(&s->bw4, np * 7);
-    if (e == cudaSuccess) e = alloc(&s->bw1, np * 4);
+    if (e == cudaSuccess) e = alloc(&s->bw1, np * 3);
+    if (e == cudaSuccess) e = alloc(&s->bw_hits, np * pbf::kHitCap);
     if (e == cudaSuccess) e = alloc(&s->bw8, np * 2);
     if (e == cudaSuccess) e = cudaMemset(s->bw4 + 5 * np, 0, sizeof(float4) * 2 * np);
     if (e == cudaSuccess) e = alloc(&s->wall_part, blocks * 6);
@@ -951,7 +953,9 @@ pbf_status pbf_backward(pbf_solver* s, const void* g_npos, const void* g_nvel, v
   a.gs = s->bw4 + 4 * np;
   a.grho = s->bw1;
   a.lbar = s->bw1 + np;
-  a.rtot = s->bw1 + 2 * np;
+  a.hit_n = (int*)(s->bw1 + 2 * np);
+  a.hits = s->bw_hits;
+  a.hit_stride = (int)np;
   a.fix = s->bw4 + 5 * np;
   a.fixv = s->bw4 + 6 * np;
   scatter_layout(s->bw_sc, np, a);

@@ -485,10 +485,10 @@ struct BackwardArgs {
   float4* gx_next;  // adjoint being built for the earlier positions
   float4* gx0;      // velocity-update part of the sorted inputs' adjoint
   float* grho;      // adjoint of the last rho (from XSPH)
-  float4* pbar;     // adjoint of the delta_p sums / pho0 ... / pho0
+  float4* pbar;     // adjoint of the delta_p sums / pho0, w lambda (XSPH: velocity, w rho; lambda: position, w
+                    // the adjoint of rho incl. the constraint's)
   float* lbar;      // adjoint of lambda
-  float4* gs;       // G_i (xyz) and Sbar_i (w)
-  float* rtot;      // adjoint of rho_i incl. the constraint's
+  float4* gs;       // G_i (xyz) and D_i (w); then 2 Sbar_i G_i and Sbar_i
   float* wall_part; // [blocks][6] per-block wall adjoints
   const float4* X0; // predicted positions (the grid's positions; set by backward)
   unsigned long long* gcell;  // packed grid cell of each particle (cell of X0)
@@ -504,9 +504,13 @@ struct BackwardArgs {
   unsigned* sc_max;           // [7][sc_stride] largest finite |term| (float bits); 0 between folds
   unsigned* sc_cnt;           // [2][sc_stride] terms per target (fix, fixv); 0 between folds
   unsigned* sc_nonfin;        // [sc_stride] non-finite terms, 3 bits per component; 0 between folds
-  unsigned* sc_ctr;           // [2] terms listed, terms beyond the capacity; listed is 0 between folds
+  unsigned* sc_ctr;           // [3] terms listed (list 0), terms beyond the capacity, terms listed (list 2)
+  int sc_list;                // the list in use: 0 or 2 (its length's index in sc_ctr)
   int sc_cap;
   int sc_stride;
+  uint32_t* hits;   // the neighbours of every particle, kHitCap each, bit 31: not reciprocal
+  int* hit_n;       // their number, -1: more than kHitCap
+  int hit_stride;   // particles the lists hold
   int lanes;        // lanes per particle below kWarpPerParticleBelow particles: 8, 16 or 32
 };
 
