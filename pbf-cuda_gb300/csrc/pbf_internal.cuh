@@ -291,6 +291,7 @@ enum CellFlag : uint32_t {
   kCellLambdaNonFinite = 1u,
   kCellRhoNotPositive = 2u,  // rho <= 0 or NaN
   kCellVelNonFinite = 4u,
+  kCellPoison = 8u,          // xsph over pairs: a density of the last lambda pass or a velocity is such
 };
 // Bits kCellSlotShift.. of cell_flags hold 1 + the group slot of a cell that
 // holds >= kGroupCell particles (0: none), set once per step by reorder.

@@ -823,14 +823,21 @@ struct XsphPass {
     if (!(r2 >= c.h2)) {  // NaN-inclusive, as getPoly6
       pair(vj, r2);
     } else if (exact) {
-      // W = 0: 2 (v_j - v_i) * 0 / (rho_i + rho_j) is NaN iff the velocity
-      // difference is not finite or the denominator is 0 or NaN
-      const float den = ri + vj.w;
-      const bool bad_den = !(den != 0.f) || isnan(den);
-      px |= bad_den || !isfinite(vj.x - vi.x);
-      py |= bad_den || !isfinite(vj.y - vi.y);
-      pz |= bad_den || !isfinite(vj.z - vi.z);
+      miss(vj);
     }
+  }
+  // A candidate outside the cutoff (W = 0): 2 (v_j - v_i) * 0 / (rho_i + rho_j) is
+  // NaN iff the velocity difference is not finite or the denominator is 0 or NaN.
+  __device__ __forceinline__ void miss(float4 vj) {
+    const float den = ri + vj.w;
+    const bool bad_den = !(den != 0.f) || isnan(den);
+    px |= bad_den || !isfinite(vj.x - vi.x);
+    py |= bad_den || !isfinite(vj.y - vi.y);
+    pz |= bad_den || !isfinite(vj.z - vi.z);
+  }
+  // miss() for a candidate outside the cutoff.
+  __device__ __forceinline__ void miss_beyond(float4 xj, float4 vj) {
+    if (dist2(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z) >= c.h2) miss(vj);
   }
   // Two particles at r2 < h2, a then b (b only if `two`), not on the exact path.
   __device__ __forceinline__ void visit_two(float4 xa, float4 xb, float4 va, float4 vb, bool two) {
@@ -904,6 +911,16 @@ __device__ __forceinline__ bool exact_path(int kind, const PassArgs& a, const Sc
            window_flagged(g, a.cell_flags, q, kCellRhoNotPositive | kCellVelNonFinite);
   }
   return false;
+}
+
+// Whether only a window's flagged cells can poison the xsph sum of a particle
+// with this velocity and density: elsewhere 0 < rho_j, v_j is finite, and
+// |v_j - v_i| then rounds to a finite number (kTameSpeed is below half a unit in
+// the last place of the largest).
+constexpr float kTameSpeed = 1e30f;
+__device__ __forceinline__ bool tame(float4 vr) {
+  return vr.w > 0.f && isfinite(vr.w) && fabsf(vr.x) < kTameSpeed && fabsf(vr.y) < kTameSpeed &&
+         fabsf(vr.z) < kTameSpeed;
 }
 
 // ---- window staging: bulk async copies into shared memory ------------------------------
@@ -1562,8 +1579,14 @@ __global__ void __launch_bounds__(kSparseThreads, 8) k_sparse_pair(PassArgs a) {
     if (kKind == kLambda) a.hit_n[h] = a.hit_n[h + 32] = grouped ? kHitsWalk : kHitsDense;
     return;
   }
-  const bool exact0 = exact_path(kKind, a, g, q, i.x), exact1 = two && exact_path(kKind, a, g, q, i.y);
-  if (!grouped && !exact0 && !exact1 && fits && fast_hits(a, x0) && fast_hits(a, x1)) {
+  bool plain = true;  // xsph: k_xsph_poison looks for what poisons the sums (see there)
+  if (kKind == kXsph && a.flags[kFlagXsphExact] != 0u) {
+    if (a.flags[kGroupCount] != 0u)  // (one particle per pair then)
+      plain = !exact_path(kKind, a, g, q, i.x) && (!two || !exact_path(kKind, a, g, q, i.y));
+    else
+      plain = tame(a.VR[i.x]) && (!two || tame(a.VR[i.y]));
+  }
+  if (!grouped && plain && fits && fast_hits(a, x0) && fast_hits(a, x1)) {
     const int3 hits = queue_pair(a, col, x0, x1);
     {
       P p(a, g, x0, i.x, false);
@@ -1582,8 +1605,70 @@ __global__ void __launch_bounds__(kSparseThreads, 8) k_sparse_pair(PassArgs a) {
   for (int u = 0; u < (two ? 2 : 1); ++u) {
     bool f;
     if (u) window_runs(g, a.cs, a.n, q, col, f);  // the first walk's queue has taken their place
-    sparse_one<kKind>(a, g, q, col, h + 32 * u, u ? i.y : i.x, u ? x1 : x0, u ? exact1 : exact0, grouped, entries,
-                      fits);
+    const int k = u ? i.y : i.x;
+    sparse_one<kKind>(a, g, q, col, h + 32 * u, k, u ? x1 : x0, exact_path(kKind, a, g, q, k), grouped, entries, fits);
+  }
+}
+
+// The exact path of the xsph pass over pairs, for the particles whose neighbours
+// k_sparse_pair took as ever: the candidates beyond them that poison the sum of a
+// tame particle lie in cells that hold a particle with such a density or
+// velocity now (k_xsph_mark; kCellRhoNotPositive has gathered those of every
+// iteration), a few of a window's 27.  Nothing to do, but for two launches (3 us
+// each), in a step without any.  The exact walk, which visits every candidate of
+// the window, held up its warp's other lanes: the pass in an ensemble of
+// 4,714,514 particles (4,303 of them not finite) 1,933 -> 735 us and 326 for
+// these two; the same code in k_sparse_pair spilled and cost a step without such
+// particles 50 us; a warp per particle, a lane per cell, took 1,048 us.  Steps
+// with grouped cells keep the walk (1,048,576 clustered particles: the pass 178 us,
+// 204 this way).
+__global__ void __launch_bounds__(256) k_xsph_mark(PassArgs a) {
+  if (a.flags[kFlagXsphExact] == 0u || a.flags[kGroupCount] != 0u) return;
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= a.n) return;
+  const float4 vr = a.VR[i];
+  if (vr.w > 0.f && isfinite(vr.w) && isfinite(vr.x) && isfinite(vr.y) && isfinite(vr.z)) return;
+  uint32_t* f = a.cell_flags + a.skeys[i];
+  if (!(*reinterpret_cast<volatile uint32_t*>(f) & kCellPoison)) atomicOr(f, (uint32_t)kCellPoison);
+}
+
+__global__ void __launch_bounds__(256) k_xsph_poison(PassArgs a) {
+  if (a.flags[kFlagXsphExact] == 0u || a.flags[kGroupCount] != 0u) return;
+  const int pair = blockIdx.x * 256 + threadIdx.x;
+  if (2 * pair >= work_count(a)) return;
+  const int2 i = __ldg(reinterpret_cast<const int2*>(a.list) + pair);
+  const bool two = i.y >= 0;
+  const float4 x0 = a.X[i.x], x1 = two ? a.X[i.y] : x0;
+  const SceneGeom g = geom_of(a.c, a.G, i.x);
+  const int3 q = cell_of(a.c, g, x0);  // x1's too
+  uint32_t cells = 0u;
+#pragma unroll
+  for (int k = 0; k < 27; ++k) {
+    const int x = q.x + k / 9 - 1, y = q.y + k / 3 % 3 - 1, z = q.z + k % 3 - 1;
+    const bool in = (unsigned)x < (unsigned)g.dims[0] && (unsigned)y < (unsigned)g.dims[1] &&
+                    (unsigned)z < (unsigned)g.dims[2];
+    if (in && (a.cell_flags[cell_index(g, x, y, z)] & kCellPoison)) cells |= 1u << k;
+  }
+  if (cells == 0u || !fast_hits(a, x0) || !fast_hits(a, x1)) return;
+  XsphPass p0(a, g, x0, i.x, true), p1(a, g, x1, two ? i.y : i.x, true);
+  if (!tame(a.VR[i.x]) || (two && !tame(a.VR[i.y]))) return;  // (walked candidate by candidate)
+  for (; cells; cells &= cells - 1u) {
+    const int k = __ffs(cells) - 1;
+    const int cell = cell_index(g, q.x + k / 9 - 1, q.y + k / 3 % 3 - 1, q.z + k % 3 - 1);
+    const int s = (int)__ldg(a.cs + cell), e = min((int)__ldg(a.cs + cell + 1), a.n);
+    if (e - s > a.c.dense_window) return;  // the window is the dense kernel's, or walked with its groups
+    for (int j = s; j < e; ++j) {
+      const float4 xj = __ldg(a.X + j), vj = __ldg(a.VR + j);
+      p0.miss_beyond(xj, vj);
+      p1.miss_beyond(xj, vj);
+    }
+  }
+  const float qnan = __int_as_float(0x7fffffff);
+  for (int u = 0; u < (two ? 2 : 1); ++u) {
+    const XsphPass& p = u ? p1 : p0;
+    if (p.px) a.NV[p.i].x = qnan;
+    if (p.py) a.NV[p.i].y = qnan;
+    if (p.pz) a.NV[p.i].z = qnan;
   }
 }
 
@@ -2792,6 +2877,10 @@ cudaError_t run_pass(const PassArgs& a, cudaStream_t stream) {
     // the sparse kernel has nothing to do
   } else if (kPairs && a.paired) {
     if constexpr (kPairs) k_sparse_pair<kKind><<<sparse_blocks, kSparseThreads, 0, stream>>>(a);
+    if constexpr (kKind == kXsph) {
+      k_xsph_mark<<<(a.n + 255) / 256, 256, 0, stream>>>(a);
+      k_xsph_poison<<<(int)((slots / 2 + 255) / 256), 256, 0, stream>>>(a);
+    }
   } else {
     k_sparse<kKind><<<sparse_blocks, kSparseThreads, 0, stream>>>(a);
   }
