@@ -311,8 +311,10 @@ pbf_status pbf_batch_get_tuning(const pbf_batch* b, pbf_tuning* t);
  * Waits for the solver's work on `stream` (device, as for pbf_step), then
  * returns PBF_ERR_TIMEOUT if a bounded device-side wait gave up since -- a
  * block's copy of candidate positions into shared memory that did not
- * complete; that block then read global memory instead, so the steps'
- * results are unchanged -- else PBF_OK, and clears the record.  No
+ * complete (that block then read global memory instead: the step's results
+ * are unchanged), or a grid barrier of a small step that not every block
+ * reached (that step's results are not valid) -- else PBF_OK, and clears the
+ * record.  No
  * counterpart in the reference, which does not check kernel errors.
  */
 pbf_status pbf_check_device(pbf_solver* s, void* stream);
@@ -323,7 +325,7 @@ pbf_status pbf_batch_check_device(pbf_batch* b, void* stream);
  * default tuning), for callers that cannot allocate device memory (no
  * pbf_solver, so no pbf_create).  It has no counterpart in the reference.  It
  * calls no cudaMalloc or cudaFree: its scratch is a fixed array of about
- * 11.6 MB inside this library's device image, held by every GPU that loads
+ * 11.4 MB inside this library's device image, held by every GPU that loads
  * the library until the process exits.
  * Limits: n <= 32768 particles and a box of at most 131072 cells at cell size
  * h; larger calls return PBF_ERR_CAPACITY.  The first call on each device

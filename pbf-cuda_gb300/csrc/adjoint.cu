@@ -294,11 +294,6 @@ __device__ __forceinline__ float lane_sum(float v) {
   return v;
 }
 
-template <int L>
-__device__ __forceinline__ Vec lane_sum(Vec v) {
-  return {lane_sum<L>(v.x), lane_sum<L>(v.y), lane_sum<L>(v.z)};
-}
-
 // phi(s) and phi'(s) / s of the spiky gradient F = phi r (|r| = s, q = s^2).
 __device__ __forceinline__ void spiky_parts(const StepConsts& c, float q, float& phi, float& k) {
   const float is = __frsqrt_rn(q), s = q * is;

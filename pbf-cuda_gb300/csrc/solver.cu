@@ -1544,7 +1544,7 @@ __global__ void PBF_SPARSE_BOUNDS k_sparse(PassArgs a) {
 // Bound by the L1 data path and instruction issue: a test reads 12 bytes per
 // lane whatever the lanes share (L1 returns 128 bytes a cycle), 800 cycles for
 // 32 particles when every thread tested for one.  1,048,576 particles at rest
-// density: lambda 226 -> 148 us, xsph 260 -> 205 us; one particle per thread
+// density: lambda 226 -> 146 us, xsph 260 -> 211 us; one particle per thread
 // with the same queue and packed arithmetic 169 and 215.  Eight blocks (64
 // registers) beat seven (no spills) and nine by 1 and 4% of the step.
 template <int kKind>
