@@ -60,16 +60,38 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 }
 
 // ---- exclusive scan of a uint32 array (reduce, scan partials, downsweep) -------
+//
+// Up to kScanSelf tiles the downsweep's blocks add up the partials before their
+// own (a few loads a thread, in L2) and k_scan_top is not launched: the three
+// launches took 10.4 us at 257 tiles (9 scans a step of 1,048,576 particles), the
+// two 6.4 (with four entries a load).  Bound by launches and latency at every size a step has.
+constexpr int kScanSelf = 4096;
+
+// The thread's kScanItems entries of a tile (in: 16-byte aligned), 0 past the end.
+__device__ __forceinline__ void load_items(const uint32_t* in, int base, int len, uint32_t (&v)[kScanItems]) {
+  static_assert(kScanItems % 4 == 0, "four entries a load");
+  if (base + kScanItems <= len) {
+#pragma unroll
+    for (int k = 0; k < kScanItems; k += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(in + base + k);
+      v[k] = q.x, v[k + 1] = q.y, v[k + 2] = q.z, v[k + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) v[k] = base + k < len ? in[base + k] : 0u;
+  }
+}
 
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_reduce(const uint32_t* __restrict__ in, int len, uint32_t* __restrict__ partials, const uint32_t* __restrict__ groups) {
   __shared__ uint32_t smem[kScanThreads / 32 + 1];
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   const bool apart = groups && *groups != 0u;
+  uint32_t v[kScanItems];
+  load_items(in, base, len, v);
   uint32_t sum = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k)
-    if (base + k < len) sum += groups ? pair_slots(in[base + k], apart) : in[base + k];
+  for (int k = 0; k < kScanItems; ++k) sum += groups ? pair_slots(v[k], apart) : v[k];
   uint32_t total;
   block_exclusive_scan<kScanThreads>(sum, smem, &total);
   if (threadIdx.x == 0) partials[blockIdx.x] = total;
@@ -98,26 +120,45 @@ k_scan_top(uint32_t* __restrict__ partials, int count) {
 
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_down(const uint32_t* in, int len, const uint32_t* __restrict__ partials, uint32_t* out,
-            const uint32_t* __restrict__ groups) {
+            const uint32_t* __restrict__ groups, int self) {
   // in and out may alias (in-place scan): every thread reads its items before
   // writing them, and no thread touches another thread's items.
   __shared__ uint32_t smem[kScanThreads / 32 + 1];
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   const bool apart = groups && *groups != 0u;
   uint32_t v[kScanItems];
-  uint32_t sum = 0;
+  load_items(in, base, len, v);
+  uint32_t before = 0, sum = 0;
+  if (self)
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += kScanThreads) before += partials[t];
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    v[k] = base + k < len ? in[base + k] : 0u;
     if (groups) v[k] = pair_slots(v[k], apart);
     sum += v[k];
   }
-  uint32_t total;
-  uint32_t run = block_exclusive_scan<kScanThreads>(sum, smem, &total) + partials[blockIdx.x];
+  uint32_t total, first;
+  if (self)
+    block_exclusive_scan<kScanThreads>(before, smem, &first);
+  else
+    first = partials[blockIdx.x];
+  uint32_t run = block_exclusive_scan<kScanThreads>(sum, smem, &total) + first;
+  if (base + kScanItems <= len) {
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    if (base + k < len) out[base + k] = run;
-    run += v[k];
+    for (int k = 0; k < kScanItems; k += 4) {
+      uint4 q;
+      q.x = run;
+      q.y = q.x + v[k];
+      q.z = q.y + v[k + 1];
+      q.w = q.z + v[k + 2];
+      run = q.w + v[k + 3];
+      *reinterpret_cast<uint4*>(out + base + k) = q;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      if (base + k < len) out[base + k] = run;
+      run += v[k];
+    }
   }
 }
 
@@ -197,8 +238,9 @@ cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t*
     return cudaGetLastError();
   }
   k_scan_reduce<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, groups);
-  k_scan_top<<<1, kTopThreads, 0, stream>>>(partials, tiles);
-  k_scan_down<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, out, groups);
+  const int self = tiles <= kScanSelf;
+  if (!self) k_scan_top<<<1, kTopThreads, 0, stream>>>(partials, tiles);
+  k_scan_down<<<tiles, kScanThreads, 0, stream>>>(in, len, partials, out, groups, self);
   return cudaGetLastError();
 }
 
@@ -419,7 +461,7 @@ int key_bits(int cells) {
 
 }  // namespace
 
-int scan_launches(int len) { return len <= kScanOne ? 1 : 3; }
+int scan_launches(int len) { return len <= kScanOne ? 1 : (len <= kScanSelf * kScanTile ? 2 : 3); }
 
 int grid_launches(const StepConsts& c, int n) {
   const int bits = key_bits(c.cells);

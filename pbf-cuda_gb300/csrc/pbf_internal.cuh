@@ -541,7 +541,7 @@ cudaError_t backward(const BackwardArgs& args, const BackwardTape& tape, const u
                      cudaStream_t stream);
 
 // Exclusive prefix of in[0, len) into out (may alias in): one launch for short
-// arrays or three (scan_launches); partials holds kMaxScanPartials entries.  groups: of pair_slots of the values,
+// arrays, else two or three (scan_launches); partials holds kMaxScanPartials entries.  groups: of pair_slots of the values,
 // apart where *groups (device) is not zero.
 cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t* partials, cudaStream_t stream,
                            const uint32_t* groups = nullptr);
