@@ -164,10 +164,10 @@ k_scan_down(const uint32_t* in, int len, const uint32_t* __restrict__ partials, 
 
 // The whole scan in one block, for arrays of up to kScanOne entries: each warp a
 // contiguous share, four entries a lane and round, every round's load in flight
-// before the first is used.  The three launches of the general scan cost 7 us at
-// 4,001 entries, this one 3.9; at 32,001 entries 8.5 and 6.2 (a thread's own
-// contiguous share instead, uncoalesced: 55).
-constexpr int kScanOneRounds = 8;
+// before the first is used.  At 4,001 entries this one takes 3.9 us, the two
+// launches of the general scan 2.5 each at least; beyond 8,192 entries those are as fast or faster
+// (a step with eight scans of 32,001 entries: 776 us, 785 with one block each).
+constexpr int kScanOneRounds = 2;
 constexpr int kScanOne = kTopThreads * 4 * kScanOneRounds;
 __global__ void __launch_bounds__(kTopThreads)
 k_scan_one(const uint32_t* in, int len, uint32_t* out, const uint32_t* __restrict__ groups) {

@@ -20,8 +20,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("box", [(0.3, 0.1, 0.3), (1.0, 1.0, 1.2), (3.2, 3.2, 1.6), (12.8, 6.4, 6.4)])
 def test_grid_edges(pbf, oracle, cuda, n, box):
     """Up to 8,192 particles sorted in one block by 1 to 3 digits of 7 bits; the
-    cell scan in one block up to 32,768 entries (the third box has 16,385, the
-    last 524,289)."""
+    cell scan in one block up to 8,192 entries (the second box has 1,201, the
+    third 16,385, the last 524,289)."""
     rng = np.random.default_rng(n)
     xs = np.zeros((n, 4), np.float32)
     xs[:, :3] = rng.uniform(-0.05, 1.05, size=(n, 3)) * np.array(box)
