@@ -355,8 +355,12 @@ __device__ __forceinline__ int list_hits(const BackwardArgs& a, const float4* __
   };
   if constexpr (L == 1) {
     // four candidates' loads in flight at a time, and room for four more entries
-    // looked at once for them (so that a list holds kHitCap - 3 at least)
+    // looked at once for them (so that a list holds kHitCap - 3 at least).  A full
+    // list ends the innermost loop only: a lane that leaves all three at once may
+    // reach the block's barriers after its warp was counted there (see solver.cu's
+    // window_flagged)
     const size_t step = hit_step<L>(a);
+    bool full = false;
     for (int dx = -1; dx <= 1; ++dx) {
       const int x = q.x + dx;
       if (x < 0 || x >= g.dims[0]) continue;
@@ -365,7 +369,7 @@ __device__ __forceinline__ int list_hits(const BackwardArgs& a, const float4* __
         if (y < 0 || y >= g.dims[1]) continue;
         int s, e;
         column_run(g, a.cs, a.n, x, y, q.z, s, e);
-        for (int j = s; j < e; j += 4) {
+        for (int j = s; j < e && !full; j += 4) {
           float4 xj[4];
           if (j + 4 <= a.n) {
 #pragma unroll
@@ -374,10 +378,10 @@ __device__ __forceinline__ int list_hits(const BackwardArgs& a, const float4* __
 #pragma unroll
             for (int u = 0; u < 4; ++u) xj[u] = ld4(X, min(j + u, a.n - 1));
           }
-          if (cnt > kHitCap - 4) return -1;
+          full = cnt > kHitCap - 4;
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            if (j + u < e && is_hit(xj[u])) {
+            if (!full && j + u < e && is_hit(xj[u])) {
               *list = (uint32_t)(j + u);
               list += step;
               ++cnt;
@@ -386,6 +390,7 @@ __device__ __forceinline__ int list_hits(const BackwardArgs& a, const float4* __
         }
       }
     }
+    if (full) cnt = kHitCap + 1;
   } else {
     // the lanes look up the nine columns side by side, and every column's first
     // L candidates are in flight before the first test

@@ -184,23 +184,26 @@ __device__ __forceinline__ int window_total(const SceneGeom& g, const uint32_t* 
   return total;
 }
 
-// Whether a cell of the window carries any of `bits`.
+// Whether a cell of the window carries any of `bits`.  No branch in it and none
+// around its loads: a cell outside the grid is read as the nearest one inside,
+// which the window holds as well.  The loops with early exits that stood here
+// let a warp's lanes leave one by one, and k_dense's barrier after them did not
+// wait for the last ones (a part sum or a run of the block's previous batch was
+// then read in place of this one's: 1 in 30 steps of 30,011 scattered particles).
 __device__ __forceinline__ bool window_flagged(const SceneGeom& g,
                                                const uint32_t* __restrict__ cell_flags, int3 q,
                                                uint32_t bits) {
-  const int zlo = max(q.z - 1, 0), zhi = min(q.z + 1, g.dims[2] - 1);
+  uint32_t any = 0u;
+#pragma unroll 1  // (nine loads in flight; all 27 cost the paired kernel registers)
   for (int dx = -1; dx <= 1; ++dx) {
-    const int x = q.x + dx;
-    if (x < 0 || x >= g.dims[0]) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = q.y + dy;
-      if (y < 0 || y >= g.dims[1]) continue;
-      const int base = g.cell_base + (x * g.dims[1] + y) * g.dims[2];
-      for (int z = zlo; z <= zhi; ++z)
-        if (cell_flags[base + z] & bits) return true;
+    const int x = min(max(q.x + dx, 0), g.dims[0] - 1);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int y = min(max(q.y + k / 3 - 1, 0), g.dims[1] - 1), z = min(max(q.z + k % 3 - 1, 0), g.dims[2] - 1);
+      any |= cell_flags[cell_index(g, x, y, z)];
     }
   }
-  return false;
+  return (any & bits) != 0u;
 }
 
 // ---- where a pass reads candidate positions ---------------------------------------------
@@ -899,16 +902,18 @@ template <> struct PassOf<kXsph> { using type = XsphPass; };
 // values or a flagged cell of its window could poison its sum.
 __device__ __forceinline__ bool exact_path(int kind, const PassArgs& a, const SceneGeom& g,
                                            int3 q, int i) {
+  // (the flags are the same for every lane; the rest is evaluated without branches)
   if (kind == kDeltaP || kind == kDeltaPFinal) {
     if (a.flags[kFlagLambdaNonFinite] == 0u) return false;
-    return !isfinite(a.lambda[i]) || window_flagged(g, a.cell_flags, q, kCellLambdaNonFinite);
+    const bool own = !isfinite(a.lambda[i]);
+    return own | window_flagged(g, a.cell_flags, q, kCellLambdaNonFinite);
   }
   if (kind == kXsph) {
     if (a.flags[kFlagXsphExact] == 0u) return false;
     const float ri = a.rho[i];
     const float4 vi = a.V[i];
-    return !(ri > 0.f && isfinite(ri)) || !isfinite(vi.x) || !isfinite(vi.y) || !isfinite(vi.z) ||
-           window_flagged(g, a.cell_flags, q, kCellRhoNotPositive | kCellVelNonFinite);
+    const bool own = !(ri > 0.f) | !isfinite(ri) | !isfinite(vi.x) | !isfinite(vi.y) | !isfinite(vi.z);
+    return own | window_flagged(g, a.cell_flags, q, kCellRhoNotPositive | kCellVelNonFinite);
   }
   return false;
 }
@@ -1721,16 +1726,20 @@ __device__ __forceinline__ void visit_part(const PassArgs& a, const uint2* runs,
   }
 }
 
-// The same hits from what the lambda pass saved; false if it did not fit.
+// Whether what the lambda pass saved is the part's hits (its first entry says so
+// where they did not fit).
+__device__ __forceinline__ bool saved_fits(const uint32_t* saved) {
+  const uint2 e = __ldg(reinterpret_cast<const uint2*>(saved));
+  return e.x != 0u || e.y == 0u;
+}
+
+// The same hits from what the lambda pass saved (saved_fits).
 template <int kKind, class P>
-__device__ __forceinline__ bool visit_saved(const PassArgs& a, P& p, QueueColumn q, const uint32_t* saved, int cap) {
+__device__ __forceinline__ void visit_saved(const PassArgs& a, P& p, QueueColumn q, const uint32_t* saved, int cap) {
   int n = 0, hits = 0;
   for (int k = 0; k < cap; ++k) {
     const uint2 e = __ldg(reinterpret_cast<const uint2*>(saved) + k);
-    if (e.x == 0u) {
-      if (e.y != 0u) return false;  // (only the first entry)
-      break;
-    }
+    if (e.x == 0u) break;
     if (n == kPartQueue) {
       visit_queued<kKind, false, kDenseThreads>(a, q, hits, p, nullptr);
       n = hits = 0;
@@ -1740,7 +1749,6 @@ __device__ __forceinline__ bool visit_saved(const PassArgs& a, P& p, QueueColumn
     hits += __popc(e.x);
   }
   visit_queued<kKind, false, kDenseThreads>(a, q, hits, p, nullptr);
-  return true;
 }
 
 // Steps of few particles are bound by the latency of a pass's chain of loads,
@@ -1842,8 +1850,8 @@ __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
     if (valid) {
       P p(a, g, xi, i, exact);
       const QueueColumn col{queue + (kStage ? 0 : threadIdx.x), nullptr};
-      if (kDp && fast && saves && visit_saved<kKind>(a, p, col, saved, words / 2)) {
-        // the lambda pass's hits
+      if (kDp && fast && saves && saved_fits(saved)) {  // the lambda pass's hits
+        visit_saved<kKind>(a, p, col, saved, words / 2);
       } else {
         int total = 0;
         if (flat) {
