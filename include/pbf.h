@@ -310,15 +310,21 @@ pbf_status pbf_batch_get_tuning(const pbf_batch* b, pbf_tuning* t);
  * Errors the solver's kernels recorded on the device since the last call.
  * Waits for the solver's work on `stream` (device, as for pbf_step), then
  * returns PBF_ERR_TIMEOUT if a bounded device-side wait gave up since -- a
- * block's copy of candidate positions into shared memory that did not
- * complete (that block then read global memory instead: the step's results
- * are unchanged), or a grid barrier of a small step that not every block
- * reached (that step's results are not valid) -- else PBF_OK, and clears the
- * record.  No
- * counterpart in the reference, which does not check kernel errors.
+ * grid barrier of a small step that not every block reached in time (the rest
+ * of that step then does nothing: its outputs are not valid, and pos, vel and
+ * iid may or may not be permuted; later steps are not affected), or a block's
+ * copy of candidate positions into shared memory that did not complete (that
+ * block then read global memory instead: the step's results are unchanged) --
+ * else PBF_OK, and clears the record.  No counterpart in the reference, which
+ * does not check kernel errors.
  */
 pbf_status pbf_check_device(pbf_solver* s, void* stream);
 pbf_status pbf_batch_check_device(pbf_batch* b, void* stream);
+/* Polls a grid barrier of the following steps makes before it gives up (0: the
+ * default, 2^21, about a second).  For tests of that path, and for callers that
+ * would rather lose a step than wait that long. */
+pbf_status pbf_set_wait_limit(pbf_solver* s, int polls);
+pbf_status pbf_batch_set_wait_limit(pbf_batch* b, int polls);
 
 /*
  * One step, same contract and results as pbf_step (bit for bit, with the
@@ -337,6 +343,8 @@ pbf_status pbf_batch_check_device(pbf_batch* b, void* stream);
 pbf_status pbf_step_noalloc(const pbf_params* params, const float ulim[3], const float llim[3],
                             void* pos, void* npos, void* vel, void* nvel, uint32_t* iid, int n,
                             void* stream);
+/* pbf_check_device for the steps of pbf_step_noalloc on the current device. */
+pbf_status pbf_noalloc_check_device(void* stream);
 
 #ifdef __cplusplus
 }

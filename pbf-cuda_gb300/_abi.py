@@ -58,7 +58,10 @@ EXPORTED = (
     "pbf_batch_get_tuning",
     "pbf_check_device",
     "pbf_batch_check_device",
+    "pbf_set_wait_limit",
+    "pbf_batch_set_wait_limit",
     "pbf_step_noalloc",
+    "pbf_noalloc_check_device",
 )
 
 # Every symbol include/pbf_ssf.h declares, in declaration order.
@@ -235,7 +238,10 @@ def _declare(L) -> None:
         "pbf_batch_get_tuning": (ctypes.c_int, [vp, P(PbfTuning)]),
         "pbf_check_device": (ctypes.c_int, [vp, vp]),
         "pbf_batch_check_device": (ctypes.c_int, [vp, vp]),
+        "pbf_set_wait_limit": (ctypes.c_int, [vp, ctypes.c_int]),
+        "pbf_batch_set_wait_limit": (ctypes.c_int, [vp, ctypes.c_int]),
         "pbf_step_noalloc": (ctypes.c_int, [P(PbfParams), f3, f3, vp, vp, vp, vp, vp, ctypes.c_int, vp]),
+        "pbf_noalloc_check_device": (ctypes.c_int, [vp]),
         "pbf_ssf_params_default": (None, [P(PbfSsfParams)]),
         "pbf_ssf_look_at": (ctypes.c_int, [P(PbfSsfParams), f3, f3, ctypes.c_float]),
         "pbf_ssf_create": (ctypes.c_int, [P(PbfSsfParams), P(vp)]),

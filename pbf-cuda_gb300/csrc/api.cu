@@ -155,6 +155,7 @@ struct pbf_solver {
   int tune_queue_dense;
   int tune_split;         // dense warps per item; 0: the default
   int tune_interleave;    // dense warps take interleaved chunks; -1: the default
+  int wait_polls;         // pbf_set_wait_limit; 0: the default
 };
 
 namespace {
@@ -189,11 +190,11 @@ pbf_status check_device_word(uint32_t* word, cudaStream_t stream, const char* wh
   if (bits == 0u) return PBF_OK;
   PBF_CUDA(cudaMemsetAsync(word, 0, sizeof(uint32_t), stream), what);
   PBF_CUDA(cudaStreamSynchronize(stream), what);
+  if (bits & pbf::kErrBarrierTimeout)
+    return fail(PBF_ERR_TIMEOUT, "%s: a block of a grid barrier did not arrive in time (the step is not complete)", what);
   if (bits & pbf::kErrStageTimeout)
     return fail(PBF_ERR_TIMEOUT, "%s: a shared-memory staging copy did not complete in time (the pass read "
                                  "global memory instead)", what);
-  if (bits & pbf::kErrBarrierTimeout)
-    return fail(PBF_ERR_TIMEOUT, "%s: a block of a grid barrier did not arrive in time (the step is not complete)", what);
   return fail(PBF_ERR_CUDA, "%s: device error bits 0x%x", what, bits);
 }
 
@@ -320,6 +321,7 @@ pbf::StepConsts make_consts(const pbf_params& p, const float ulim[3], const floa
   c.queue_dense = pbf::kDefaultQueueDense;
   c.dense_split = pbf::kDefaultDenseSplit;
   c.dense_interleave = pbf::kDefaultDenseInterleave;
+  c.wait_polls = pbf::kDefaultWaitPolls;
   return c;
 }
 
@@ -834,6 +836,7 @@ pbf_status pbf_step(pbf_solver* s, void* pos, void* npos, void* vel, void* nvel,
   if (s->tune_queue_dense > 0) P.c.queue_dense = s->tune_queue_dense;
   if (s->tune_split > 0) P.c.dense_split = s->tune_split;
   if (s->tune_interleave >= 0) P.c.dense_interleave = s->tune_interleave;
+  if (s->wait_polls > 0) P.c.wait_polls = s->wait_polls;
   P.G = pbf::Geometry{nullptr, nullptr};
   P.grid = &s->grid;
   P.sol = &s->sol;
@@ -1119,6 +1122,10 @@ pbf_status set_error(pbf_status s, const char* msg) { return fail(s, "%s", msg);
 
 pbf_status set_cuda_error(cudaError_t e, const char* what) { return cuda_fail(e, what); }
 
+pbf_status check_error_word(uint32_t* word, cudaStream_t stream, const char* what) {
+  return check_device_word(word, stream, what);
+}
+
 pbf_status validate_step_setup(const pbf_params* params, const float ulim[3], const float llim[3],
                                long long max_cells, StepConsts* out) {
   pbf_status st = check_params(params);
@@ -1178,6 +1185,7 @@ struct pbf_batch {
   int tune_queue_dense = 0;
   int tune_split = 0;
   int tune_interleave = -1;
+  int wait_polls = 0;  // pbf_batch_set_wait_limit; 0: the default
 };
 
 namespace {
@@ -1367,6 +1375,7 @@ pbf_status pbf_batch_step(pbf_batch* b, void* pos, void* npos, void* vel, void* 
   if (b->tune_queue_dense > 0) P.c.queue_dense = b->tune_queue_dense;
   if (b->tune_split > 0) P.c.dense_split = b->tune_split;
   if (b->tune_interleave >= 0) P.c.dense_interleave = b->tune_interleave;
+  if (b->wait_polls > 0) P.c.wait_polls = b->wait_polls;
   P.G = pbf::Geometry{b->d_geom, b->d_sid};
   P.grid = &b->grid;
   P.sol = &b->sol;
@@ -1713,6 +1722,20 @@ pbf_status pbf_check_device(pbf_solver* s, void* stream) {
 pbf_status pbf_batch_check_device(pbf_batch* b, void* stream) {
   if (!b) return fail(PBF_ERR_INVALID_ARG, "batch is NULL");
   return check_device_word(b->sol.flags + pbf::kErrorWord, (cudaStream_t)stream, "pbf_batch_check_device");
+}
+
+pbf_status pbf_set_wait_limit(pbf_solver* s, int polls) {
+  if (!s) return fail(PBF_ERR_INVALID_ARG, "solver is NULL");
+  if (polls < 0) return fail(PBF_ERR_INVALID_ARG, "polls must be >= 0 (got %d)", polls);
+  s->wait_polls = polls;
+  return PBF_OK;
+}
+
+pbf_status pbf_batch_set_wait_limit(pbf_batch* b, int polls) {
+  if (!b) return fail(PBF_ERR_INVALID_ARG, "batch is NULL");
+  if (polls < 0) return fail(PBF_ERR_INVALID_ARG, "polls must be >= 0 (got %d)", polls);
+  b->wait_polls = polls;
+  return PBF_OK;
 }
 
 pbf_status pbf_batch_autotune(pbf_batch* b, const void* pos, const void* vel, const uint32_t* iid, int steps,

@@ -246,12 +246,16 @@ cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int len, uint32_t*
 
 namespace {
 
-// Up to three arrays set to zero in one launch.
+// Up to three arrays set to zero in one launch, and the group tables after a
+// step that gave up.
 __global__ void __launch_bounds__(256) k_clear(ClearList c) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
     if (k < c.len[a]) c.words[a][k] = 0u;
+  if (c.dirty && *c.dirty)
+    for (int a = 0; a < 5; ++a)
+      for (size_t t = k; t < c.tables_len[a]; t += (size_t)gridDim.x * blockDim.x) c.tables[a][t] = 0u;
 }
 
 // ---- predict + hash ---------------------------------------------------------------

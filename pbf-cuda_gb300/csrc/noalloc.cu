@@ -41,6 +41,7 @@
 namespace pbf {
 pbf_status set_error(pbf_status s, const char* msg);
 pbf_status set_cuda_error(cudaError_t e, const char* what);
+pbf_status check_error_word(uint32_t* word, cudaStream_t stream, const char* what);
 pbf_status validate_step_setup(const pbf_params* params, const float ulim[3], const float llim[3],
                                long long max_cells, StepConsts* out);
 pbf_status validate_step_buffers(const void* pos, const void* npos, const void* vel, const void* nvel,
@@ -277,4 +278,11 @@ extern "C" pbf_status pbf_step_noalloc(const pbf_params* params, const float uli
       (e = pbf::launch_vorticity(c, G, (const float4*)npos, g.cell_start, n, s, (float4*)nvel, strm)) != cudaSuccess)
     return pbf::set_cuda_error(e, "pbf_step_noalloc: vorticity");
   return PBF_OK;
+}
+
+extern "C" pbf_status pbf_noalloc_check_device(void* stream) {
+  unsigned char* base = nullptr;
+  if (const pbf_status st = scratch_base(&base); st != PBF_OK) return st;
+  return pbf::check_error_word((uint32_t*)(base + kOffFlags) + pbf::kErrorWord, (cudaStream_t)stream,
+                               "pbf_noalloc_check_device");
 }

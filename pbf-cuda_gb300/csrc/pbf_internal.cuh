@@ -62,6 +62,7 @@ struct StepConsts {
   int queue_dense;         // hit-queue chunks per thread of the dense kernel (1: none)
   int dense_split;         // warps of the dense kernel sharing one item's windows: 1, 2, 4 or 8
   int dense_interleave;    // 1: those warps take every dense_split-th chunk; 0: contiguous parts
+  int wait_polls;          // polls of a grid barrier before it gives up
   SceneGeom geom;          // the box of a single-scene step
 };
 
@@ -193,10 +194,15 @@ constexpr int kSortTile = 2048;
 int sort_tiles(int n);
 size_t radix_counts_len(int max_particles);
 
-// Two arrays of words that a step starts from zero, cleared with the grid's own.
+// Two arrays of words that a step starts from zero, cleared with the grid's own,
+// and where *dirty (device; null: never) is not zero the group tables' words,
+// which the kernels of a step otherwise leave at zero themselves.
 struct ClearList {
   uint32_t* words[3];
   int len[3];
+  const uint32_t* dirty;
+  uint32_t* tables[5];
+  size_t tables_len[5];
 };
 
 // Hash (optionally predicting x* = x + dt (v + dt g) first), count cells,
@@ -365,13 +371,17 @@ enum StepFlag {
   kBucketIdentity = 15,      // 1: the current buckets are every particle, in order
   kBarrierCount = 16,        // grid_barrier
   kBarrierGen = 17,
-  kNumFlags = 18
+  kStepFailed = 18,          // 1: a grid barrier of this step gave up; the rest of the step does nothing
+  kNumFlags = 19
 };
 
-// One more word after the step flags, cleared only when the host reads it:
-// device-side errors (ErrorBit) recorded by any step since.
+// Two more words after the step flags.  The first is cleared only when the host
+// reads it: device-side errors (ErrorBit) recorded by any step since.  The second
+// says that a step which gave up left the group tables half written; the next
+// step's clear sets them back to zero (ClearList).
 constexpr int kErrorWord = kNumFlags;
-constexpr int kFlagWords = kNumFlags + 1;
+constexpr int kDirtyWord = kNumFlags + 1;
+constexpr int kFlagWords = kNumFlags + 2;
 enum ErrorBit : uint32_t {
   kErrStageTimeout = 1u,     // a shared-memory staging copy did not complete in time
   kErrBarrierTimeout = 2u,   // a block of a small step's grid barrier did not arrive in time
@@ -442,6 +452,8 @@ constexpr int kDefaultQueueSparse = 1;
 constexpr int kDefaultQueueDense = 1;
 constexpr int kDefaultDenseSplit = 8;
 constexpr int kDefaultDenseInterleave = 0;
+// Polls of a small step's grid barrier before it gives up (about a second).
+constexpr int kDefaultWaitPolls = 1 << 21;
 
 // Vorticity confinement after XSPH, on its output NV (positions X = npos):
 // omega_i = sum_j (u_j - u_i) x g_ij and eta_i = sum_j |omega_j| g_ij over

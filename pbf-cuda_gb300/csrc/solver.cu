@@ -1783,7 +1783,7 @@ __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
   }
   // the slots the sparse kernel listed, or all of them, 32 per item
   const int work = work_count(a);
-  const uint32_t listed = a.dense_all ? (uint32_t)work : a.flags[a.counter];
+  const uint32_t listed = a.flags[kStepFailed] ? 0u : (a.dense_all ? (uint32_t)work : a.flags[a.counter]);
   const uint32_t count = (listed + 31) / 32;
   // kSplit warps share an item (each walks one contiguous part of every
   // lane's window); the block runs kDenseWarps / kSplit items at a time.  The
@@ -1907,6 +1907,7 @@ k_reorder(const uint32_t* __restrict__ perm, const float4* __restrict__ pos,
           int* __restrict__ grp_off, int* __restrict__ grp_item_off, int* __restrict__ grp_item_slot, int chunk) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
+  if (k == 0) flags[kDirtyWord] = 0u;  // the grid's clear has seen to it
   const uint32_t key = skeys[k];
   const uint32_t pop = cs[key + 1] - cs[key];
   if ((uint32_t)k == cs[key] && pop >= (uint32_t)kGroupCell) {
@@ -2589,12 +2590,16 @@ WorkArgs work_args(const SolverScratch& s, int n) {
 // phases and every list bucketed).
 
 constexpr int kMovedShare = 8;
-constexpr int kBarrierSpins = 1 << 21;
 
 // Every block of the (cooperative) grid arrives before any goes on; writes
-// before it are visible after it.  Bounded: a block that waited kBarrierSpins
-// polls records kErrBarrierTimeout and returns false (its caller returns).
-__device__ __forceinline__ bool grid_barrier(uint32_t* flags) {
+// before it are visible after it.  Bounded: a block that has polled `polls`
+// times, or finds that another one gave up, records kErrBarrierTimeout and
+// returns false (its caller returns).  A block goes past a barrier only when
+// every block has reached it, so what it reads there is complete; the block that
+// gave up is missing at the next one, where the others give up too.  The step's
+// later kernels then do nothing (kStepFailed): they read lists that were not
+// finished, and would count this kernel's arrivals as theirs.
+__device__ __forceinline__ bool grid_barrier(uint32_t* flags, int polls) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -2607,12 +2612,12 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* flags) {
       __threadfence();
       atomicAdd(&flags[kBarrierGen], 1u);
     } else {
-      int k = 0;
-      while (*gen == g && ++k < kBarrierSpins) {
-      }
-      if (k >= kBarrierSpins) {
-        ok = 0;
+      volatile uint32_t* failed = &flags[kStepFailed];
+      for (int k = 1; ok && *gen == g; ++k) ok = k < polls && ((k & 63) != 0 || *failed == 0u);
+      if (!ok) {
         atomicOr(&flags[kErrorWord], (uint32_t)kErrBarrierTimeout);
+        *failed = 1u;
+        flags[kDirtyWord] = 1u;
       }
     }
     __threadfence();
@@ -2636,6 +2641,11 @@ struct SmallArgs {
   int buckets;       // current-cell order is on
 };
 
+// Whether an earlier kernel of the step gave up (one answer for the block).
+__device__ __forceinline__ bool step_failed(const uint32_t* flags) {
+  return __syncthreads_or(*(volatile const uint32_t*)&flags[kStepFailed] != 0u) != 0;
+}
+
 // kLast: the delta_p pass whose followers come first (kDeltaPFinal: xsph follows).
 template <int kLast>
 __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
@@ -2646,6 +2656,8 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
   const bool groups = a.groups && flags[kGroupCount] != 0u;
   const uint32_t moved = a.buckets && a.iteration > 0 ? flags[kMoved0 + ((a.iteration + 1) & 1)] : 0u;
   const bool buckets = a.buckets && moved > (uint32_t)n / kMovedShare;  // uniform over the grid
+  const int polls = a.p.c.wait_polls;
+  if ((groups || buckets) && step_failed(flags)) return;
   const int cells1 = a.p.c.cells + 1;
   if (buckets)
     for (int k = i; k < cells1; k += gridDim.x * kWorkThreads) a.bcnt[k] = 0u;
@@ -2653,20 +2665,20 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
   if (groups) {
     if (a.iteration > 0) {
       follow_group<kLast>(a.p, a.w.follow, i);
-      if (!grid_barrier(flags)) return;
+      if (!grid_barrier(flags, polls)) return;
     }
     if constexpr (kXsphNext) {
       group_insert<kGroupsXsph>(a.g);
-      if (!grid_barrier(flags)) return;
+      if (!grid_barrier(flags, polls)) return;
       group_devmax<kGroupsXsph>(a.g);
-      if (!grid_barrier(flags)) return;
+      if (!grid_barrier(flags, polls)) return;
       group_devsum<kGroupsXsph>(a.g);
     } else {
       group_insert<kGroupsPos>(a.g);
-      if (!grid_barrier(flags)) return;
+      if (!grid_barrier(flags, polls)) return;
       computes = work_mark(a.w);
       if (!buckets) {
-        if (!grid_barrier(flags)) return;
+        if (!grid_barrier(flags, polls)) return;
         work_list(a.w);
       }
     }
@@ -2675,7 +2687,7 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
       flags[kWorkCount] = (uint32_t)n;
       flags[kWorkIdentity] = 1u;
     }
-    if (buckets && !grid_barrier(flags)) return;
+    if (buckets && !grid_barrier(flags, polls)) return;
   }
   if (!a.buckets) return;
   const bool listed = groups && !kXsphNext;
@@ -2689,7 +2701,7 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
   if (!buckets) return;
   // count, exclusive scan over the cells (every block a share), scatter
   if (computes) bucket_count(a.p, i, i, a.bcnt, a.bent);
-  if (!grid_barrier(flags)) return;
+  if (!grid_barrier(flags, polls)) return;
   __shared__ int sh[80];
   const int per_block = (cells1 + (int)gridDim.x - 1) / (int)gridDim.x;
   const int per_thread = (per_block + kWorkThreads - 1) / kWorkThreads;
@@ -2701,7 +2713,7 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
   int total;
   int run = block_scan_value(sum, sh, total);
   if (threadIdx.x == 0) a.bpart[blockIdx.x] = (uint32_t)total;
-  if (!grid_barrier(flags)) return;
+  if (!grid_barrier(flags, polls)) return;
   int before;  // the sum of the blocks before this one
   block_scan_value(threadIdx.x < blockIdx.x ? (int)a.bpart[threadIdx.x] : 0, sh, before);
   run += before;
@@ -2709,7 +2721,7 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
     a.bstart[k] = (uint32_t)run;
     run += (int)a.bcnt[k];
   }
-  if (!grid_barrier(flags)) return;
+  if (!grid_barrier(flags, polls)) return;
   if (listed && i == 0) flags[kBucketCount] = flags[kWorkCount];
   if (computes) {
     const uint2 e = a.bent[i];
@@ -2718,11 +2730,12 @@ __global__ void __launch_bounds__(kWorkThreads, 1) k_small_before(SmallArgs a) {
 }
 
 __global__ void __launch_bounds__(kWorkThreads, 1) k_small_between(SmallArgs a) {
-  if (a.p.flags[kGroupCount] == 0u) return;
+  const int polls = a.p.c.wait_polls;
+  if (a.p.flags[kGroupCount] == 0u || step_failed(a.p.flags)) return;
   follow_group<kLambda>(a.p, a.w.follow, blockIdx.x * kWorkThreads + threadIdx.x);
-  if (!grid_barrier(a.p.flags)) return;
+  if (!grid_barrier(a.p.flags, polls)) return;
   group_devmax<kGroupsLambda>(a.g);
-  if (!grid_barrier(a.p.flags)) return;
+  if (!grid_barrier(a.p.flags, polls)) return;
   group_devsum<kGroupsLambda>(a.g);
 }
 
@@ -2926,7 +2939,14 @@ cudaError_t set_pass_kernel_attributes() {
 }
 
 ClearList step_clears(const StepConsts& c, const SolverScratch& s) {
-  return ClearList{{s.cell_flags, s.flags, nullptr}, {c.cells + 1, kNumFlags, 0}};
+  // (the group tables as alloc_groups leaves them)
+  const size_t np = (size_t)s.grp_pool, slots = group_slots(s.grp_pool);
+  return ClearList{{s.cell_flags, s.flags, nullptr},
+                   {c.cells + 1, kNumFlags, 0},
+                   s.flags + kDirtyWord,
+                   {(uint32_t*)s.grp_hash, (uint32_t*)s.grp_max, (uint32_t*)s.grp_acc, (uint32_t*)s.grp_list_n,
+                    (uint32_t*)s.grp_done},
+                   {8 * np, np, 6 * np, slots, slots}};
 }
 
 cudaError_t reorder(const StepConsts& c, const uint32_t* perm, const float4* pos, const float4* vel,

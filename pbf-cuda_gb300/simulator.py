@@ -190,6 +190,11 @@ class Simulator:
         steps since the last check gave up (pbf_check_device)."""
         check(self._L.pbf_check_device(self._h, _stream_handle(stream)), "pbf_check_device")
 
+    def set_wait_limit(self, polls: int = 0) -> None:
+        """Polls a grid barrier of the following steps makes before it gives up
+        (pbf_set_wait_limit); 0: the default."""
+        check(self._L.pbf_set_wait_limit(self._h, int(polls)), "pbf_set_wait_limit")
+
     def autotune(self, pos: torch.Tensor, vel: torch.Tensor, iid: torch.Tensor, nparticle: Optional[int] = None,
                  steps: int = 3, stream=None) -> dict:
         """Time the dense-kernel choices on copies of this state (pbf_autotune)
@@ -331,6 +336,10 @@ class Ensemble:
         """Raise PbfError (PBF_ERR_TIMEOUT) if a bounded device-side wait of the
         steps since the last check gave up (pbf_batch_check_device)."""
         check(self._L.pbf_batch_check_device(self._h, _stream_handle(stream)), "pbf_batch_check_device")
+
+    def set_wait_limit(self, polls: int = 0) -> None:
+        """pbf_batch_set_wait_limit."""
+        check(self._L.pbf_batch_set_wait_limit(self._h, int(polls)), "pbf_batch_set_wait_limit")
 
     def density(self, stream=None) -> torch.Tensor:
         out = torch.empty(max(self.n, 1), dtype=torch.float32, device="cuda")
