@@ -8,6 +8,8 @@
 //   updateVelocity           -> fused into the last delta_p pass
 //   correctVelocity (XSPH)   -> solver.cu xsph
 // All of it is enqueued on the caller's stream without host synchronisation.
+#include <cuda.h>  // types of the driver calls that are resolved at run time
+
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -106,7 +108,7 @@ struct pbf_solver {
   int max_particles;
   int max_cells;
   int device;
-  int num_sms;
+  int num_sms;  // of cap_stream's context
   int last_n;  // particles of the last completed step (for pbf_get_density)
   pbf::GridScratch grid;
   pbf::SolverScratch sol;
@@ -325,14 +327,39 @@ pbf::StepConsts make_consts(const pbf_params& p, const float ulim[3], const floa
   return c;
 }
 
-// Streaming multiprocessors of the current device (1 if it cannot be queried).
-int current_sms() {
+// A driver entry point, found through the runtime (no link against the driver
+// library); null where there is none.
+void* driver_entry(const char* name, unsigned version) {
+  void* f = nullptr;
+  cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+  if (cudaGetDriverEntryPointByVersion(name, &f, version, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return f;
+}
+
+// Streaming multiprocessors that work on `stream` may use: the current device's,
+// or the share of them that the stream's green context holds (1 if they cannot
+// be queried).  Sizes the grids, and decides whether a small step's cooperative
+// launches fit (is_small).
+int stream_sms(cudaStream_t stream) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
+  using GetCtx = CUresult (*)(CUstream, CUcontext*);
+  using GetResource = CUresult (*)(CUcontext, CUdevResource*, CUdevResourceType);
+  static const GetCtx get_ctx = (GetCtx)driver_entry("cuStreamGetCtx", 12000);
+  static const GetResource get_resource = (GetResource)driver_entry("cuCtxGetDevResource", 12040);
+  CUcontext ctx = nullptr;
+  CUdevResource r;
+  if (get_ctx && get_resource && get_ctx((CUstream)stream, &ctx) == CUDA_SUCCESS && ctx &&
+      get_resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS && r.sm.smCount > 0 && (int)r.sm.smCount < sms)
+    sms = (int)r.sm.smCount;
   return sms;
 }
 
@@ -569,9 +596,9 @@ pbf_status pbf_create(const pbf_params* params, const float ulim[3], const float
   if (e == cudaSuccess) e = alloc(&s->sol.cell_flags, nc);
   if (e == cudaSuccess) e = alloc_groups(s->sol, max_particles);
   if (e == cudaSuccess) e = alloc_buckets(s->sol, np, nc);
-  if (e == cudaSuccess) s->num_sms = current_sms();
   if (e == cudaSuccess) e = pbf::set_pass_kernel_attributes();
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) s->num_sms = stream_sms(s->cap_stream);
   s->use_graph = true;
   if (e != cudaSuccess) {
     free_all(s);
@@ -828,7 +855,8 @@ pbf_status pbf_step(pbf_solver* s, void* pos, void* npos, void* vel, void* nvel,
   const bool prof = s->profile;
   s->prof_iters = 0;
   StepPlan P;
-  P.c = make_consts(s->params, s->ulim, s->llim, dims, s->num_sms);
+  // (a graph's kernels run in the context it was captured in)
+  P.c = make_consts(s->params, s->ulim, s->llim, dims, s->use_graph ? s->num_sms : stream_sms(st_));
   if (s->tune_window > 0) P.c.dense_window = s->tune_window;
   P.c.dense_all = s->tune_all;
   if (s->tune_order >= 0) P.c.order = s->tune_order;
@@ -1127,7 +1155,7 @@ pbf_status check_error_word(uint32_t* word, cudaStream_t stream, const char* wha
 }
 
 pbf_status validate_step_setup(const pbf_params* params, const float ulim[3], const float llim[3],
-                               long long max_cells, StepConsts* out) {
+                               long long max_cells, cudaStream_t stream, StepConsts* out) {
   pbf_status st = check_params(params);
   if (st != PBF_OK) return st;
   if (!ulim || !llim) return fail(PBF_ERR_INVALID_ARG, "limits are NULL");
@@ -1136,7 +1164,7 @@ pbf_status validate_step_setup(const pbf_params* params, const float ulim[3], co
   if ((st = grid_dims(ulim, llim, params->h, dims, &cells)) != PBF_OK) return st;
   if (cells > max_cells)
     return fail(PBF_ERR_CAPACITY, "box needs %lld cells, the limit is %lld", cells, max_cells);
-  *out = make_consts(*params, ulim, llim, dims, current_sms());
+  *out = make_consts(*params, ulim, llim, dims, stream_sms(stream));
   return PBF_OK;
 }
 
@@ -1306,7 +1334,7 @@ pbf_status pbf_batch_create(const pbf_params* params, int nscenes, const float* 
     cudaGetLastError();
     return cuda_fail(e, "pbf_batch_create");
   }
-  b->num_sms = current_sms();
+  b->num_sms = stream_sms(b->cap_stream);
   b->use_graph = true;
   *out = b;
   return PBF_OK;
@@ -1366,7 +1394,7 @@ pbf_status pbf_batch_step(pbf_batch* b, void* pos, void* npos, void* vel, void* 
   }
   StepPlan P;
   int unit_dims[3] = {1, 1, 1};
-  P.c = make_consts(b->params, &b->ulim[0], &b->llim[0], unit_dims, b->num_sms);
+  P.c = make_consts(b->params, &b->ulim[0], &b->llim[0], unit_dims, b->use_graph ? b->num_sms : stream_sms(st_));
   P.c.cells = (int)cells;
   if (b->tune_window > 0) P.c.dense_window = b->tune_window;
   P.c.dense_all = b->tune_all;

@@ -43,7 +43,7 @@ pbf_status set_error(pbf_status s, const char* msg);
 pbf_status set_cuda_error(cudaError_t e, const char* what);
 pbf_status check_error_word(uint32_t* word, cudaStream_t stream, const char* what);
 pbf_status validate_step_setup(const pbf_params* params, const float ulim[3], const float llim[3],
-                               long long max_cells, StepConsts* out);
+                               long long max_cells, cudaStream_t stream, StepConsts* out);
 pbf_status validate_step_buffers(const void* pos, const void* npos, const void* vel, const void* nvel,
                                  const void* iid);
 }  // namespace pbf
@@ -177,7 +177,7 @@ extern "C" pbf_status pbf_step_noalloc(const pbf_params* params, const float uli
     return pbf::set_error(PBF_ERR_CAPACITY,
                           "pbf_step_noalloc: n exceeds the fixed scratch limit of 32768 particles");
   pbf::StepConsts c;
-  pbf_status st = pbf::validate_step_setup(params, ulim, llim, kNoAllocMaxCells, &c);
+  pbf_status st = pbf::validate_step_setup(params, ulim, llim, kNoAllocMaxCells, (cudaStream_t)stream, &c);
   if (st != PBF_OK) return st;
   if (n == 0) return PBF_OK;
   if ((st = pbf::validate_step_buffers(pos, npos, vel, nvel, iid)) != PBF_OK) return st;
