@@ -445,6 +445,18 @@ cudaError_t alloc_buckets(pbf::SolverScratch& sol, size_t np, size_t nc) {
   return e;
 }
 
+// The reverse pass's scratch (not the tape's records).
+void free_reverse(pbf_solver* s) {
+  for (void* p : {(void*)s->bw4, (void*)s->bw1, (void*)s->bw8, (void*)s->wall_part, (void*)s->bw_sc, (void*)s->bw_hits})
+    if (p) cudaFree(p);
+  s->bw4 = nullptr;
+  s->bw1 = nullptr;
+  s->bw8 = nullptr;
+  s->wall_part = nullptr;
+  s->bw_sc = nullptr;
+  s->bw_hits = nullptr;
+}
+
 void free_all(pbf_solver* s) {
   void* ptrs[] = {s->grid.keys_a, s->grid.keys_b, s->grid.vals_a, s->grid.vals_b,
                   s->grid.cell_count, s->grid.cell_start, s->grid.radix_counts,
@@ -467,9 +479,8 @@ void free_all(pbf_solver* s) {
   s->cache.clear();
   s->bw_cache.clear();
   if (s->cap_stream) cudaStreamDestroy(s->cap_stream);
-  void* tape[] = {s->tape_mem, s->bw4, s->bw1, s->bw8, s->wall_part, s->bw_sc, s->bw_hits};
-  for (void* p : tape)
-    if (p) cudaFree(p);
+  if (s->tape_mem) cudaFree(s->tape_mem);
+  free_reverse(s);
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
@@ -934,7 +945,8 @@ pbf_status pbf_tape_enable(pbf_solver* s, int depth) {
     // the exact-scatter scratch starts (and is left by every fold) at zero
     if (e == cudaSuccess) e = alloc(&s->bw_sc, pbf::scatter_bytes(np));
     if (e == cudaSuccess) e = cudaMemset(s->bw_sc, 0, pbf::scatter_bytes(np));
-    if (e != cudaSuccess) {
+    if (e != cudaSuccess) {  // all of it or none: the next call starts over
+      free_reverse(s);
       cudaGetLastError();
       return cuda_fail(e, "pbf_tape_enable");
     }
