@@ -344,6 +344,7 @@ __device__ __forceinline__ unsigned group_mask() {
 template <int L>
 __device__ __forceinline__ int list_hits(const BackwardArgs& a, const float4* __restrict__ X, float4 xi, int i,
                                          int lane) {
+  if (!a.hits) return -1;
   const StepConsts& c = a.c;
   const SceneGeom g = geom_of(c, a.G, i);
   const int3 q = cell_of(c, g, xi);

@@ -421,18 +421,27 @@ cudaError_t alloc_groups(pbf::SolverScratch& sol, int max_particles) {
   return e;
 }
 
-// Positions with lambda, component copies and hit lists of the passes.
+// Positions with lambda, component copies and the hit lists' lengths.
 cudaError_t alloc_pass_lists(pbf::SolverScratch& sol, int max_particles) {
   const size_t stride = (size_t)pbf::particle_stride(max_particles);
   sol.stride = (int)stride;
   cudaError_t e = alloc(&sol.xl, (size_t)max_particles);
   if (e == cudaSuccess) e = alloc(&sol.sa, 3 * stride);
   if (e == cudaSuccess) e = alloc(&sol.sb, 3 * stride);
-  const size_t slots = pbf::list_slots(max_particles);
-  sol.hit_stride = (int)slots;
-  if (e == cudaSuccess) e = alloc(&sol.hits, (size_t)pbf::kHitCap * slots);
-  if (e == cudaSuccess) e = alloc(&sol.hit_n, slots);
+  if (e == cudaSuccess) e = alloc(&sol.hit_n, pbf::list_slots(max_particles));
   return e;
+}
+
+// The hit lists, over half of a solver's scratch and the last of it: a device
+// without room for them does without (the delta_p passes then walk the windows
+// again, with the same results).
+void alloc_hit_lists(pbf::SolverScratch& sol, int max_particles) {
+  const size_t slots = pbf::hit_slots(max_particles);
+  if (alloc(&sol.hits, (size_t)pbf::kHitCap * slots) != cudaSuccess) {
+    cudaGetLastError();
+    sol.hits = nullptr;
+  }
+  sol.hit_stride = sol.hits ? (int)slots : 0;
 }
 
 // Current-cell buckets (StepConsts::order) for up to np particles and nc - 1 cells.
@@ -610,6 +619,7 @@ pbf_status pbf_create(const pbf_params* params, const float ulim[3], const float
   if (e == cudaSuccess) e = pbf::set_pass_kernel_attributes();
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) s->num_sms = stream_sms(s->cap_stream);
+  if (e == cudaSuccess) alloc_hit_lists(s->sol, max_particles);
   s->use_graph = true;
   if (e != cudaSuccess) {
     free_all(s);
@@ -938,7 +948,6 @@ pbf_status pbf_tape_enable(pbf_solver* s, int depth) {
     const size_t blocks = (np * 32 + 127) / 128;  // the reverse kernels' blocks at 32 lanes per particle
     cudaError_t e = alloc(&s->bw4, np * 7);
     if (e == cudaSuccess) e = alloc(&s->bw1, np * 3);
-    if (e == cudaSuccess) e = alloc(&s->bw_hits, np * pbf::kHitCap);
     if (e == cudaSuccess) e = alloc(&s->bw8, np * 2);
     if (e == cudaSuccess) e = cudaMemset(s->bw4 + 5 * np, 0, sizeof(float4) * 2 * np);
     if (e == cudaSuccess) e = alloc(&s->wall_part, blocks * 6);
@@ -966,6 +975,12 @@ pbf_status pbf_tape_enable(pbf_solver* s, int depth) {
     }
     s->tape_iters = it;
     s->tape_cap = cap;
+  }
+  // the reverse pass's neighbour lists last: a device without room for them does
+  // without (its sums then walk the windows)
+  if (!s->bw_hits && alloc(&s->bw_hits, np * pbf::kHitCap) != cudaSuccess) {
+    cudaGetLastError();
+    s->bw_hits = nullptr;
   }
   s->tape_depth = depth;
   return PBF_OK;
@@ -1346,6 +1361,7 @@ pbf_status pbf_batch_create(const pbf_params* params, int nscenes, const float* 
     cudaGetLastError();
     return cuda_fail(e, "pbf_batch_create");
   }
+  alloc_hit_lists(b->sol, (int)np);
   b->num_sms = stream_sms(b->cap_stream);
   b->use_graph = true;
   *out = b;

@@ -237,8 +237,8 @@ struct SolverScratch {
   // [kHitCap][hit_stride] the lambda pass's hit lists, by thread slot, or the hit
   // masks of a step whose particles are all dense (null: none kept)
   uint32_t* hits;
-  int* hit_n;          // [hit_stride] their lengths, or a HitCode
-  int hit_stride;      // list_slots(max_particles)
+  int* hit_n;          // [list_slots(max_particles)] their lengths, or a HitCode
+  int hit_stride;      // hit_slots(max_particles), 0 without lists
   uint32_t* cell_flags;         // [max_cells + 1] CellFlag bits per cell, zero when a step starts (step_clears)
   const uint32_t* keys_sorted;  // the grid's sorted cell ids (set before the passes)
   const uint32_t* cell_start;   // the grid's cell prefix (set before the passes)
@@ -344,6 +344,12 @@ constexpr int particle_stride(int max_particles) { return (max_particles + 7) & 
 // 1.39).
 __host__ __device__ constexpr uint32_t pair_slots(uint32_t count, bool apart) {
   return apart ? 2u * count : (count + 1u) & ~1u;
+}
+// Particles with a hit list: paired buckets take a slot more for every cell with
+// an odd number of particles (6% more than particles at rest density).  Slots
+// beyond these have no list, and their particles walk the window in both passes.
+constexpr size_t hit_slots(int max_particles) {
+  return ((size_t)max_particles + (size_t)max_particles / 4 + 127) / 64 * 64;
 }
 // Slots of a pass's list; whole groups of a warp's pairs.
 constexpr size_t list_slots(int max_particles) { return (2 * (size_t)max_particles + 127) / 64 * 64; }
@@ -521,7 +527,7 @@ struct BackwardArgs {
   int sc_list;                // the list in use: 0 or 2 (its length's index in sc_ctr)
   int sc_cap;
   int sc_stride;
-  uint32_t* hits;   // the neighbours of every particle, kHitCap each, bit 31: not reciprocal
+  uint32_t* hits;   // the neighbours of every particle, kHitCap each, bit 31: not reciprocal (null: no lists)
   int* hit_n;       // their number, -1: more than kHitCap
   int hit_stride;   // particles the lists hold
   int lanes;        // lanes per particle below kWarpPerParticleBelow particles: 8, 16 or 32

@@ -103,7 +103,7 @@ struct PassArgs {
   int stride;             // of S
   uint32_t* hits;         // hit lists: lambda writes them, delta_p reads them
   int* hit_n;
-  int hit_stride;
+  int hit_stride;         // slots with a list
   uint32_t* cell_flags;   // CellFlag bits per cell
   const uint32_t* skeys;  // stale cell of each sorted slot
   float* lambda;          // lambda: out;  delta_p: in
@@ -1280,6 +1280,10 @@ __device__ __forceinline__ void for_chunks(uint2 run, F&& f) {
 // with more than fit its chunks (so that the delta_p pass's warps take one path).
 template <int kKind, bool kSecond, class P>
 __device__ __forceinline__ int finish_queued(const PassArgs& a, QueueColumn col, int n, int hits, P& p, int h) {
+  if (kKind == kLambda && h >= a.hit_stride) {  // no list (the same answer for the warp)
+    visit_queued<kKind, kSecond, kSparseThreads>(a, col, hits, p, nullptr);
+    return kHitsWalk;
+  }
   const bool list = kKind == kLambda && __all_sync(__activemask(), hits <= kHitCap);
   visit_queued<kKind, kSecond, kSparseThreads>(a, col, hits, p, list ? a.hits + h : nullptr);
   if (kKind != kLambda || list) return hits;
@@ -1312,14 +1316,14 @@ __device__ __forceinline__ int walk_hits(const PassArgs& a, QueueColumn col, P& 
         col.run[n * kSparseThreads] = make_uint2(m, (uint32_t)base);
         hits += __popc(m);
       } else {
-        if (kKind == kLambda && n < kHitCap / 2) put_chunk(a, h, n, m, (uint32_t)base);
+        if (kKind == kLambda && n < kHitCap / 2 && h < a.hit_stride) put_chunk(a, h, n, m, (uint32_t)base);
         visit_mask<kKind>(a, m, base, p);
       }
       ++n;
     });
   }
   if (fits) return finish_queued<kKind, false>(a, col, n, hits, p, h);
-  return kKind == kLambda && n <= kHitCap / 2 ? kHitsMasks - n : (int)kHitsWalk;
+  return kKind == kLambda && n <= kHitCap / 2 && h < a.hit_stride ? kHitsMasks - n : (int)kHitsWalk;
 }
 
 // The same walk for two particles of one cell, up to the queue: the masks of
@@ -1488,13 +1492,15 @@ __global__ void PBF_SPARSE_BOUNDS k_sparse(PassArgs a) {
   constexpr bool kDp = kKind == kDeltaP || kKind == kDeltaPFinal;
   __shared__ uint2 queue[kQueueSlots * kSparseThreads];
   const int count = work_count(a);
-  if ((int)(blockIdx.x * kSparseThreads) >= count) return;  // uniform over the block
+  const bool apart = a.paired && a.flags[kGroupCount] != 0u;  // pair_slots: a particle on every even slot
+  if ((int)(blockIdx.x * kSparseThreads << (apart ? 1 : 0)) >= count) return;  // uniform over the block
   const QueueColumn col{queue + threadIdx.x, nullptr};
   // h: the thread's hit list.  Paired, the lambda pass's warp w lists the first
   // particles of its 32 pairs at 64 w + lane and the second ones at 64 w + 32 +
-  // lane, so that its stores and these loads take consecutive words.
+  // lane, so that its stores and these loads take consecutive words; apart, pair
+  // h's particle at h.
   const int h = blockIdx.x * kSparseThreads + threadIdx.x;
-  const int t = a.paired ? (h & ~63) + 2 * (h & 31) + (h >> 5 & 1) : h;
+  const int t = apart ? 2 * h : (a.paired ? (h & ~63) + 2 * (h & 31) + (h >> 5 & 1) : h);
   const int i = t < count ? work_particle(a, t) : -1;
   const bool valid = i >= 0;
   const float4 xi = valid ? a.X[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1561,7 +1567,8 @@ __global__ void __launch_bounds__(kSparseThreads, 8) k_sparse_pair(PassArgs a) {
   if ((int)(2 * blockIdx.x * kSparseThreads) >= count) return;  // uniform over the block
   const QueueColumn col{queue + threadIdx.x, second + threadIdx.x};
   const int pair = blockIdx.x * kSparseThreads + threadIdx.x;
-  const int h = 2 * (pair & ~31) + (pair & 31);  // hit list of the first; the second's is h + 32
+  // hit list of the first; the second's is h + 32 (see k_sparse)
+  const int h = a.flags[kGroupCount] != 0u ? pair : 2 * (pair & ~31) + (pair & 31);
   const bool valid = 2 * pair < count;
   const int2 i = valid ? __ldg(reinterpret_cast<const int2*>(a.list) + pair) : make_int2(-1, -1);
   const bool two = i.y >= 0;
@@ -1581,7 +1588,10 @@ __global__ void __launch_bounds__(kSparseThreads, 8) k_sparse_pair(PassArgs a) {
   fits = __all_sync(kFull, fits || !valid || go_dense || grouped);
   if (!valid) return;
   if (go_dense) {
-    if (kKind == kLambda) a.hit_n[h] = a.hit_n[h + 32] = grouped ? kHitsWalk : kHitsDense;
+    if (kKind == kLambda) {
+      a.hit_n[h] = grouped ? kHitsWalk : kHitsDense;
+      if (two) a.hit_n[h + 32] = a.hit_n[h];
+    }
     return;
   }
   bool plain = true;  // xsph: k_xsph_poison looks for what poisons the sums (see there)
