@@ -650,6 +650,7 @@ struct pbf_ssf {
   int sky_size = 0;
   unsigned long long* frag_count = nullptr;
   const float* final_depth = nullptr;  // the image shading read in the last render
+  bool splat_clear = false;            // zkey and tfx hold their clear values
   int profile = 0;
   bool have_events = false;
   bool events_recorded = false;
@@ -794,6 +795,7 @@ pbf_status pbf_ssf_create(const pbf_ssf_params* p, pbf_ssf** out) {
     k_ssf_clear<<<(int)((npix + 255) / 256), 256>>>((int)npix, s->zkey, s->tfx);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    s->splat_clear = e == cudaSuccess;
   }
   for (int k = 0; e == cudaSuccess && k < 5; ++k) e = cudaEventCreate(&s->ev[k]);
   if (e == cudaSuccess) s->have_events = true;
@@ -883,8 +885,15 @@ pbf_status pbf_ssf_render(pbf_ssf* s, const void* pos, int n, void* color, void*
     e = cudaMemsetAsync(s->frag_count, 0, 8, st);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev[0], st);
   }
+  // a render whose launches failed half way left the splat's images as they were
+  if (e == cudaSuccess && !s->splat_clear) {
+    k_ssf_clear<<<(npix + 255) / 256, 256, 0, st>>>(npix, s->zkey, s->tfx);
+    ++launches;
+    e = cudaGetLastError();
+  }
   // 1-2. depth and thickness splats, resolved into depth_a / thick
   if (e == cudaSuccess) {
+    s->splat_clear = false;
     if (n > 0) {
       unsigned long long* frags = prof ? s->frag_count : nullptr;
       if (2.0 * c.r < 0.999)  // 2 r 2^32 < 2^32, with room for its rounding
@@ -896,6 +905,7 @@ pbf_status pbf_ssf_render(pbf_ssf* s, const void* pos, int n, void* color, void*
     k_ssf_resolve<<<(npix + 255) / 256, 256, 0, st>>>(npix, s->zkey, s->tfx, s->depth_a, s->thick);
     ++launches;
     e = cudaGetLastError();
+    s->splat_clear = e == cudaSuccess;
   }
   if (e == cudaSuccess && prof) e = cudaEventRecord(s->ev[1], st);
   // 3. smoothing: pass k reads a and writes b for odd k, the reverse for even k
