@@ -958,7 +958,8 @@ __device__ __forceinline__ bool reaches(const NodeBox& b, float4 x, float h2) {
 
 template <int kSplit>
 __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kGridThreads)
-k_density_grid(const float4* __restrict__ pos, int n, Lattice L, unsigned bricks, float* __restrict__ grid) {
+k_density_grid(const float4* __restrict__ pos, int n, Lattice L, unsigned bricks, unsigned batch,
+               float* __restrict__ grid) {
   namespace cg = cooperative_groups;
   __shared__ float4 keep[kGridBatch];
   __shared__ int counts[33];
@@ -977,18 +978,20 @@ k_density_grid(const float4* __restrict__ pos, int n, Lattice L, unsigned bricks
     const NodeBox warp_box = node_box(L, w0[0], w0[1], w0[2], 2, 4, 4);
     float d = 0.f;
     // unsigned: base passes 2^31 for the largest n
-    for (unsigned base = part * kGridBatch; base < (unsigned)n; base += kSplit * kGridBatch) {
+    for (unsigned base = part * batch; base < (unsigned)n; base += kSplit * batch) {
       float4 x[kGridUnroll];
-      unsigned ballot[kGridUnroll];
+      unsigned ballot[kGridUnroll], some = 0u;
+      const unsigned end = min(base + batch, (unsigned)n);
 #pragma unroll
-      for (int u = 0; u < kGridUnroll; ++u) x[u] = __ldg(pos + min(base + u * kGridThreads + threadIdx.x, (unsigned)n - 1u));
+      for (int u = 0; u < kGridUnroll; ++u) x[u] = __ldg(pos + min(base + u * kGridThreads + threadIdx.x, end - 1u));
 #pragma unroll
       for (int u = 0; u < kGridUnroll; ++u) {
-        const bool in = base + u * kGridThreads + threadIdx.x < (unsigned)n;
+        const bool in = base + u * kGridThreads + threadIdx.x < end;
         ballot[u] = __ballot_sync(0xffffffffu, in && reaches(brick_box, x[u], L.h2));
+        some |= ballot[u];
         if (lane == 0) counts[u * kGridWarps + warp] = __popc(ballot[u]);
       }
-      __syncthreads();
+      if (!__syncthreads_or(some != 0u)) continue;  // no survivor: nobody reads counts
       if (warp == 0) {  // exclusive offsets of the batch's 32 (round, warp) groups
         const int v = counts[lane];
         int s = v;
@@ -1070,10 +1073,14 @@ cudaError_t density_grid(const float4* pos, int n, const float lo[3], const floa
   const long long bricks = ((long long)dims[0] + kBrickX - 1) / kBrickX * (((long long)dims[1] + kBrickY - 1) / kBrickY) *
                            (((long long)dims[2] + kBrickZ - 1) / kBrickZ);
   const unsigned resident = (unsigned)min(bricks, (long long)kGridMaxBricks);
+  // few particles: shorter batches, so that every block of a cluster has one (1,000
+  // particles on 8^3 nodes: 41 us with whole batches)
+  const unsigned batch = min((unsigned)kGridBatch, max(32u, ((unsigned)n / kGridSplit + 31u) / 32u * 32u));
   if (bricks <= kGridSplitBelow)
-    k_density_grid<kGridSplit><<<resident * kGridSplit, kGridThreads, 0, stream>>>(pos, n, L, (unsigned)bricks, grid);
+    k_density_grid<kGridSplit><<<resident * kGridSplit, kGridThreads, 0, stream>>>(pos, n, L, (unsigned)bricks, batch,
+                                                                                     grid);
   else
-    k_density_grid<1><<<resident, kGridThreads, 0, stream>>>(pos, n, L, (unsigned)bricks, grid);
+    k_density_grid<1><<<resident, kGridThreads, 0, stream>>>(pos, n, L, (unsigned)bricks, kGridBatch, grid);
   return cudaGetLastError();
 }
 
