@@ -918,7 +918,7 @@ pbf_status pbf_step(pbf_solver* s, void* pos, void* npos, void* vel, void* nvel,
   const int niter = s->params.niter;
   s->last_grid_launches = pbf::grid_launches(c, n);
   s->last_launches = s->last_grid_launches + 1 + pbf::pass_launches(c, n) * (2 * niter + 1) +
-                     (c.order && pbf::pass_launches(c, n) > 1 ? 2 : 0) +  // k_xsph_mark, k_xsph_poison
+                     pbf::poison_launches(c, n) +
                      pbf::group_launches(c, n, niter) + pbf::bucket_launches(c, n, niter) +
                      (c.vort_eps > 0.f ? pbf::kVorticityLaunches : 0);
   if (prof) s->prof_iters = niter < kMaxProfiledIters ? niter : kMaxProfiledIters;

@@ -474,6 +474,8 @@ constexpr int kVorticityLaunches = 2;
 // Kernel launches of one neighbour pass of n particles (sparse kernel unless
 // every warp goes dense, dense kernel).
 int pass_launches(const StepConsts& c, int n);
+// Launches an ordered step's XSPH pass adds for sums that far particles poison.
+int poison_launches(const StepConsts& c, int n);
 // Group-table, work-list and follower launches of one step of n particles at
 // niter iterations.
 int group_launches(const StepConsts& c, int n, int niter);

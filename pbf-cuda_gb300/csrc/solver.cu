@@ -76,6 +76,7 @@ constexpr int kDenseThreads = 32 * kDenseWarps;
 // (pbf_autotune).
 constexpr int kMaxFields = 6;                   // partial-sum fields of the largest pass
 constexpr unsigned kFull = 0xffffffffu;
+constexpr float kNormalMin = 1.17549435e-38f;  // the smallest normal float
 
 // Whether every particle takes the dense kernel.
 bool dense_for_all(const StepConsts& c, int n) { return c.dense_all >= 0 ? c.dense_all != 0 : n < kDenseAllBelow; }
@@ -1398,7 +1399,7 @@ __device__ __forceinline__ void visit_chunks(const PassArgs& a, const uint32_t* 
 // Whether walk_hits and the hit lists hold for a particle at xi: keps2 a normal
 // number (a pair below it has no gradient; rsqrt_normal), xi finite.
 __device__ __forceinline__ bool fast_hits(const PassArgs& a, float4 xi) {
-  return a.c.keps2 >= 1.17549435e-38f && isfinite(xi.x) && isfinite(xi.y) && isfinite(xi.z);
+  return a.c.keps2 >= kNormalMin && isfinite(xi.x) && isfinite(xi.y) && isfinite(xi.z);
 }
 
 // The 9 column runs of the window of cell q into the column; returns the
@@ -2869,13 +2870,19 @@ PassArgs base_args(const StepConsts& c, const Geometry& G, const float4* X, cons
   return a;
 }
 
+// Whether the sparse kernel takes two particles a thread where the passes take
+// the buckets: not with a kernel_eps that leaves it no packed walk (fast_hits),
+// where the two would be walked one after the other (kernel_eps 0, 262,144
+// particles: a step 922 us in pairs, 894 the other way).
+bool takes_pairs(const StepConsts& c) { return c.keps2 >= kNormalMin; }
+
 // The pass takes the buckets (the delta_p passes of an iteration those of its
 // lambda pass: the same positions).
 void use_buckets(PassArgs& a, const SolverScratch& s) {
   a.list = s.bucket;
   a.count_word = kBucketCount;
   a.identity_word = -1;
-  a.paired = !a.dense_all;
+  a.paired = !a.dense_all && takes_pairs(a.c);
 }
 
 // Makes the pass take its computing particles in current-cell order: buckets
@@ -2884,7 +2891,7 @@ cudaError_t bucket_by_cell(PassArgs& a, const SolverScratch& s, int n, cudaStrea
   cudaError_t e = cudaMemsetAsync(s.bcnt, 0, sizeof(uint32_t) * (a.c.cells + 1), stream);
   if (e != cudaSuccess) return e;
   const int blocks = (n + 255) / 256;
-  a.paired = !a.dense_all;
+  a.paired = !a.dense_all && takes_pairs(a.c);
   k_bucket_count<<<blocks, 256, 0, stream>>>(a, s.bcnt, s.bent);
   if ((e = exclusive_scan(s.bcnt, s.bstart, a.c.cells + 1, s.bpart, stream,
                           a.paired ? s.flags + kGroupCount : nullptr)) != cudaSuccess)
@@ -3183,6 +3190,11 @@ namespace pbf {
 
 int pass_launches(const StepConsts& c, int n) {
   return dense_for_all(c, n) ? 1 : 2;
+}
+
+// k_xsph_mark and k_xsph_poison.
+int poison_launches(const StepConsts& c, int n) {
+  return c.order && !dense_for_all(c, n) && takes_pairs(c) ? 2 : 0;
 }
 
 // launch_groups: 1 launch before each lambda pass, 2 before each delta_p pass, 3 before xsph;

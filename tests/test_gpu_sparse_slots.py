@@ -35,3 +35,27 @@ def test_orders_agree(pbf, cuda, spacing, piled):
             torch.cuda.synchronize()
         out.append([t.cpu().numpy().tobytes() for t in (st.pos, st.vel, st.iid)])
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("which", ["scene", "reference"])
+def test_orders_agree_without_kernel_eps(pbf, cuda, which):
+    """kernel_eps 0 leaves the sparse kernel no packed walk: one particle a thread
+    in either order, the exact rules (scattered particles) included."""
+    import torch
+
+    from test_gpu_small_steps import small_scene
+
+    rng = np.random.default_rng(11)
+    pos, vel, box = small_scene(pbf, 9001, False, rng)
+    p = pbf.scenes.scene_params() if which == "scene" else ref_params(pbf)
+    p.kernel_eps = 0.0
+    out = []
+    for order in (0, 1):
+        st = pbf.ParticleState(pos, vel)
+        with pbf.Simulator(p, box, (0.0, 0.0, 0.0), len(pos)) as sim:
+            sim.set_tuning(dense_all=0, order=order)
+            for _ in range(4):
+                st.step(sim)
+            torch.cuda.synchronize()
+        out.append([t.cpu().numpy().tobytes() for t in (st.pos, st.vel, st.iid)])
+    assert out[0] == out[1]
