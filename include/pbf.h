@@ -31,9 +31,13 @@ extern "C" {
 #define PBF_ABI_VERSION 4
 
 /* Largest max_particles of a solver, and largest total of a batch: 2^27.
- * The solver's per-particle tables are indexed with 32-bit integers, the
- * largest holding 16 words per particle.  At the limit a solver holds about
- * 37 GB of scratch (~272 B per particle) besides the caller's buffers. */
+ * The solver's per-particle tables are indexed with 32-bit integers (the hit
+ * lists with 64-bit ones), the largest of them holding 8 words per particle.  At
+ * the limit a solver holds about 80 GB of scratch (~592 B per particle, 320 of
+ * them hit lists, which a solver created on a device without room for them does
+ * without: ~272 B) besides the caller's buffers and ~20 B per reserved cell; the
+ * first pbf_tape_enable adds ~640 B per particle (256 of them lists, as above)
+ * and the tape's records. */
 #define PBF_MAX_PARTICLES 134217728
 
 typedef enum pbf_status {
@@ -249,12 +253,12 @@ pbf_status pbf_batch_use_graphs(pbf_batch* b, int on);
  * the windows of 32 particles), whether every particle does, the order in
  * which the passes take particles (the cell order of the grid, or the cell
  * each particle is in at that iteration), how many warps of the dense kernel
- * split a batch's windows, how many neighbour chunks its threads queue before
- * running their pair terms, and how many candidate positions a block of that
- * kernel may stage in shared memory (bulk asynchronous copies of the column
- * runs its particles' windows share, read there instead of through L1) -- by running `steps` steps per choice from copies of the
- * caller's state (pos, vel, iid: device, n entries; they are not modified),
- * and keeps the fastest for the solver's following steps.  The window and
+ * split a batch's windows, how many candidate positions a block of that kernel
+ * may stage in shared memory (bulk asynchronous copies of the column runs its
+ * particles' windows share, read there instead of through L1), and where it
+ * matters how many neighbour chunks its threads queue before running their pair
+ * terms -- by running `steps` steps per choice from copies of the caller's state
+ * (pos, vel, iid: device, n entries; they are not modified), and keeps the fastest for the solver's following steps.  The window and
  * dense choices change the order in which window sums are added, so results
  * differ by rounding only, and so does the dense split; the particle order,
  * the queues and the staging change nothing (each particle's sums are the
@@ -280,7 +284,9 @@ typedef struct pbf_tuning {
                          window */
   int queue_dense;    /* neighbour chunks of 32 candidates whose hits a thread of the dense
                          kernel queues before running their pair terms in one loop (1: each
-                         chunk's right away; at most 8) */
+                         chunk's right away; at most 8), in the walks that take them so: a
+                         step with grouped cells, interleaved or staged windows (the others
+                         queue by themselves) */
   int dense_split;    /* warps of the dense kernel that split one batch of 32 particles'
                          windows: 1, 2, 4 or 8 (a block of 8 warps takes 8 / dense_split
                          batches at a time) */

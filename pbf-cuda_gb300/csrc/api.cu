@@ -1527,19 +1527,21 @@ constexpr int kTuneStageDense[] = {0, 1536, 3072};
 // One configuration of the neighbour passes (the fields of pbf_tuning that
 // pbf_autotune times).
 struct TuneChoice {
-  int window, all, order, split, queue_sparse, queue_dense, stage_sparse, stage_dense, interleave;
+  int window, all, order, split, queue_dense, stage_dense, interleave;
   bool operator==(const TuneChoice& o) const {
     return window == o.window && all == o.all && order == o.order && split == o.split &&
-           queue_sparse == o.queue_sparse && queue_dense == o.queue_dense && stage_sparse == o.stage_sparse &&
-           stage_dense == o.stage_dense && interleave == o.interleave;
+           queue_dense == o.queue_dense && stage_dense == o.stage_dense && interleave == o.interleave;
   }
 };
 
 TuneChoice default_choice(int n) {
   return TuneChoice{pbf::kDefaultDenseWindow, n < pbf::kDenseAllBelow ? 1 : 0, 1, pbf::kDefaultDenseSplit,
-                    pbf::kDefaultQueueSparse, pbf::kDefaultQueueDense, pbf::kDefaultStageSparse,
-                    pbf::kDefaultStageDense, pbf::kDefaultDenseInterleave};
+                    pbf::kDefaultQueueDense, pbf::kDefaultStageDense, pbf::kDefaultDenseInterleave};
 }
+
+// pbf_tuning's stage_sparse and queue_sparse are checked, kept and reported, and
+// have no effect.
+constexpr int kMaxQueueSparse = 16, kDefaultQueueSparse = 1, kDefaultStageSparse = 0;
 
 // The tuning fields a solver or batch keeps (0 / -1: the defaults).
 struct TuneState {
@@ -1568,8 +1570,10 @@ void set_tune_state(T* h, const TuneState& t) {
 }
 
 TuneState state_of(const TuneChoice& c) {
-  return TuneState{c.window,       c.all,          c.order,        c.split,     c.queue_sparse,
-                   c.queue_dense,  c.stage_sparse, c.stage_dense,  c.interleave};
+  TuneState t;
+  t.window = c.window, t.all = c.all, t.order = c.order, t.split = c.split;
+  t.queue_dense = c.queue_dense, t.stage_dense = c.stage_dense, t.interleave = c.interleave;
+  return t;
 }
 
 // pbf_tuning fields of a tune state (defaults resolved).
@@ -1578,9 +1582,9 @@ void fill_tuning(const TuneState& t, pbf_tuning* out) {
   out->dense_all = t.all;
   out->order = t.order >= 0 ? t.order : 1;
   out->dense_split = t.split > 0 ? t.split : pbf::kDefaultDenseSplit;
-  out->queue_sparse = t.queue_sparse > 0 ? t.queue_sparse : pbf::kDefaultQueueSparse;
+  out->queue_sparse = t.queue_sparse > 0 ? t.queue_sparse : kDefaultQueueSparse;
   out->queue_dense = t.queue_dense > 0 ? t.queue_dense : pbf::kDefaultQueueDense;
-  out->stage_sparse = t.stage_sparse >= 0 ? t.stage_sparse : pbf::kDefaultStageSparse;
+  out->stage_sparse = t.stage_sparse >= 0 ? t.stage_sparse : kDefaultStageSparse;
   out->stage_dense = t.stage_dense >= 0 ? t.stage_dense : pbf::kDefaultStageDense;
   out->dense_interleave = t.interleave >= 0 ? t.interleave : pbf::kDefaultDenseInterleave;
 }
@@ -1588,11 +1592,13 @@ void fill_tuning(const TuneState& t, pbf_tuning* out) {
 // Runs `steps` steps per candidate on copies of (pos, vel, iid) through
 // step(choice, bufs...) and returns the fastest choice: first over the
 // window, dense and order choices with the other fields at their defaults,
-// then, from the best so far, one field at a time: the dense split, the
-// dense kernel's hit queue and its stage.
+// then, from the best so far, one field at a time: the dense split, its
+// interleaving, the dense kernel's stage, and its hit queue where the best choice
+// uses it (elsewhere the choice would be noise).  group_count (device): the
+// grouped cells of the last step.
 template <class Step>
 pbf_status autotune(int n, const void* pos, const void* vel, const uint32_t* iid, int steps, cudaStream_t st,
-                    Step step, pbf_tuning* out) {
+                    const uint32_t* group_count, Step step, pbf_tuning* out) {
   if (!pos || !vel || !iid || !out || n <= 0 || steps < 1)
     return fail(PBF_ERR_INVALID_ARG, "NULL argument, n <= 0 or steps < 1");
   float4 *p[2] = {nullptr, nullptr}, *v[2] = {nullptr, nullptr};
@@ -1661,8 +1667,13 @@ pbf_status autotune(int n, const void* pos, const void* vel, const uint32_t* iid
   };
   sweep(&TuneChoice::split, kTuneSplits, 4);
   if (best_ch.split > 1) sweep(&TuneChoice::interleave, kTuneInterleave, 2);
-  sweep(&TuneChoice::queue_dense, kTuneQueueDense, 3);
   sweep(&TuneChoice::stage_dense, kTuneStageDense, 3);
+  uint32_t groups = 0u;
+  if (e == cudaSuccess && result == PBF_OK) {
+    e = cudaMemcpyAsync(&groups, group_count, sizeof(groups), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  if (groups || best_ch.interleave || best_ch.stage_dense > 0) sweep(&TuneChoice::queue_dense, kTuneQueueDense, 3);
   for (void* q : {(void*)p[0], (void*)p[1], (void*)v[0], (void*)v[1], (void*)id})
     if (q) cudaFree(q);
   if (e0) cudaEventDestroy(e0);
@@ -1690,10 +1701,10 @@ pbf_status check_tuning(const pbf_tuning* t) {
       t->stage_dense > pbf::kStageMax)
     return fail(PBF_ERR_INVALID_ARG, "stage_sparse / stage_dense must be -1 to %d (got %d / %d)", pbf::kStageMax,
                 t->stage_sparse, t->stage_dense);
-  if (t->queue_sparse < 0 || t->queue_sparse > pbf::kMaxQueueSparse || t->queue_dense < 0 ||
+  if (t->queue_sparse < 0 || t->queue_sparse > kMaxQueueSparse || t->queue_dense < 0 ||
       t->queue_dense > pbf::kMaxQueueDense)
     return fail(PBF_ERR_INVALID_ARG, "queue_sparse must be 0 to %d and queue_dense 0 to %d (got %d / %d)",
-                pbf::kMaxQueueSparse, pbf::kMaxQueueDense, t->queue_sparse, t->queue_dense);
+                kMaxQueueSparse, pbf::kMaxQueueDense, t->queue_sparse, t->queue_dense);
   if (t->dense_split != 0 && t->dense_split != 1 && t->dense_split != 2 && t->dense_split != 4 &&
       t->dense_split != 8)
     return fail(PBF_ERR_INVALID_ARG, "dense_split must be 0, 1, 2, 4 or 8 (got %d)", t->dense_split);
@@ -1720,7 +1731,7 @@ pbf_status pbf_autotune(pbf_solver* s, const void* pos, const void* vel, const u
   s->tape_depth = 0;  // the trial steps are not taped
   const TuneState keep = tune_state(s);
   const pbf_status st = autotune(
-      n, pos, vel, iid, steps, (cudaStream_t)stream,
+      n, pos, vel, iid, steps, (cudaStream_t)stream, s->sol.flags + pbf::kGroupCount,
       [&](const TuneChoice& ch, float4* p, float4* np, float4* v, float4* nv, uint32_t* id, cudaStream_t strm) {
         set_tune_state(s, state_of(ch));
         return pbf_step(s, p, np, v, nv, id, n, strm);
@@ -1800,7 +1811,7 @@ pbf_status pbf_batch_autotune(pbf_batch* b, const void* pos, const void* vel, co
   if (!b) return fail(PBF_ERR_INVALID_ARG, "batch is NULL");
   const TuneState keep = tune_state(b);
   const pbf_status st = autotune(
-      b->n, pos, vel, iid, steps, (cudaStream_t)stream,
+      b->n, pos, vel, iid, steps, (cudaStream_t)stream, b->sol.flags + pbf::kGroupCount,
       [&](const TuneChoice& ch, float4* p, float4* np, float4* v, float4* nv, uint32_t* id, cudaStream_t strm) {
         set_tune_state(b, state_of(ch));
         return pbf_batch_step(b, p, np, v, nv, id, strm);

@@ -444,17 +444,13 @@ inline int group_chunk(const StepConsts& c, int n) {
 }
 constexpr int kDenseAllBelow = 131072;
 // Slots a block of the dense pass kernel stages in shared memory (0: no
-// staging; pbf_autotune can override, up to kStageMax).  The tuning's
-// stage_sparse and queue_sparse are kept and have no effect: the sparse kernel
-// reads through L1 and always queues.
-constexpr int kDefaultStageSparse = 0;
+// staging; pbf_autotune can override, up to kStageMax).
 constexpr int kDefaultStageDense = 0;
-// Hit-queue capacities (chunks per thread; 1: the pair body right after each
-// chunk) and the dense kernel's warps per item (defaults; pbf_autotune can
-// override, queues up to kMaxQueue* chunks).
-constexpr int kMaxQueueSparse = 16;
+// The dense kernel's hit-queue capacity (chunks per thread; 1: the pair body right
+// after each chunk) where it walks with grouped cells, interleaved, staged or on
+// the exact path, and its warps per item (defaults; pbf_autotune can override,
+// the queue up to kMaxQueueDense chunks).
 constexpr int kMaxQueueDense = 8;
-constexpr int kDefaultQueueSparse = 1;
 constexpr int kDefaultQueueDense = 1;
 constexpr int kDefaultDenseSplit = 8;
 constexpr int kDefaultDenseInterleave = 0;
