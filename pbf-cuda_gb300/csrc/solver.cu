@@ -1737,19 +1737,21 @@ __device__ __forceinline__ void visit_part(const PassArgs& a, const uint2* runs,
   }
 }
 
-// Whether what the lambda pass saved is the part's hits (its first entry says so
-// where they did not fit).
-__device__ __forceinline__ bool saved_fits(const uint32_t* saved) {
-  const uint2 e = __ldg(reinterpret_cast<const uint2*>(saved));
-  return e.x != 0u || e.y == 0u;
+// The first entry of what the lambda pass saved, and whether it says that the
+// part's hits are there (not where they did not fit).
+__device__ __forceinline__ uint2 saved_entry(const uint32_t* saved, int k) {
+  return __ldg(reinterpret_cast<const uint2*>(saved) + k);
 }
+__device__ __forceinline__ bool saved_fits(uint2 first) { return first.x != 0u || first.y == 0u; }
 
 // The same hits from what the lambda pass saved (saved_fits).
 template <int kKind, class P>
-__device__ __forceinline__ void visit_saved(const PassArgs& a, P& p, QueueColumn q, const uint32_t* saved, int cap) {
+__device__ __forceinline__ void visit_saved(const PassArgs& a, P& p, QueueColumn q, const uint32_t* saved, uint2 first,
+                                            int cap) {
   int n = 0, hits = 0;
+  uint2 e = first;
   for (int k = 0; k < cap; ++k) {
-    const uint2 e = __ldg(reinterpret_cast<const uint2*>(saved) + k);
+    if (k) e = saved_entry(saved, k);
     if (e.x == 0u) break;
     if (n == kPartQueue) {
       visit_queued<kKind, false, kDenseThreads>(a, q, hits, p, nullptr);
@@ -1861,8 +1863,10 @@ __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
     if (valid) {
       P p(a, g, xi, i, exact);
       const QueueColumn col{queue + (kStage ? 0 : threadIdx.x), nullptr};
-      if (kDp && fast && saves && saved_fits(saved)) {  // the lambda pass's hits
-        visit_saved<kKind>(a, p, col, saved, words / 2);
+      const bool look = kDp && fast && saves;
+      const uint2 entry = look ? saved_entry(saved, 0) : make_uint2(0u, ~0u);
+      if (look && saved_fits(entry)) {  // the lambda pass's hits
+        visit_saved<kKind>(a, p, col, saved, entry, words / 2);
       } else {
         int total = 0;
         if (flat) {
