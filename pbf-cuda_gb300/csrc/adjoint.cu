@@ -316,7 +316,7 @@ __device__ __forceinline__ void spiky_parts(const StepConsts& c, float q, float&
 // before (with one lane per particle, a warp each: a crowded scene of 262,144
 // particles 31.9 -> 26.0 ms).  Reverse pass of 262,144 particles at rest, 4
 // iterations: 2,906 -> 1,060 us; of 15,625 (32 lanes per particle): 559 -> 231.
-// Bounds: k_bwd_window (109 us of 262,144 particles) issues instructions (64% of
+// Bounds: k_bwd_window (107 us a pass of 262,144 particles) issues instructions (64% of
 // the slots: 85 million, three quarters of them tests and list entries), the
 // sums over the lists wait for their gathers (47% of the slots).
 
@@ -915,15 +915,16 @@ __device__ __forceinline__ float node_coord(const Lattice& L, int a, int k) {
 // brick and ~15 per survivor and warp, against ~10 per particle and NODE when
 // every node tested every particle (the earlier kernel).  A brick smaller than
 // 256 nodes would stream the particles through more blocks (L2 reads), a
-// larger one leaves its warps more survivors.  Measured on
-// GB300: 262,144 particles on 32^3 nodes 4,549 -> 190 us, 15,625 on 32 x 16 x 16
+// larger one leaves its warps more survivors.  The kernel's time on GB300:
+// 262,144 particles on 32^3 nodes 4,549 -> 127 us, 15,625 on 32 x 16 x 16
 // 275 -> 25 us.
 constexpr int kGridThreads = 256, kGridSplit = 8;
-// Up to one brick per SM a cluster shares it; with more bricks whole blocks
-// fill the chip and streaming the particles eight times costs more than it
-// gains (262,144 particles: 128 bricks 190 us split, 294 whole; 512 bricks
-// 440 split, 304 whole; 15,625 particles: 26 / 35 and 70 / 36).
-constexpr int kGridSplitBelow = 152;
+// A cluster shares a brick where there is at most one brick per SM; with more,
+// whole blocks fill the chip, and streaming the particles through eight times the
+// blocks costs more than it gains where they are few or spread over the lattice
+// (15,625 particles: 128 bricks 17 us split, 48 whole; 512 bricks 52 and 37;
+// 262,144 in an eighth of the lattice's box, whose bricks hold unequal work: 184
+// and 733, 226 and 412, 1,024 bricks 398 and 330).
 constexpr int kGridMaxBricks = 1 << 20;              // bricks in flight (the blocks loop over the rest)
 constexpr int kGridUnroll = 4;                       // particles in flight per thread
 constexpr int kGridBatch = kGridThreads * kGridUnroll;
@@ -1076,7 +1077,7 @@ cudaError_t density_grid(const float4* pos, int n, const float lo[3], const floa
   // few particles: shorter batches, so that every block of a cluster has one (1,000
   // particles on 8^3 nodes: 41 us with whole batches)
   const unsigned batch = min((unsigned)kGridBatch, max(32u, ((unsigned)n / kGridSplit + 31u) / 32u * 32u));
-  if (bricks <= kGridSplitBelow)
+  if (bricks <= device_sms())
     k_density_grid<kGridSplit><<<resident * kGridSplit, kGridThreads, 0, stream>>>(pos, n, L, (unsigned)bricks, batch,
                                                                                      grid);
   else

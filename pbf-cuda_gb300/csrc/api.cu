@@ -345,12 +345,7 @@ void* driver_entry(const char* name, unsigned version) {
 // be queried).  Sizes the grids, and decides whether a small step's cooperative
 // launches fit (is_small).
 int stream_sms(cudaStream_t stream) {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
+  int sms = pbf::device_sms();
   using GetCtx = CUresult (*)(CUstream, CUcontext*);
   using GetResource = CUresult (*)(CUcontext, CUdevResource*, CUdevResourceType);
   static const GetCtx get_ctx = (GetCtx)driver_entry("cuStreamGetCtx", 12000);
@@ -1172,6 +1167,16 @@ pbf_status pbf_build_grid(pbf_solver* s, const void* xstar, int n, uint32_t* key
 // ---- helpers for other translation units of the library ---------------------------
 
 namespace pbf {
+
+int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  return sms;
+}
 
 pbf_status set_error(pbf_status s, const char* msg) { return fail(s, "%s", msg); }
 

@@ -191,6 +191,9 @@ constexpr int kScanTile = 2048;
 constexpr int kMaxScanPartials = 8192;
 constexpr int kSortTile = 2048;
 
+// Streaming multiprocessors of the current device (1 if they cannot be queried).
+int device_sms();
+
 int sort_tiles(int n);
 size_t radix_counts_len(int max_particles);
 

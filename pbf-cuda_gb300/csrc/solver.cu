@@ -2890,7 +2890,7 @@ void use_buckets(PassArgs& a, const SolverScratch& s) {
 }
 
 // Makes the pass take its computing particles in current-cell order: buckets
-// them (kBucketLaunches launches) and points the pass at the buckets.
+// them (bucket_launches) and points the pass at the buckets.
 cudaError_t bucket_by_cell(PassArgs& a, const SolverScratch& s, int n, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(s.bcnt, 0, sizeof(uint32_t) * (a.c.cells + 1), stream);
   if (e != cudaSuccess) return e;

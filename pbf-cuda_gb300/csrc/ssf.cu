@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) k_ssf_clear(int npix, uint32_t* __restric
 constexpr int kSplatThreads = 128;
 // Sprites of a warp: 32, or 8 where 32 would leave the SMs short of warps
 // (32,768 particles at 640 x 480: a frame 123 us with 32, 88 with 8).
-constexpr int kSplatFewBelow = 32 * 32 * 152;
+constexpr int splat_few_below(int sms) { return 32 * 32 * sms; }
 
 // Bound by the images' atomics (two for each fragment, resolved in L2) and
 // instruction issue.  A whole warp draws one sprite, so that an atomic's lanes
@@ -222,12 +222,12 @@ __global__ void __launch_bounds__(kSplatThreads) k_ssf_splat(SsfConsts c, const 
 
 template <bool kNarrow>
 void launch_splat(const SsfConsts& c, const float4* pos, int n, uint32_t* zkey, unsigned long long* tfx,
-                  unsigned long long* frags, cudaStream_t st) {
+                  unsigned long long* frags, int sms, cudaStream_t st) {
   const auto blocks = [n](int sprites) {
     const long long per_block = (long long)kSplatThreads / 32 * sprites;
     return (int)((n + per_block - 1) / per_block);
   };
-  if (n < kSplatFewBelow)
+  if (n < splat_few_below(sms))
     k_ssf_splat<8, kNarrow><<<blocks(8), kSplatThreads, 0, st>>>(c, pos, n, zkey, tfx, frags);
   else
     k_ssf_splat<32, kNarrow><<<blocks(32), kSplatThreads, 0, st>>>(c, pos, n, zkey, tfx, frags);
@@ -650,6 +650,7 @@ struct pbf_ssf {
   int sky_size = 0;
   unsigned long long* frag_count = nullptr;
   const float* final_depth = nullptr;  // the image shading read in the last render
+  int sms = 1;                         // streaming multiprocessors of the device
   bool splat_clear = false;            // zkey and tfx hold their clear values
   int profile = 0;
   bool have_events = false;
@@ -782,6 +783,7 @@ pbf_status pbf_ssf_create(const pbf_ssf_params* p, pbf_ssf** out) {
     delete s;
     return pbf::set_error(PBF_ERR_INVALID_ARG, "ssf create: view matrix is singular");
   }
+  s->sms = pbf::device_sms();
   const size_t npix = (size_t)p->width * p->height;
   cudaError_t e = cudaMalloc(&s->zkey, 4 * npix);
   if (e == cudaSuccess) e = cudaMalloc(&s->tfx, 8 * npix);
@@ -897,9 +899,9 @@ pbf_status pbf_ssf_render(pbf_ssf* s, const void* pos, int n, void* color, void*
     if (n > 0) {
       unsigned long long* frags = prof ? s->frag_count : nullptr;
       if (2.0 * c.r < 0.999)  // 2 r 2^32 < 2^32, with room for its rounding
-        launch_splat<true>(c, (const float4*)pos, n, s->zkey, s->tfx, frags, st);
+        launch_splat<true>(c, (const float4*)pos, n, s->zkey, s->tfx, frags, s->sms, st);
       else
-        launch_splat<false>(c, (const float4*)pos, n, s->zkey, s->tfx, frags, st);
+        launch_splat<false>(c, (const float4*)pos, n, s->zkey, s->tfx, frags, s->sms, st);
       ++launches;
     }
     k_ssf_resolve<<<(npix + 255) / 256, 256, 0, st>>>(npix, s->zkey, s->tfx, s->depth_a, s->thick);
