@@ -190,7 +190,7 @@ __device__ __forceinline__ int window_total(const SceneGeom& g, const uint32_t* 
 // which the window holds as well.  The loops with early exits that stood here
 // let a warp's lanes leave one by one, and k_dense's barrier after them did not
 // wait for the last ones (a part sum or a run of the block's previous batch was
-// then read in place of this one's: 1 in 30 steps of 30,011 scattered particles).
+// then read in place of this one's: 2 to 4 of 100 runs of four steps of 30,011 scattered particles).
 __device__ __forceinline__ bool window_flagged(const SceneGeom& g,
                                                const uint32_t* __restrict__ cell_flags, int3 q,
                                                uint32_t bits) {
@@ -1485,7 +1485,7 @@ __device__ __forceinline__ void sparse_one(const PassArgs& a, const SceneGeom& g
 // costs one coalesced load and one gathered one (position and lambda), kept
 // kListAhead ahead, and two entries share the packed arithmetic.  Bound by the
 // gathers (L1 data path 70% busy: 32 lanes' neighbours lie in ~10 lines).
-// 1,048,576 particles at rest density: 167 -> 72 us a pass (saved masks, whose
+// 1,048,576 particles at rest density: 167 -> 77 us a pass (saved masks, whose
 // bits a warp visits chunk by chunk, before).
 template <int kKind>
 __global__ void PBF_SPARSE_BOUNDS k_sparse(PassArgs a) {
@@ -1556,7 +1556,7 @@ __global__ void PBF_SPARSE_BOUNDS k_sparse(PassArgs a) {
 // Bound by the L1 data path and instruction issue: a test reads 12 bytes per
 // lane whatever the lanes share (L1 returns 128 bytes a cycle), 800 cycles for
 // 32 particles when every thread tested for one.  1,048,576 particles at rest
-// density: lambda 226 -> 146 us, xsph 260 -> 211 us; one particle per thread
+// density: lambda 226 -> 145 us, xsph 260 -> 212 us; one particle per thread
 // with the same queue and packed arithmetic 169 and 215.  Eight blocks (64
 // registers) beat seven (no spills) and nine by 1 and 4% of the step.
 template <int kKind>
@@ -1769,8 +1769,8 @@ __device__ __forceinline__ void visit_saved(const PassArgs& a, P& p, QueueColumn
 // own index, the runs of the batch's windows are loaded by all its warps at once
 // and shared, a part's tests have twelve 16-byte loads in flight, and where every
 // particle is dense the delta_p passes take the hits the lambda pass saved.
-// 1,728 particles: lambda 13.1 -> 9.0 us, delta_p 15.7 -> 7.2;
-// 65,231: 36 -> 36 and 43 -> 26.
+// 1,728 particles: lambda 13.1 -> 9.0 us, delta_p 15.7 -> 7.6;
+// 65,231: 36 -> 37 and 43 -> 29.
 template <int kKind, bool kStage>
 __global__ void PBF_DENSE_BOUNDS k_dense(PassArgs a) {
   using P = typename PassOf<kKind>::type;
